@@ -1,5 +1,6 @@
 // cplx.cuh -- FP64 complex arithmetic for device (and host) code.
 //
+// 16-byte aligned, so that an element is one 128-bit load or store.
 // Layout is two doubles {re, im}, the same as C99 `double _Complex` and
 // LAPACK COMPLEX*16, so matrices cross the C ABI without conversion.
 // Transcendentals are built on CUDA's double-precision exp, log, sincos,
@@ -10,7 +11,7 @@
 
 #define MSG_HD __host__ __device__ __forceinline__
 
-struct zc {
+struct __align__(16) zc {
     double re, im;
 };
 

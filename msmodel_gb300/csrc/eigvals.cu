@@ -37,7 +37,7 @@ namespace msg {
 
 // shared memory: the assembly's and the reductions' LuSmem; the Householder
 // vector overlays its two tile buffers (4096 complex values: n <= 4097)
-constexpr int EIG_NMAX = NB * (TM + TN) + 1;
+constexpr int EIG_NMAX = NB * (TM + LuSmem::TNC) + 1;
 
 struct EigParams {
     int nitem;
@@ -354,7 +354,8 @@ __global__ void __launch_bounds__(NT, 2) k_eigvals(EigParams P) {
     for (int it = blockIdx.x; it < P.nitem; it += gridDim.x) {
         const int n = P.item_n[it];
         const zc k = mk(P.ks[2 * it], P.ks[2 * it + 1]);
-        assemble(A, nullptr, n, P.item_d[it], P.pos + P.item_pos[it], P.item_model[it], k, s);
+        EntryRange rg;
+        assemble(A, nullptr, n, P.item_d[it], P.pos + P.item_pos[it], P.item_model[it], k, s, Solo{}, rg);
         __syncthreads();
         if (P.normalized) {
             // build_normalized_matrix (ms_matrix_util.c:50): off the diagonal -G(k, r_ij) / I(k, 0),

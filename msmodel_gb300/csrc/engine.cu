@@ -1,10 +1,10 @@
 // engine.cu -- batched Foldy-Lax engine: persistent kernels over a device
 // work queue, the runtime (device, workspace, jobs) and the msgpu_* C ABI.
 //
-// One CTA takes the next (k, realisation) item from an atomic counter,
-// assembles M(k) (and dM/dk) into its private slot of the workspace, factors
-// it and reduces the trace-log or the trace of M^-1 dM/dk, then takes the
-// next item.  Items are dealt largest-n first, so uneven sizes balance.
+// A team (one CTA, or a cluster of CTAs where the batch would leave SMs idle)
+// takes the next (k, realisation) item from an atomic counter, assembles M(k)
+// (and dM/dk) into its slot of the workspace, factors it and reduces the
+// trace-log or the trace of M^-1 dM/dk, then takes the next item.  Items are dealt largest-n first, so uneven sizes balance.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
@@ -15,154 +15,17 @@
 #include <vector>
 
 #include "msgpu.h"
-#include "lu64.cuh"
+#include "fp64_engine.cuh"
 #include "green_df.cuh"
-#include "engine_internal.h"
 
 using namespace msg;
 
 namespace msg {
 
-// complex elements of one CTA slot: the matrix, plus dM/dk (kind 1) or the
-// right-hand side (kind 2)
-__host__ __device__ inline size_t slot_elems(int kind, size_t slot, int nmax) {
-    if (kind == 1) return 2 * slot;
-    // kind 2: the matrix, its copy for the refinement residual (mixed engine), four vectors;
-    // kinds 1, 3: the matrix and a right-hand-side matrix; kind 4: the matrix and two vectors
-    const size_t vec = (((size_t)nmax + 15) / 16) * 16;
-    if (kind == 2) return 2 * slot + 4 * vec;
-    if (kind == 1 || kind == 3) return 2 * slot;
-    if (kind == 4) return slot + 2 * vec;
-    return slot;
-}
-
-// cnormalize (complex_vector_util.c:47): x /= fac, fac = |x| x_i0/|x_i0| with
-// x_i0 the first nonzero entry (locks the phase); returns fac
-static __device__ zc cnormalize_block(zc* __restrict__ x, int n, LuSmem& s) {
-    double nr = 0.0, z0 = 0.0, z1 = 0.0;
-    for (int i = threadIdx.x; i < n; i += NT) nr += zabs2(x[i]);
-    block_sum3(nr, z0, z1, s);
-    double nzv = -1.0;
-    int nzi = n;
-    for (int i = threadIdx.x; i < n; i += NT)
-        if (x[i].re != 0.0 || x[i].im != 0.0) {
-            nzv = 1.0;
-            nzi = min(nzi, i);
-        }
-    int i0;
-    block_argmax(nzv, nzi, s, i0);
-    if (i0 >= n) return mk(1.0);
-    const zc xi = x[i0];
-    const zc fac = (sqrt(nr) / zabs(xi)) * xi;
-    __syncthreads();  // every thread read x[i0] before it is rescaled
-    const zc rf = 1.0 / fac;
-    for (int i = threadIdx.x; i < n; i += NT) x[i] = x[i] * rf;
-    __syncthreads();
-    return fac;
-}
-
-// inverse_iteration (ms_matrix_util.c:279) on the LU already in A: from
-// `start` (n complex values, the caller's previous eigenvector) or else the
-// constant unit vector, x <- normalize(A^-1 x) until |x - x_old| < 1e-10 or 50
-// steps (the reference's ivit_maxit / ivit_toler); returns lambda = 1 / fac,
-// the eigenvalue of smallest modulus, x the eigenvector; conv = 0 if not reached.
-static __device__ zc inverse_iteration(const zc* __restrict__ A, zc* __restrict__ x, zc* __restrict__ xold, int n,
-                                       const int* __restrict__ ipiv, LuSmem& s, int& conv,
-                                       const double* __restrict__ start) {
-    for (int i = threadIdx.x; i < n; i += NT) x[i] = start ? mk(start[2 * i], start[2 * i + 1]) : mk(1.0);
-    __syncthreads();
-    zc fac = cnormalize_block(x, n, s);
-    conv = 0;
-    for (int it = 0; it < 50; ++it) {
-        for (int i = threadIdx.x; i < n; i += NT) xold[i] = x[i];
-        __syncthreads();
-        lu_solve_vec(A, x, n, ipiv, s);
-        fac = cnormalize_block(x, n, s);
-        double d2 = 0.0, z0 = 0.0, z1 = 0.0;
-        for (int i = threadIdx.x; i < n; i += NT) d2 += zabs2(x[i] - xold[i]);
-        block_sum3(d2, z0, z1, s);
-        if (sqrt(d2) < 1e-10) {
-            conv = 1;
-            break;
-        }
-    }
-    return 1.0 / fac;
-}
-
+// Two CTAs of 256 threads per SM, every update on the FP64 pipe.
 __global__ void __launch_bounds__(NT, 2) k_engine_fp64(EngineParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    LuSmem& s = *reinterpret_cast<LuSmem*>(smem_raw);
-    zc* A = P.ws + (size_t)blockIdx.x * slot_elems(P.kind, P.slot, P.piv_stride);
-    zc* B = (P.kind >= 1) ? A + P.slot : nullptr;
-    int* ipiv = P.piv + (size_t)blockIdx.x * P.piv_stride;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const unsigned q = atomicAdd(P.counter, 1u);
-            s.item = q < P.counter[1] ? (int)q : P.nitem;
-            s.info = 0;
-        }
-        __syncthreads();
-        const int q = s.item;
-        if (q >= P.nitem) break;
-        const int it = P.order[q];
-        const MedDev md = P.media[P.item_med[it]];
-        const zc k = mk(P.ks[2 * it], P.ks[2 * it + 1]);
-        assemble(A, P.kind == 1 ? B : nullptr, md.n, md.d, md.pos, md.model, k, s);
-        zc res;
-        int conv = 1;
-        if (P.kind == 3) {
-            // traceinv (ms_matrix_util.c:319): tr(M^-1 I) by the n-right-hand-side solve
-            for (size_t e = threadIdx.x; e < (size_t)md.n * md.n; e += NT)
-                B[e] = (e % (md.n + 1) == 0) ? mk(1.0) : mk(0.0);
-            __syncthreads();
-        }
-        if (P.kind == 2) {
-            // incident plane wave along +x (reference incident_wave_util.c:76, ms_core.c:616-618)
-            for (int i = threadIdx.x; i < md.n; i += NT) B[i] = zexp(mk(0.0, 1.0) * k * md.pos[i * md.d]);
-            __syncthreads();
-        }
-        lu_factor(A, md.n, ipiv, s);
-        if (P.kind == 0) {
-            res = lu_tracelog(A, md.n, ipiv, s);
-        } else if (P.kind == 1 || P.kind == 3) {
-            res = lu_trace_solve(A, B, md.n, ipiv, s);
-        } else if (P.kind == 4) {
-            const size_t vec = (((size_t)P.piv_stride + 15) / 16) * 16;
-            res = inverse_iteration(A, B, B + vec, md.n, ipiv, s, conv,
-                                    P.warm && P.amps ? P.amps + 2 * P.amp_off[it] : nullptr);
-            if (P.amps)
-                for (int i = threadIdx.x; i < md.n; i += NT) {
-                    P.amps[2 * (P.amp_off[it] + i)] = B[i].re;
-                    P.amps[2 * (P.amp_off[it] + i) + 1] = B[i].im;
-                }
-        } else {
-            lu_solve_vec(A, B, md.n, ipiv, s);
-            // optical theorem sigma = -Im(conj(phi).a)/k (reference ms_matrix_util.c:361)
-            double dr = 0.0, di = 0.0, z = 0.0;
-            for (int i = threadIdx.x; i < md.n; i += NT) {
-                zc ph = zexp(mk(0.0, 1.0) * k * md.pos[i * md.d]);
-                zc t = conjz(ph) * B[i];
-                dr += t.re;
-                di += t.im;
-                if (P.amps) {
-                    P.amps[2 * (P.amp_off[it] + i)] = B[i].re;
-                    P.amps[2 * (P.amp_off[it] + i) + 1] = B[i].im;
-                }
-            }
-            block_sum3(dr, di, z, s);
-            res = mk(-di, 0.0) / k;
-        }
-        if (threadIdx.x == 0) {
-            P.out[2 * it] = res.re;
-            P.out[2 * it + 1] = res.im;
-            int st = 0;
-            if (s.info) st |= MSGPU_S_SINGULAR;
-            if (!isfinite(res.re) || !isfinite(res.im)) st |= MSGPU_S_NONFINITE;
-            if (!conv) st |= MSGPU_S_NOCONV;
-            P.status[it] = st;
-        }
-        __syncthreads();
-    }
+    run_items_fp64(P, *reinterpret_cast<LuSmem*>(smem_raw), this_team(), DfmaUpdate{});
 }
 
 // single-matrix assembly for the drop-in layer (build_matrix.cu)
@@ -174,7 +37,7 @@ __global__ void __launch_bounds__(NT, 1) k_tracelog_matrix(zc* A, int n, int* ip
     LuSmem& s = *reinterpret_cast<LuSmem*>(smem_raw);
     if (threadIdx.x == 0) s.info = 0;
     __syncthreads();
-    lu_factor(A, n, ipiv, s);
+    lu_factor(A, n, ipiv, false, s, Solo{}, DfmaUpdate{});
     zc r = lu_tracelog(A, n, ipiv, s);
     if (threadIdx.x == 0) {
         out[0] = r.re;
@@ -234,6 +97,7 @@ std::string g_err;
 int g_dev = -1;
 int g_sms = 0;
 int g_ctas_fp64 = 0;
+int g_teams[5] = {};  // FP64 kernel: clusters of 2^j CTAs the device holds at once
 std::atomic<uint64_t> g_launches{0};
 void* g_ws = nullptr;
 size_t g_ws_bytes = 0;
@@ -285,6 +149,9 @@ int init_locked(int device) {
     int occ = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_engine_fp64, NT, smem_bytes()));
     g_ctas_fp64 = std::max(1, occ);
+    CK(cudaFuncSetAttribute(k_engine_fp64, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (int j = 1; j < 5; ++j) g_teams[j] = max_teams(k_engine_fp64, 1 << j, NT, smem_bytes());
+    g_teams[0] = g_sms * g_ctas_fp64;
     g_dev = device;
     return 0;
 }
@@ -313,6 +180,35 @@ static size_t ws_budget() {
     return std::min(cap, avail > ((size_t)4 << 30) ? avail - ((size_t)4 << 30) : avail / 2);
 }
 
+static int ilog2(int v) {
+    int j = 0;
+    while ((2 << j) <= v) ++j;
+    return j;
+}
+
+// CTAs per matrix: the team size whose estimated time is least.  A matrix
+// takes a part s of its time in steps one CTA does (the panels) and 1 - s in
+// steps the team shares; the items go in waves of as many teams as the device
+// holds at once.
+static int pick_team(int nitem, int nmax) {
+    const double s = 0.3;
+    int best = 1;
+    double t_best = 0.0;
+    for (int j = 0; j < 5; ++j) {
+        const int team = 1 << j, teams = g_teams[j];
+        if (teams < 1 || (team > 1 && nmax < 16 * team)) break;
+        // CTAs that share an SM share its FP64 pipe
+        const double waves = (nitem + teams - 1) / teams;
+        const double share = (double)std::min(nitem, teams) * team > g_sms ? 1.6 : 1.0;
+        const double t = waves * share * (s + (1.0 - s) / team);
+        if (j == 0 || t < 0.95 * t_best) {
+            best = team;
+            t_best = t;
+        }
+    }
+    return best;
+}
+
 struct msgpu_job {
     int kind = 0, precision = 0, nitem = 0, nmed = 0, nmax = 0;
     int cap = 0;  // item capacity of the device arrays
@@ -336,6 +232,7 @@ struct msgpu_job {
     int* d_piv = nullptr;
     size_t slot = 0;
     size_t ws_bytes = 0;
+    int team = 1;            // FP64: CTAs that share one matrix
     long long amp_total = 0, amp_cap = 0;
     double* d_amps = nullptr;
     long long* d_amp_off = nullptr;
@@ -658,9 +555,11 @@ msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int n
     }
     // per-CTA slots
     J->slot = (size_t)J->nmax * J->nmax;
+    const bool fp64 = J->precision == MSGPU_FP64;
     const size_t per_cta = slot_elems(kind, J->slot, J->nmax) * sizeof(zc);
     const int ctas = te.ctas ? std::min(te.ctas, g_ctas_fp64) : g_ctas_fp64;
-    int grid = std::min(nitem, g_sms * ctas);
+    if (fp64) J->team = pick_team(nitem, J->nmax);
+    int grid = std::min(nitem, J->team > 1 ? g_teams[ilog2(J->team)] : g_sms * ctas);
     size_t budget = ws_budget();
     while (grid > 1 && (size_t)grid * per_cta > budget) grid--;
     J->grid = grid;
@@ -713,8 +612,8 @@ static int launch_locked(msgpu_job* J, void* ws, cudaStream_t st) {
         if (e) return set_err(e, "mixed engine launch failed");
         return 0;
     }
-    k_engine_fp64<<<J->grid, NT, smem_bytes(), st>>>(P);
-    CK(cudaGetLastError());
+    const int e = launch_teams(k_engine_fp64, J->grid, J->team, NT, smem_bytes(), st, P);
+    if (e) return set_err(e, std::string("FP64 engine launch failed: ") + cudaGetErrorString(cudaGetLastError()));
     return 0;
 }
 

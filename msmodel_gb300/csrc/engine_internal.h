@@ -38,6 +38,44 @@ struct EngineParams {
 // adds to the library's count of kernel launches (msgpu_launch_count)
 void count_launches(int n);
 
+// Launches `teams` clusters of `team` CTAs (a plain launch for team = 1).
+template <class... KArgs, class... Args>
+int launch_teams(void (*kern)(KArgs...), int teams, int team, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(teams * team));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)team;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = team > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...) == cudaSuccess ? 0 : MSGPU_E_CUDA;
+}
+
+// clusters of `team` CTAs the device holds at once (0: none of that size)
+template <class K>
+int max_teams(K kern, int team, int threads, size_t smem) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)team);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)team;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 // Mixed-precision engine (mixed.cu).  Returns 0 when it ran the job, a
 // negative MSGPU_E* code on error.
 // d3only: every medium of the job has d = 3 (selects the d = 3 kernel instantiation);

@@ -223,8 +223,9 @@ MSG_D zc invf(const msgpu_model& m, int d, zc k) {
 }
 
 // diagonal of dM/dk: central difference with step 1e-4 (reference ms_matrix_util.c:69-70)
+constexpr double DK_INVF_STEP = 1e-4;
 MSG_D zc dk_invf(const msgpu_model& m, int d, zc k) {
-    const double h = 1e-4;
+    const double h = DK_INVF_STEP;
     return (invf(m, d, k + h) - invf(m, d, k - h)) / (2.0 * h);
 }
 

@@ -1,8 +1,10 @@
 // lu64.cuh -- CTA-level FP64 complex dense kernels: blocked right-looking
 // LU with partial pivoting, the triangular solves of LAPACK zgetrs, and the
-// Foldy-Lax matrix assembly.  One CTA owns one matrix in global memory
-// (column-major, leading dimension n) and works on it alone, so thousands of
-// (k, realisation) matrices factor concurrently with no inter-CTA traffic.
+// Foldy-Lax matrix assembly.  A matrix lives in global memory (column-major,
+// leading dimension n) and belongs to a team: one CTA where there are matrices
+// enough to fill the chip, so that thousands of (k, realisation) matrices
+// factor concurrently with no inter-CTA traffic, or the CTAs of a cluster.
+// Every element takes the same operations in the same order in any team.
 //
 // The FP64 pipe of GB300 is the roofline of this path (about 2 FP64 FMA
 // lanes per SM per clock): every loop below keeps the SM's FP64 FMAs fed
@@ -22,22 +24,74 @@ namespace msg {
 
 constexpr int NT = 256;  // threads per CTA
 constexpr int NB = 32;   // panel width
-constexpr int TM = 64;   // trailing-update tile rows
-constexpr int TN = 64;   // trailing-update tile columns
+constexpr int TM = 64;   // DFMA trailing-update tile rows
 
-struct __align__(16) LuSmem {
+// complex a - l u in two FMAs per component: a product, an FMA and a difference
+// (what a - l * u compiles to) would hold the FP64 pipe half as long again
+MSG_D zc zfms(zc a, zc l, zc u) {
+    a.re = fma(-l.re, u.re, a.re);
+    a.re = fma(l.im, u.im, a.re);
+    a.im = fma(-l.re, u.im, a.im);
+    a.im = fma(-l.im, u.re, a.im);
+    return a;
+}
+
+// The CTAs that factor one matrix together.  Solo: one CTA, the barrier is
+// __syncthreads.  ClusterTeam: the CTAs of a thread-block cluster; its barrier
+// (release / acquire at cluster scope) orders their global-memory accesses.
+struct Solo {
+    static constexpr int rank = 0, size = 1;
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+// A batch that leaves SMs idle gives each matrix several CTAs: the 32 targets of
+// one resonance search at n = 100 take 45 ms against 83 ms with one CTA each
+// (the panel's share included), one dlogf at d = 2, n = 50 1.7 against 2.5 ms.
+struct ClusterTeam {
+    int rank, size;
+    __device__ __forceinline__ void sync() const {
+        if (size == 1) {
+            __syncthreads();
+        } else {
+            asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        }
+    }
+};
+
+__device__ __forceinline__ ClusterTeam this_team() {
+    uint32_t r, n;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+    return ClusterTeam{(int)r, (int)n};
+}
+// the same shared-memory variable in CTA `rank` of the cluster := v
+__device__ __forceinline__ void cluster_store(int* p, int rank, int v) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// shared memory of a CTA of NTH threads: NTH / 16 x 4 = TNC columns per DFMA tile
+template <int NTHREADS>
+struct __align__(16) LuSmemT {
+    static constexpr int NTH = NTHREADS;
+    static constexpr int TNC = NTHREADS / 4;  // trailing-update tile columns (64 for 256 threads)
     zc As[NB][TM];       // 32 KB  L21 tile  (k-major)
-    zc Bs[NB][TN];       // 32 KB  U12 tile  (k-major)
+    zc Bs[NB][TNC];      // U12 tile  (k-major)
     zc T[NB][NB + 1];    // 16.5 KB diagonal block / assembly transpose
     zc urow[NB];         // pivot row of the panel
+    zc piv, rpiv;        // the pivot and its reciprocal
     zc diag[2];          // F^-1(k), d F^-1/dk
-    double red_v[NT / 32];
-    int red_i[NT / 32];
-    double red_s[3][NT / 32];
+    long long red_k[2][NTHREADS / 32];
+    int red_p[2][NTHREADS / 32];
+    double red_v[NTHREADS / 32];
+    int red_i[NTHREADS / 32];
+    double red_s[3][NTHREADS / 32];
     int info;
     int bcast_i;
     int item;
+    int nz;
 };
+using LuSmem = LuSmemT<NT>;
 
 template <class S>
 __device__ __forceinline__ void block_argmax(double v, int i, S& s, int& oi) {
@@ -54,7 +108,7 @@ __device__ __forceinline__ void block_argmax(double v, int i, S& s, int& oi) {
     if (threadIdx.x == 0) {
         double bv = s.red_v[0];
         int bi = s.red_i[0];
-        for (int w = 1; w < NT / 32; w++) {
+        for (int w = 1; w < S::NTH / 32; w++) {
             double v2 = s.red_v[w];
             int i2 = s.red_i[w];
             if (v2 > bv || (v2 == bv && i2 < bi)) { bv = v2; bi = i2; }
@@ -79,64 +133,161 @@ __device__ __forceinline__ void block_sum3(double& a, double& b, double& c, S& s
     if (lane == 0) { s.red_s[0][warp] = a; s.red_s[1][warp] = b; s.red_s[2][warp] = c; }
     __syncthreads();
     a = b = c = 0.0;
-    for (int w = 0; w < NT / 32; w++) { a += s.red_s[0][w]; b += s.red_s[1][w]; c += s.red_s[2][w]; }
+    for (int w = 0; w < S::NTH / 32; w++) { a += s.red_s[0][w]; b += s.red_s[1][w]; c += s.red_s[2][w]; }
     __syncthreads();
 }
 
-// Factor the panel A[j0:n, j0:j0+jb) in place; interchanges inside the panel only.
-static __device__ void panel_factor(zc* __restrict__ A, int n, int j0, int jb, int* __restrict__ ipiv, LuSmem& s) {
+// Pivot keys: |Re| + |Im| >= 0 as its bit pattern, which orders like the value,
+// so that the search compares integers and leaves the FP64 pipe alone; a NaN
+// (never chosen, as in IZAMAX's comparison) and "no row" are -1.
+MSG_D long long pivot_key(zc a) {
+    const long long b = __double_as_longlong(abs1(a));
+    return b > 0x7FF0000000000000LL ? -1LL : b;
+}
+
+// row of the CTA's largest key (smallest row on ties), in every thread; one
+// barrier: the warps' candidates are double-buffered by `par`
+template <class S>
+__device__ __forceinline__ int block_pivot(long long key, int row, int par, S& s) {
+    constexpr int NW = S::NTH / 32;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const long long k2 = __shfl_xor_sync(FULL, key, off);
+        const int r2 = __shfl_xor_sync(FULL, row, off);
+        if (k2 > key || (k2 == key && r2 < row)) { key = k2; row = r2; }
+    }
+    if (lane == 0) { s.red_k[par][warp] = key; s.red_p[par][warp] = row; }
+    __syncthreads();
+    key = s.red_k[par][lane & (NW - 1)];
+    row = s.red_p[par][lane & (NW - 1)];
+#pragma unroll
+    for (int off = NW / 2; off > 0; off >>= 1) {
+        const long long k2 = __shfl_xor_sync(FULL, key, off);
+        const int r2 = __shfl_xor_sync(FULL, row, off);
+        if (k2 > key || (k2 == key && r2 < row)) { key = k2; row = r2; }
+    }
+    return row;
+}
+
+// Factor the panel A[j0:n, j0:j0+jb) in place by one CTA; interchanges inside
+// the panel only.  Sub-panels of SWP columns: inside one the rank-1 updates
+// touch only its own columns, the rest of the panel then takes one rank-SWP
+// update (U rows by unit-lower substitution), so the panel is read and written
+// once per sub-panel and not once per column; each element still takes its
+// updates in the order of the columns.  Per column the pivot's reciprocal is
+// one lane's work (256 threads each doing the hypot and the divisions held
+// the FP64 pipe, 2 lanes a clock, for ~10k cycles a column) and there are two
+// barriers.  4096 ln det at n = 64 (d = 3): 19.6 ms with the full-width rank-1
+// form and a reciprocal per thread, 11.6 ms now.
+constexpr int SWP = 4;
+template <class S>
+static __device__ __noinline__ void panel_factor(zc* A, int n, int j0, int jb, int* ipiv, S& s) {
+    constexpr int NTH = S::NTH;
     const int tid = threadIdx.x;
     const int cend = j0 + jb;
-    double bv = -1.0;
+    long long bk = -1;
     int bi = n;
-    for (int i = j0 + tid; i < n; i += NT) {
-        double v = abs1(A[i + (size_t)j0 * n]);
-        if (v > bv) { bv = v; bi = i; }
+    for (int i = j0 + tid; i < n; i += NTH) {
+        const long long k = pivot_key(A[i + (size_t)j0 * n]);
+        if (k > bk) { bk = k; bi = i; }
     }
-    for (int c = j0; c < cend; ++c) {
-        int p;
-        block_argmax(bv, bi, s, p);
-        if (p >= n) p = c;
-        const zc piv = A[p + (size_t)c * n];
-        const bool nz = !is_zero(piv);
-        if (tid == 0) {
-            ipiv[c] = p;
-            if (!nz && s.info == 0) s.info = c + 1;
+    for (int c0 = j0; c0 < cend; c0 += SWP) {
+        const int sw = min(c0 + SWP, cend);
+        for (int c = c0; c < sw; ++c) {
+            int p = block_pivot(bk, bi, c & 1, s);
+            if (p >= n) p = c;
+            if (tid < 32) {
+                // the interchange of rows c and p within the panel, one column a lane
+                const size_t col = (size_t)(j0 + tid) * n;
+                zc a = mk(0.0), b = mk(0.0);
+                if (tid < jb) {
+                    a = A[c + col];
+                    b = p != c ? A[p + col] : a;
+                    s.urow[tid] = b;
+                }
+                const bool nz = __shfl_sync(0xffffffffu, (int)!is_zero(b), c - j0) != 0;
+                if (nz && p != c && tid < jb) {
+                    A[c + col] = b;
+                    A[p + col] = a;
+                }
+                if (!nz && tid < jb) s.urow[tid] = a;  // a zero column: no interchange
+                if (tid == c - j0) {
+                    ipiv[c] = p;
+                    if (!nz && s.info == 0) s.info = c + 1;
+                    const bool recip = nz && zabs(b) >= DBL_MIN;
+                    s.nz = nz ? (recip ? 1 : 2) : 0;
+                    s.piv = b;
+                    s.rpiv = recip ? zrecip(b) : mk(0.0);
+                }
+            }
+            __syncthreads();
+            const int nz = s.nz;
+            const zc r = s.rpiv;
+            bk = -1;
+            bi = n;
+            if (nz) {
+                for (int i = c + 1 + tid; i < n; i += NTH) {
+                    zc l = A[i + (size_t)c * n];
+                    l = nz == 1 ? l * r : l / s.piv;
+                    A[i + (size_t)c * n] = l;
+                    if (c + 1 < sw) {
+                        const zc a = zfms(A[i + (size_t)(c + 1) * n], l, s.urow[c + 1 - j0]);
+                        A[i + (size_t)(c + 1) * n] = a;
+                        const long long k = pivot_key(a);
+                        if (k > bk) { bk = k; bi = i; }
+                        for (int cc = c + 2; cc < sw; ++cc) {
+                            zc* q = A + i + (size_t)cc * n;
+                            *q = zfms(*q, l, s.urow[cc - j0]);
+                        }
+                    }
+                }
+            } else if (c + 1 < sw) {
+                for (int i = c + 1 + tid; i < n; i += NTH) {
+                    const long long k = pivot_key(A[i + (size_t)(c + 1) * n]);
+                    if (k > bk) { bk = k; bi = i; }
+                }
+            }
         }
-        __syncthreads();  // every thread holds the pivot before row p is swapped away
-        if (nz && p != c && tid < jb) {
-            const size_t col = (size_t)(j0 + tid) * n;
-            zc t = A[c + col];
-            A[c + col] = A[p + col];
-            A[p + col] = t;
-        }
-        __syncthreads();
-        if (tid < jb && j0 + tid > c) s.urow[tid] = A[c + (size_t)(j0 + tid) * n];
-        __syncthreads();
-        bv = -1.0;
-        bi = n;
-        if (nz) {
-            const bool recip = zabs(piv) >= DBL_MIN;
-            const zc r = recip ? 1.0 / piv : mk(0.0);
-            for (int i = c + 1 + tid; i < n; i += NT) {
-                zc l = A[i + (size_t)c * n];
-                l = recip ? l * r : l / piv;
-                A[i + (size_t)c * n] = l;
-                if (c + 1 < cend) {
-                    zc a = A[i + (size_t)(c + 1) * n] - l * s.urow[c + 1 - j0];
-                    A[i + (size_t)(c + 1) * n] = a;
-                    double v = abs1(a);
-                    if (v > bv) { bv = v; bi = i; }
-                    for (int cc = c + 2; cc < cend; ++cc) {
-                        zc* q = A + i + (size_t)cc * n;
-                        *q = *q - l * s.urow[cc - j0];
+        if (sw < cend) {
+            const int cw = sw - c0, rem = cend - sw;
+            __syncthreads();  // the sub-panel's last column is complete
+            // U rows of the sub-panel right of it: u_r = a_r - sum_{q<r} L_rq u_q
+            if (tid < rem) {
+                const size_t col = (size_t)(sw + tid) * n;
+                zc u[SWP];
+#pragma unroll
+                for (int r = 0; r < SWP; ++r) {
+                    if (r < cw) {
+                        zc a = A[c0 + r + col];
+#pragma unroll
+                        for (int q = 0; q < r; ++q) a = zfms(a, A[c0 + r + (size_t)(c0 + q) * n], u[q]);
+                        u[r] = a;
+                        A[c0 + r + col] = a;
+                        s.T[r][tid] = a;
                     }
                 }
             }
-        } else if (c + 1 < cend) {
-            for (int i = c + 1 + tid; i < n; i += NT) {
-                double v = abs1(A[i + (size_t)(c + 1) * n]);
-                if (v > bv) { bv = v; bi = i; }
+            __syncthreads();
+            bk = -1;
+            bi = n;
+            for (int i = sw + tid; i < n; i += NTH) {
+                zc l[SWP];
+#pragma unroll
+                for (int q = 0; q < SWP; ++q) l[q] = q < cw ? A[i + (size_t)(c0 + q) * n] : mk(0.0);
+                for (int t = 0; t < rem; ++t) {
+                    zc* q = A + i + (size_t)(sw + t) * n;
+                    zc a = *q;
+#pragma unroll
+                    for (int e = 0; e < SWP; ++e)
+                        if (e < cw) a = zfms(a, l[e], s.T[e][t]);
+                    *q = a;
+                    if (t == 0) {
+                        const long long k = pivot_key(a);
+                        if (k > bk) { bk = k; bi = i; }
+                    }
+                }
             }
         }
     }
@@ -157,18 +308,19 @@ __device__ __forceinline__ void col_solve_lower_unit(zc* __restrict__ b, int jb,
         for (int q = 0; q < rb; ++q) {
             const zc xq = b[q];
 #pragma unroll
-            for (int r = 0; r < CH; ++r) y[r] -= T[rb + r][q] * xq;
+            for (int r = 0; r < CH; ++r) y[r] = zfms(y[r], T[rb + r][q], xq);
         }
 #pragma unroll
         for (int r = 1; r < CH; ++r)
 #pragma unroll
-            for (int q = 0; q < r; ++q) y[r] -= T[rb + r][rb + q] * y[q];
+            for (int q = 0; q < r; ++q) y[r] = zfms(y[r], T[rb + r][rb + q], y[q]);
 #pragma unroll
         for (int r = 0; r < CH; ++r)
             if (rb + r < jb) b[rb + r] = y[r];
     }
 }
 
+// the upper solve; T's diagonal holds the reciprocals of U_rr
 __device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, const zc (*T)[NB + 1]) {
     for (int rb = ((jb - 1) / CH) * CH; rb >= 0; rb -= CH) {
         zc y[CH];
@@ -177,15 +329,15 @@ __device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, cons
         for (int q = rb + CH; q < jb; ++q) {
             const zc xq = b[q];
 #pragma unroll
-            for (int r = 0; r < CH; ++r) y[r] -= T[rb + r][q] * xq;
+            for (int r = 0; r < CH; ++r) y[r] = zfms(y[r], T[rb + r][q], xq);
         }
 #pragma unroll
         for (int r = CH - 1; r >= 0; --r) {
             if (rb + r < jb) {
                 zc acc = y[r];
 #pragma unroll
-                for (int q = r + 1; q < CH; ++q) acc -= T[rb + r][rb + q] * y[q];
-                y[r] = acc / T[rb + r][rb + r];
+                for (int q = r + 1; q < CH; ++q) acc = zfms(acc, T[rb + r][rb + q], y[q]);
+                y[r] = acc * T[rb + r][rb + r];
             }
         }
 #pragma unroll
@@ -194,17 +346,30 @@ __device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, cons
     }
 }
 
+// first column and stride of this thread when a team deals columns in blocks
+// of 32 (one per warp), CTA by CTA, so that few columns still spread over it
+template <class S, class Team>
+__device__ __forceinline__ void team_columns(const Team& tm, int& first, int& step) {
+    first = ((threadIdx.x >> 5) * tm.size + tm.rank) * 32 + (threadIdx.x & 31);
+    step = S::NTH * tm.size;
+}
+
 // Apply the panel's interchanges to every other column and compute
-// U12 = L11^-1 A12 (columns right of the panel).
-static __device__ void panel_swaps_trsm(zc* __restrict__ A, int n, int j0, int jb, const int* __restrict__ ipiv,
-                                 LuSmem& s) {
-    const int tid = threadIdx.x;
-    for (int e = tid; e < NB * NB; e += NT) {
+// U12 = L11^-1 A12 (columns right of the panel).  keep_l = false leaves the
+// columns left of the panel alone: a ln det reads only U's diagonal and the
+// pivots afterwards.
+template <class S, class Team>
+static __device__ void panel_swaps_trsm(zc* A, int n, int j0, int jb, const int* ipiv, bool keep_l,
+                                        S& s, const Team& tm) {
+    for (int e = threadIdx.x; e < NB * NB; e += S::NTH) {
         int r = e % NB, q = e / NB;
         s.T[r][q] = (r < jb && q < r) ? A[(j0 + r) + (size_t)(j0 + q) * n] : mk(0.0);
     }
     __syncthreads();
-    for (int col = tid; col < n; col += NT) {
+    int first, step;
+    team_columns<S>(tm, first, step);
+    const int base = keep_l ? 0 : j0 + jb;
+    for (int col = base + first; col < n; col += step) {
         if (col >= j0 && col < j0 + jb) continue;
         zc* a = A + (size_t)col * n;
         for (int c = j0; c < j0 + jb; ++c) {
@@ -213,28 +378,35 @@ static __device__ void panel_swaps_trsm(zc* __restrict__ A, int n, int j0, int j
         }
         if (col >= j0 + jb) col_solve_lower_unit(a + j0, jb, s.T);
     }
-    __syncthreads();
+    tm.sync();
 }
 
 // C[m x nn] -= Ablk[m x kk] * Bblk[kk x nn] (all column-major); kk <= NB.
-// tri != 0: only tiles that hold some element with row >= col are updated
-// (row/col counted from the C origin plus rofs/cofs).
-static __device__ void gemm_sub(zc* __restrict__ C, int ldc, const zc* __restrict__ Ab, int lda, const zc* __restrict__ Bb,
-                         int ldb, int m, int nn, int kk, LuSmem& s, int tri = 0, int rofs = 0, int cofs = 0) {
+// tri != 0: only tiles that hold some element with row >= col are updated.
+// The team deals the tiles round robin; the caller's barrier ends the update.
+template <class S, class Team>
+static __device__ void gemm_sub(zc* C, int ldc, const zc* Ab, int lda, const zc* Bb,
+                         int ldb, int m, int nn, int kk, S& s, const Team& tm, int tri = 0) {
+    constexpr int NTH = S::NTH, TNC = S::TNC, CST = NTH / 16;
     if (m <= 0 || nn <= 0 || kk <= 0) return;
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
+    int t = 0;
     for (int ti = 0; ti < m; ti += TM) {
-        if (tri && rofs + ti + TM - 1 < cofs) continue;  // whole row band above every column
-        for (int e = tid; e < NB * TM; e += NT) {
-            int r = e % TM, k = e / TM;
-            zc v = mk(0.0);
-            if (k < kk && ti + r < m) v = Ab[(ti + r) + (size_t)k * lda];
-            s.As[k][r] = v;
-        }
-        for (int tj = 0; tj < nn; tj += TN) {
-            if (tri && rofs + ti + TM - 1 < cofs + tj) break;
-            for (int e = tid; e < NB * TN; e += NT) {
+        bool have_a = false;
+        for (int tj = 0; tj < nn; tj += TNC) {
+            if (tri && ti + TM - 1 < tj) break;
+            if (tm.size > 1 && t++ % tm.size != tm.rank) continue;
+            if (!have_a) {
+                have_a = true;
+                for (int e = tid; e < NB * TM; e += NTH) {
+                    int r = e % TM, k = e / TM;
+                    zc v = mk(0.0);
+                    if (k < kk && ti + r < m) v = Ab[(ti + r) + (size_t)k * lda];
+                    s.As[k][r] = v;
+                }
+            }
+            for (int e = tid; e < NB * TNC; e += NTH) {
                 int k = e % NB, c = e / NB;
                 zc v = mk(0.0);
                 if (k < kk && tj + c < nn) v = Bb[k + (size_t)(tj + c) * ldb];
@@ -246,7 +418,7 @@ static __device__ void gemm_sub(zc* __restrict__ C, int ldc, const zc* __restric
             for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    int r = ti + tx + 16 * a, c = tj + ty + 16 * b;
+                    int r = ti + tx + 16 * a, c = tj + ty + CST * b;
                     acc[a][b] = (r < m && c < nn) ? C[r + (size_t)c * ldc] : mk(0.0);
                 }
 #pragma unroll 2
@@ -255,22 +427,17 @@ static __device__ void gemm_sub(zc* __restrict__ C, int ldc, const zc* __restric
 #pragma unroll
                 for (int a = 0; a < 4; ++a) av[a] = s.As[k][tx + 16 * a];
 #pragma unroll
-                for (int b = 0; b < 4; ++b) bw[b] = s.Bs[k][ty + 16 * b];
+                for (int b = 0; b < 4; ++b) bw[b] = s.Bs[k][ty + CST * b];
 #pragma unroll
                 for (int a = 0; a < 4; ++a)
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        acc[a][b].re = fma(-av[a].re, bw[b].re, acc[a][b].re);
-                        acc[a][b].re = fma(av[a].im, bw[b].im, acc[a][b].re);
-                        acc[a][b].im = fma(-av[a].re, bw[b].im, acc[a][b].im);
-                        acc[a][b].im = fma(-av[a].im, bw[b].re, acc[a][b].im);
-                    }
+                    for (int b = 0; b < 4; ++b) acc[a][b] = zfms(acc[a][b], av[a], bw[b]);
             }
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    int r = ti + tx + 16 * a, c = tj + ty + 16 * b;
+                    int r = ti + tx + 16 * a, c = tj + ty + CST * b;
                     if (r < m && c < nn) C[r + (size_t)c * ldc] = acc[a][b];
                 }
             __syncthreads();
@@ -278,22 +445,42 @@ static __device__ void gemm_sub(zc* __restrict__ C, int ldc, const zc* __restric
     }
 }
 
-// In-place LU of A (n x n, ld n).  ipiv 0-based.  Sets s.info (1-based first zero pivot).
-static __device__ void lu_factor(zc* __restrict__ A, int n, int* __restrict__ ipiv, LuSmem& s) {
+// the trailing update on the FP64 pipe (DFMA); another kernel may pass its own
+struct EntryRange;
+struct DfmaUpdate {
+    template <class S, class Team>
+    __device__ __forceinline__ void begin(const EntryRange&, int, S&, const Team&) const {}
+    template <class S, class Team>
+    __device__ __forceinline__ bool failed(S&, const Team&) const { return false; }
+    template <class S, class Team>
+    __device__ __forceinline__ void operator()(zc* C, int ldc, const zc* Ab, int lda, const zc* Bb, int ldb, int m, int nn,
+                                               int kk, int tri, S& s, const Team& tm) const {
+        gemm_sub(C, ldc, Ab, lda, Bb, ldb, m, nn, kk, s, tm, tri);
+    }
+};
+
+// In-place LU of A (n x n, ld n).  ipiv 0-based.  Sets s.info of the team's
+// first CTA (1-based first zero pivot).
+template <class S, class Team, class Update>
+static __device__ void lu_factor(zc* A, int n, int* ipiv, bool keep_l, S& s, const Team& tm,
+                                 const Update& update) {
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
-        panel_factor(A, n, j0, jb, ipiv, s);
-        panel_swaps_trsm(A, n, j0, jb, ipiv, s);
+        if (tm.rank == 0) panel_factor(A, n, j0, jb, ipiv, s);
+        if (tm.size > 1) tm.sync();
+        panel_swaps_trsm(A, n, j0, jb, ipiv, keep_l, s, tm);
         const int r0 = j0 + jb;
-        gemm_sub(A + r0 + (size_t)r0 * n, n, A + r0 + (size_t)j0 * n, n, A + j0 + (size_t)r0 * n, n, n - r0, n - r0,
-                 jb, s);
+        update(A + r0 + (size_t)r0 * n, n, A + r0 + (size_t)j0 * n, n, A + j0 + (size_t)r0 * n, n, n - r0, n - r0, jb, 0, s,
+               tm);
+        if (tm.size > 1) tm.sync();
     }
 }
 
 // ln det(A)/n with the reference's branch: sum log|U_ii| + i (sum Arg U_ii + pi [odd interchanges]).
-static __device__ zc lu_tracelog(const zc* __restrict__ A, int n, const int* __restrict__ ipiv, LuSmem& s) {
+template <class S>
+static __device__ zc lu_tracelog(const zc* A, int n, const int* ipiv, S& s) {
     double lr = 0.0, ar = 0.0, odd = 0.0;
-    for (int i = threadIdx.x; i < n; i += NT) {
+    for (int i = threadIdx.x; i < n; i += S::NTH) {
         zc u = A[i + (size_t)i * n];
         lr += log(hypot(u.re, u.im));
         ar += atan2(u.im, u.re);
@@ -307,46 +494,57 @@ static __device__ zc lu_tracelog(const zc* __restrict__ A, int n, const int* __r
 // tr(A^-1 B) given the LU of A (LAPACK layout) and B (n x n, ld n), B destroyed:
 // B <- P B, forward solve with unit-lower L, backward solve with U restricted
 // to the rows each diagonal element needs (X_jj depends on rows >= j only).
-static __device__ zc lu_trace_solve(const zc* __restrict__ A, zc* __restrict__ B, int n, const int* __restrict__ ipiv,
-                             LuSmem& s) {
+template <class S, class Team, class Update>
+static __device__ zc lu_trace_solve(const zc* A, zc* B, int n, const int* ipiv,
+                             S& s, const Team& tm, const Update& update) {
+    constexpr int NTH = S::NTH;
     const int tid = threadIdx.x;
-    for (int col = tid; col < n; col += NT) {
+    int first, step;
+    team_columns<S>(tm, first, step);
+    for (int col = first; col < n; col += step) {
         zc* b = B + (size_t)col * n;
         for (int i = 0; i < n; ++i) {
             int p = ipiv[i];
             if (p != i) { zc t = b[i]; b[i] = b[p]; b[p] = t; }
         }
     }
-    __syncthreads();
+    tm.sync();
     // forward: L X = P B
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
-        for (int e = tid; e < NB * NB; e += NT) {
+        for (int e = tid; e < NB * NB; e += NTH) {
             int r = e % NB, q = e / NB;
             s.T[r][q] = (r < jb && q < r) ? A[(j0 + r) + (size_t)(j0 + q) * n] : mk(0.0);
         }
         __syncthreads();
-        for (int col = tid; col < n; col += NT) col_solve_lower_unit(B + (size_t)col * n + j0, jb, s.T);
-        __syncthreads();
+        for (int col = first; col < n; col += step) col_solve_lower_unit(B + (size_t)col * n + j0, jb, s.T);
+        tm.sync();
         const int r0 = j0 + jb;
-        gemm_sub(B + r0, n, A + r0 + (size_t)j0 * n, n, B + j0, n, n - r0, n, jb, s);
+        update(B + r0, n, A + r0 + (size_t)j0 * n, n, B + j0, n, n - r0, n, jb, 0, s, tm);
+        if (tm.size > 1) tm.sync();
     }
     // backward: U X = Y, columns [0, j0+jb) of block row j0 only
     const int nblk = (n + NB - 1) / NB;
     for (int kb = nblk - 1; kb >= 0; --kb) {
         const int j0 = kb * NB, jb = min(NB, n - j0), ncol = j0 + jb;
-        for (int e = tid; e < NB * NB; e += NT) {
+        for (int e = tid; e < NB * NB; e += NTH) {
             int r = e % NB, q = e / NB;
-            s.T[r][q] = (r < jb && q < jb && q >= r) ? A[(j0 + r) + (size_t)(j0 + q) * n] : mk(r == q ? 1.0 : 0.0);
+            zc v = mk(r == q ? 1.0 : 0.0);
+            if (r < jb && q < jb && q >= r) {
+                v = A[(j0 + r) + (size_t)(j0 + q) * n];
+                if (q == r) v = 1.0 / v;
+            }
+            s.T[r][q] = v;
         }
         __syncthreads();
-        for (int col = tid; col < ncol; col += NT) col_solve_upper(B + (size_t)col * n + j0, jb, s.T);
-        __syncthreads();
+        for (int col = first; col < ncol; col += step) col_solve_upper(B + (size_t)col * n + j0, jb, s.T);
+        tm.sync();
         // Y[0:j0, 0:ncol] -= U[0:j0, j0:j0+jb] X[j0:j0+jb, 0:ncol]   (rows >= cols only)
-        gemm_sub(B, n, A + (size_t)j0 * n, n, B + j0, n, j0, ncol, jb, s, 1, 0, 0);
+        update(B, n, A + (size_t)j0 * n, n, B + j0, n, j0, ncol, jb, 1, s, tm);
+        if (tm.size > 1) tm.sync();
     }
     double tr = 0.0, ti = 0.0, z = 0.0;
-    for (int i = tid; i < n; i += NT) {
+    for (int i = tid; i < n; i += NTH) {
         zc v = B[i + (size_t)i * n];
         tr += v.re;
         ti += v.im;
@@ -359,8 +557,9 @@ static __device__ zc lu_trace_solve(const zc* __restrict__ A, zc* __restrict__ B
 // interchanges, then blocked forward and backward substitution; each block's
 // small triangle is solved by warp 0 (one row per lane), the rectangular
 // remainder by all threads (one row per thread, coalesced column reads).
-static __device__ void lu_solve_vec(const zc* __restrict__ A, zc* __restrict__ x, int n, const int* __restrict__ ipiv,
-                             LuSmem& s) {
+template <class S>
+static __device__ void lu_solve_vec(const zc* A, zc* x, int n, const int* ipiv,
+                             S& s) {
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid == 0)
@@ -380,7 +579,7 @@ static __device__ void lu_solve_vec(const zc* __restrict__ A, zc* __restrict__ x
             if (lane < jb) x[j0 + lane] = v;
         }
         __syncthreads();
-        for (int i = j0 + jb + tid; i < n; i += NT) {
+        for (int i = j0 + jb + tid; i < n; i += S::NTH) {
             zc acc = x[i];
             for (int q = 0; q < jb; ++q) acc -= A[i + (size_t)(j0 + q) * n] * x[j0 + q];
             x[i] = acc;
@@ -400,7 +599,7 @@ static __device__ void lu_solve_vec(const zc* __restrict__ A, zc* __restrict__ x
             if (lane < jb) x[j0 + lane] = v;
         }
         __syncthreads();
-        for (int i = tid; i < j0; i += NT) {
+        for (int i = tid; i < j0; i += S::NTH) {
             zc acc = x[i];
             for (int q = 0; q < jb; ++q) acc -= A[i + (size_t)(j0 + q) * n] * x[j0 + q];
             x[i] = acc;
@@ -438,13 +637,13 @@ __device__ __forceinline__ int k_regime(zc k, double r) {
 // and on return), then consecutive threads take consecutive list entries;
 // put(ii, jj, m, dm) receives each element.  Entries of a list are in no
 // fixed order, but every element is a function of (k, r) alone.
-template <class Put>
+template <int NTH, class Put>
 __device__ __forceinline__ void tile_pairs_grouped(int I, int J, int n, int d, const double* __restrict__ pos, zc k,
                                                    bool want_deriv, unsigned short* list, int* cnt, Put put) {
     const int tid = threadIdx.x;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int p = tid + NT * q, ii = p & 31, jj = p >> 5;
+    for (int q = 0; q < 1024 / NTH; ++q) {
+        const int p = tid + NTH * q, ii = p & 31, jj = p >> 5;
         const int i = I * 32 + ii, j = J * 32 + jj;
         if (i < n && j < n && i < j) {
             const int reg = k_regime(k, atom_distance(d, pos, i, j));
@@ -453,7 +652,7 @@ __device__ __forceinline__ void tile_pairs_grouped(int I, int J, int n, int d, c
     }
     __syncthreads();
     const int c0 = cnt[0], c1 = cnt[1], tot = c0 + c1 + cnt[2];
-    for (int w = tid; w < tot; w += NT) {
+    for (int w = tid; w < tot; w += NTH) {
         const int p = w < c0 ? list[w] : (w < c0 + c1 ? list[1024 + w - c0] : list[2048 + w - c0 - c1]);
         const int ii = p & 31, jj = p >> 5;
         zc m, dm = mk(0.0);
@@ -464,18 +663,36 @@ __device__ __forceinline__ void tile_pairs_grouped(int I, int J, int n, int d, c
     if (tid < 3) cnt[tid] = 0;
 }
 
+// The largest and the smallest non-zero max(|Re|, |Im|) of the entries a thread
+// has seen, as the high words of the doubles (which order like the values).
+struct EntryRange {
+    int hi = 0, lo = 0x7fffffff;
+    __device__ __forceinline__ void add(zc v) {
+        const int a = max(__double2hiint(v.re) & 0x7fffffff, __double2hiint(v.im) & 0x7fffffff);
+        hi = max(hi, a);
+        if (a > 0) lo = min(lo, a);
+    }
+};
+
 // Assemble M(k) into A and, if B != nullptr, dM/dk into B (ld n, column-major).
 // Tiles of 32 x 32 pairs above the diagonal are evaluated once and written to
-// both triangles, the mirrored tile through shared memory to keep stores coalesced.
+// both triangles, the mirrored tile through shared memory to keep stores
+// coalesced; a team deals the tiles round robin.
+template <class S, class Team>
 static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, int d, const double* __restrict__ pos,
-                         const msgpu_model& mdl, zc k, LuSmem& s) {
+                         const msgpu_model& mdl, zc k, S& s, const Team& tm, EntryRange& rg) {
+    constexpr int NTH = S::NTH, RQ = NTH / 32, NQ = 32 / RQ;  // tile rows per pass, passes
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        s.diag[0] = invf(mdl, d, k);
-        if (B) s.diag[1] = dk_invf(mdl, d, k);
-    }
+    // F^-1 and the two sides of its central difference (dk_invf), a long scalar
+    // FP64 chain each, by one thread of three warps
+    const double h = DK_INVF_STEP;
+    if (tid == 0) s.diag[0] = invf(mdl, d, k);
+    if (B && tid == 32) s.urow[0] = invf(mdl, d, k + h);
+    if (B && tid == 64) s.urow[1] = invf(mdl, d, k - h);
     __syncthreads();
-    const zc dg0 = s.diag[0], dg1 = s.diag[1];
+    const zc dg0 = s.diag[0], dg1 = B ? (s.urow[0] - s.urow[1]) / (2.0 * h) : mk(0.0);
+    rg.add(dg0);
+    if (B) rg.add(dg1);
     zc (*T2)[NB + 1] = reinterpret_cast<zc(*)[NB + 1]>(&s.As[0][0]);
     // d != 3: pair lists of the regime grouping in the (idle) U12 tile buffer
     unsigned short* list = reinterpret_cast<unsigned short*>(&s.Bs[0][0]);
@@ -484,16 +701,22 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
     if (grouped && tid < 3) cnt[tid] = 0;
     __syncthreads();
     const int nt = (n + 31) / 32;
+    int tile = 0;
     for (int J = 0; J < nt; ++J) {
         for (int I = 0; I <= J; ++I) {
+            if (tm.size > 1 && tile++ % tm.size != tm.rank) continue;
             if (grouped) {
-                tile_pairs_grouped(I, J, n, d, pos, k, B != nullptr, list, cnt, [&](int ii, int jj, zc m, zc dm) {
+                tile_pairs_grouped<NTH>(I, J, n, d, pos, k, B != nullptr, list, cnt, [&](int ii, int jj, zc m, zc dm) {
                     s.T[jj][ii] = m;
-                    if (B) T2[jj][ii] = dm;
+                    rg.add(m);
+                    if (B) {
+                        T2[jj][ii] = dm;
+                        rg.add(dm);
+                    }
                 });
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int ii = tid & 31, jj = (tid >> 5) + 8 * q;
+                for (int q = 0; q < NQ; ++q) {
+                    const int ii = tid & 31, jj = (tid >> 5) + RQ * q;
                     const int i = I * 32 + ii, j = J * 32 + jj;
                     if (i < n && j < n && i <= j) {
                         A[i + (size_t)j * n] = i < j ? s.T[jj][ii] : dg0;
@@ -502,8 +725,8 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
                 }
             } else {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int ii = tid & 31, jj = (tid >> 5) + 8 * q;
+            for (int q = 0; q < NQ; ++q) {
+                const int ii = tid & 31, jj = (tid >> 5) + RQ * q;
                 const int i = I * 32 + ii, j = J * 32 + jj;
                 if (i < n && j < n && i <= j) {
                     zc m, dm = mk(0.0);
@@ -515,7 +738,9 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
                     }
                     A[i + (size_t)j * n] = m;
                     s.T[jj][ii] = m;
+                    rg.add(m);
                     if (B) {
+                        rg.add(dm);
                         B[i + (size_t)j * n] = dm;
                         T2[jj][ii] = dm;
                     }
@@ -524,8 +749,8 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
             }
             __syncthreads();
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int jj = tid & 31, ii = (tid >> 5) + 8 * q;
+            for (int q = 0; q < NQ; ++q) {
+                const int jj = tid & 31, ii = (tid >> 5) + RQ * q;
                 const int i = I * 32 + ii, j = J * 32 + jj;
                 if (j < n && i < j) {
                     A[j + (size_t)i * n] = s.T[jj][ii];
@@ -535,6 +760,7 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
             __syncthreads();
         }
     }
+    if (tm.size > 1) tm.sync();
 }
 
 }  // namespace msg

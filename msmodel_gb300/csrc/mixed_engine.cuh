@@ -96,6 +96,7 @@ struct MixGemm {
 // of its job can need it) allocates only the four-slice part of the union and
 // leaves the rest of the SM's 256 KB of shared memory to the L1 cache.
 struct MixSmem {
+    static constexpr int NTH = NT;  // threads of the CTA (the block reductions of lu64.cuh)
     uint64_t bar_a, bar_b, bar_mma;
     uint32_t tmem;
     int err;
@@ -778,7 +779,7 @@ static __device__ __noinline__ float2 assemble_tile_grouped(float4* __restrict__
         df a = df_from_double(v.re), b = df_from_double(v.im);
         return make_float4(a.h, a.l, b.h, b.l);
     };
-    tile_pairs_grouped(I, J, n, d, pos, k, B != nullptr, s.u.p.list, s.u.p.cnt, [&](int ii, int jj, zc m, zc dm) {
+    tile_pairs_grouped<NT>(I, J, n, d, pos, k, B != nullptr, s.u.p.list, s.u.p.cnt, [&](int ii, int jj, zc m, zc dm) {
         const float4 fm = cvt(m);
         rg = entry_range(rg, fm);
         s.u.p.T[jj][ii] = fm;
