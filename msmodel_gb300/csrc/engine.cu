@@ -97,7 +97,7 @@ std::string g_err;
 int g_dev = -1;
 int g_sms = 0;
 int g_ctas_fp64 = 0;
-int g_teams[5] = {};  // FP64 kernel: clusters of 2^j CTAs the device holds at once
+int g_teams[2][5] = {};  // FP64 kernels (0: FP64 pipe, 1: tensor cores): clusters of 2^j CTAs the device holds at once
 std::atomic<uint64_t> g_launches{0};
 void* g_ws = nullptr;
 size_t g_ws_bytes = 0;
@@ -150,8 +150,12 @@ int init_locked(int device) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_engine_fp64, NT, smem_bytes()));
     g_ctas_fp64 = std::max(1, occ);
     CK(cudaFuncSetAttribute(k_engine_fp64, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    for (int j = 1; j < 5; ++j) g_teams[j] = max_teams(k_engine_fp64, 1 << j, NT, smem_bytes());
-    g_teams[0] = g_sms * g_ctas_fp64;
+    for (int j = 0; j < 5; ++j) {
+        g_teams[0][j] = max_teams(k_engine_fp64, 1 << j, NT, smem_bytes());
+        g_teams[1][j] = tc64_max_teams(1 << j);
+    }
+    g_teams[0][0] = g_sms * g_ctas_fp64;
+    g_teams[1][0] = g_sms;
     g_dev = device;
     return 0;
 }
@@ -190,16 +194,16 @@ static int ilog2(int v) {
 // takes a part s of its time in steps one CTA does (the panels) and 1 - s in
 // steps the team shares; the items go in waves of as many teams as the device
 // holds at once.
-static int pick_team(int nitem, int nmax) {
-    const double s = 0.3;
+static int pick_team(int tc, int nitem, int nmax) {
+    const double s = tc ? 0.2 : 0.3;
     int best = 1;
     double t_best = 0.0;
     for (int j = 0; j < 5; ++j) {
-        const int team = 1 << j, teams = g_teams[j];
+        const int team = 1 << j, teams = g_teams[tc][j];
         if (teams < 1 || (team > 1 && nmax < 16 * team)) break;
-        // CTAs that share an SM share its FP64 pipe
+        // CTAs of the FP64-pipe kernel that share an SM share its FP64 pipe
         const double waves = (nitem + teams - 1) / teams;
-        const double share = (double)std::min(nitem, teams) * team > g_sms ? 1.6 : 1.0;
+        const double share = (double)std::min(nitem, teams) * team > g_sms ? (tc ? 1.0 : 1.6) : 1.0;
         const double t = waves * share * (s + (1.0 - s) / team);
         if (j == 0 || t < 0.95 * t_best) {
             best = team;
@@ -232,7 +236,9 @@ struct msgpu_job {
     int* d_piv = nullptr;
     size_t slot = 0;
     size_t ws_bytes = 0;
+    bool tc = false;         // FP64: the kernel whose trailing updates run on the tensor cores
     int team = 1;            // FP64: CTAs that share one matrix
+    size_t img_off = 0;      // tc: offset of the operand images in the workspace
     long long amp_total = 0, amp_cap = 0;
     double* d_amps = nullptr;
     long long* d_amp_off = nullptr;
@@ -556,14 +562,18 @@ msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int n
     // per-CTA slots
     J->slot = (size_t)J->nmax * J->nmax;
     const bool fp64 = J->precision == MSGPU_FP64;
-    const size_t per_cta = slot_elems(kind, J->slot, J->nmax) * sizeof(zc);
+    J->tc = fp64 && J->nmax >= TC_NMIN;
+    const size_t slot_b = slot_elems(kind, J->slot, J->nmax) * sizeof(zc);
+    const size_t img_b = J->tc ? (tc64_image_bytes(J->nmax) + 127) / 128 * 128 : 0;
+    const size_t per_cta = slot_b + img_b;
     const int ctas = te.ctas ? std::min(te.ctas, g_ctas_fp64) : g_ctas_fp64;
-    if (fp64) J->team = pick_team(nitem, J->nmax);
-    int grid = std::min(nitem, J->team > 1 ? g_teams[ilog2(J->team)] : g_sms * ctas);
+    if (fp64) J->team = pick_team(J->tc ? 1 : 0, nitem, J->nmax);
+    int grid = std::min(nitem, J->team > 1 ? g_teams[J->tc][ilog2(J->team)] : J->tc ? g_sms : g_sms * ctas);
     size_t budget = ws_budget();
     while (grid > 1 && (size_t)grid * per_cta > budget) grid--;
     J->grid = grid;
-    J->ws_bytes = (size_t)grid * per_cta;
+    J->img_off = ((size_t)grid * slot_b + 127) / 128 * 128;
+    J->ws_bytes = J->img_off + (size_t)grid * img_b;
     if (cudaMalloc(&J->d_piv, sizeof(int) * (size_t)grid * J->nmax) != cudaSuccess) return fail("alloc piv");
     void* ws = nullptr;
     if (ensure_ws(J->ws_bytes, &ws)) {
@@ -612,7 +622,8 @@ static int launch_locked(msgpu_job* J, void* ws, cudaStream_t st) {
         if (e) return set_err(e, "mixed engine launch failed");
         return 0;
     }
-    const int e = launch_teams(k_engine_fp64, J->grid, J->team, NT, smem_bytes(), st, P);
+    const int e = J->tc ? tc64_run(P, J->grid, J->team, J->nmax, static_cast<unsigned char*>(ws) + J->img_off, st)
+                        : launch_teams(k_engine_fp64, J->grid, J->team, NT, smem_bytes(), st, P);
     if (e) return set_err(e, std::string("FP64 engine launch failed: ") + cudaGetErrorString(cudaGetLastError()));
     return 0;
 }

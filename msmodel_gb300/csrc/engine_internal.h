@@ -76,6 +76,18 @@ int max_teams(K kern, int team, int threads, size_t smem) {
     return n;
 }
 
+// FP64 engine with the trailing updates on the tensor cores (tc64.cu): `teams`
+// matrices at a time, `team` CTAs on each; img: teams x tc64_image_bytes(nmax)
+// rounded up to 128 bytes.
+int tc64_run(const EngineParams& P, int teams, int team, int nmax, void* img, cudaStream_t st);
+size_t tc64_image_bytes(int nmax);
+int tc64_max_teams(int team);
+// Rows from which an item's trailing updates run on the tensor cores.  Smaller items stay on the FP64 pipe: 912 ln det take 4.6 ms there against
+// 5.5 ms at n = 96, 8.6 against 7.0 at n = 112 (dlogf 11.4 against 9.9 and 20.0
+// against 12.7).  The rule looks at the item alone, so that no result depends
+// on the batch it is in.
+constexpr int TC_NMIN = 97;
+
 // Mixed-precision engine (mixed.cu).  Returns 0 when it ran the job, a
 // negative MSGPU_E* code on error.
 // d3only: every medium of the job has d = 3 (selects the d = 3 kernel instantiation);

@@ -1,4 +1,6 @@
-// fp64_engine.cuh -- the FP64 engine's work loop (k_engine_fp64, engine.cu).
+// fp64_engine.cuh -- the FP64 engine's work loop, shared by its two kernels:
+// k_engine_fp64 (engine.cu; every update on the FP64 pipe) and k_engine_tc64
+// (tc64.cu; trailing updates on the tensor cores).
 #pragma once
 #include "lu64.cuh"
 #include "engine_internal.h"

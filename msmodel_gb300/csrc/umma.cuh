@@ -162,6 +162,14 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
     for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 2 consecutive f32 columns of this thread's TMEM lane (32x32b shape, x2)
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, float& a, float& b) {
+    uint32_t r0, r1;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(taddr) : "memory");
+    a = __uint_as_float(r0);
+    b = __uint_as_float(r1);
+}
+
 // 8 consecutive f32 columns of this thread's TMEM lane (32x32b shape, x8)
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
     uint32_t r[8];
