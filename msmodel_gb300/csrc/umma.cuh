@@ -109,6 +109,36 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t
         : "memory");
 }
 
+// The same issued by a whole warp, one lane of which leads (lead != 0): the
+// branch around the MMAs is then uniform and their descriptors stay in uniform
+// registers (issued by one thread of a divergent branch, each MMA took ~84
+// cycles to set up, against ~16 of tensor-pipe time for 128 x 32 x 16).
+__device__ __forceinline__ void umma_bf16_lead(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc,
+                                               uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_lead(uint64_t* bar, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)),
+        "r"(lead)
+        : "memory");
+}
+
+// one lane of a converged warp
+__device__ __forceinline__ uint32_t elect_lane() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e;
+}
+
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                      smem_u32(bar))
