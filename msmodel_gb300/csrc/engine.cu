@@ -32,20 +32,6 @@ __global__ void __launch_bounds__(NT, 2) k_engine_fp64(EngineParams P) {
 __global__ void __launch_bounds__(NT, 1) k_build_matrix(zc* A, int n, int d, const double* pos, msgpu_model m,
                                                         double kre, double kim, int deriv);
 
-__global__ void __launch_bounds__(NT, 1) k_tracelog_matrix(zc* A, int n, int* ipiv, double* out, int* info) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    LuSmem& s = *reinterpret_cast<LuSmem*>(smem_raw);
-    if (threadIdx.x == 0) s.info = 0;
-    __syncthreads();
-    lu_factor(A, n, ipiv, false, s, Solo{}, DfmaUpdate{});
-    zc r = lu_tracelog(A, n, ipiv, s);
-    if (threadIdx.x == 0) {
-        out[0] = r.re;
-        out[1] = r.im;
-        *info = s.info;
-    }
-}
-
 // device special functions for the checks against the reference goldens (special.cu)
 __global__ void k_eval_special(int which, int d, msgpu_model m, int n, const double* ks, const double* rs,
                                double* out);
@@ -145,7 +131,6 @@ int init_locked(int device) {
     g_sms = pr.multiProcessorCount;
     CK(cudaFuncSetAttribute(k_engine_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()));
     CK(cudaFuncSetAttribute(k_build_matrix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()));
-    CK(cudaFuncSetAttribute(k_tracelog_matrix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()));
     int occ = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_engine_fp64, NT, smem_bytes()));
     g_ctas_fp64 = std::max(1, occ);
@@ -373,31 +358,6 @@ int msgpu_build_matrix(const msgpu_medium* med, const double* k, int deriv, doub
     return 0;
 }
 
-int msgpu_tracelog_matrix(int n, const double* mat, double* out, int* info) {
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (int e = init_locked(-1)) return e;
-    if (n < 1 || !mat || !out) return set_err(MSGPU_E_ARG, "bad argument");
-    zc* dA = nullptr;
-    int* dp = nullptr;
-    double* dout = nullptr;
-    CK(cudaMalloc(&dA, sizeof(zc) * (size_t)n * n));
-    CK(cudaMalloc(&dp, sizeof(int) * (size_t)n + 64));
-    CK(cudaMalloc(&dout, 64));
-    CK(cudaMemcpy(dA, mat, sizeof(zc) * (size_t)n * n, cudaMemcpyHostToDevice));
-    k_tracelog_matrix<<<1, NT, smem_bytes()>>>(dA, n, dp, dout, reinterpret_cast<int*>(dout + 2));
-    g_launches++;
-    CK(cudaGetLastError());
-    double h[3];
-    CK(cudaMemcpy(h, dout, sizeof(double) * 3, cudaMemcpyDeviceToHost));
-    out[0] = h[0];
-    out[1] = h[1];
-    if (info) std::memcpy(info, &h[2], sizeof(int));
-    cudaFree(dA);
-    cudaFree(dp);
-    cudaFree(dout);
-    return 0;
-}
-
 // Could the entries of M(k) (and of dM/dk for kind 1) of an item span more
 // than the mixed engine's four-slice budget?  For d = 3 and the "maximum"
 // model the moduli are known in closed form: off the diagonal
@@ -615,6 +575,8 @@ static int launch_locked(msgpu_job* J, void* ws, cudaStream_t st) {
     P.kind = J->kind;
     P.wide_ok = J->wide ? 1 : 0;
     P.warm = J->warm ? 1 : 0;
+    P.given_n = 0;
+    P.info = nullptr;
     P.amps = J->d_amps;
     P.amp_off = J->d_amp_off;
     if (J->precision == MSGPU_MIXED) {
@@ -625,6 +587,50 @@ static int launch_locked(msgpu_job* J, void* ws, cudaStream_t st) {
     const int e = J->tc ? tc64_run(P, J->grid, J->team, J->nmax, static_cast<unsigned char*>(ws) + J->img_off, st)
                         : launch_teams(k_engine_fp64, J->grid, J->team, NT, smem_bytes(), st, P);
     if (e) return set_err(e, std::string("FP64 engine launch failed: ") + cudaGetErrorString(cudaGetLastError()));
+    return 0;
+}
+
+// One matrix of the caller's through the FP64 engine: it goes straight into the
+// engine's slot and is shared by a cluster of CTAs (n = 300: one CTA took 14 ms).
+int msgpu_tracelog_matrix(int n, const double* mat, double* out, int* info) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (int e = init_locked(-1)) return e;
+    if (n < 1 || !mat || !out) return set_err(MSGPU_E_ARG, "bad argument");
+    const bool tc = n >= TC_NMIN;
+    const size_t mat_b = sizeof(zc) * (size_t)n * n, img_off = (mat_b + 127) / 128 * 128;
+    const size_t piv_off = img_off + (tc ? (tc64_image_bytes(n) + 127) / 128 * 128 : 0);
+    const size_t out_off = piv_off + (sizeof(int) * (size_t)n + 127) / 128 * 128;
+    void* ws = nullptr;
+    if (int e = ensure_ws(out_off + 256, &ws)) return e;
+    unsigned char* b = static_cast<unsigned char*>(ws);
+    // results and queue: {out[2], info, status}, then the counter words {0, 1}
+    const unsigned queue[2] = {0u, 1u};
+    CK(cudaMemcpy(b, mat, mat_b, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(b + out_off + 128, queue, sizeof(queue), cudaMemcpyHostToDevice));
+    EngineParams P{};
+    P.nitem = 1;
+    P.ws = reinterpret_cast<zc*>(ws);
+    P.slot = (size_t)n * n;
+    P.piv = reinterpret_cast<int*>(b + piv_off);
+    P.piv_stride = n;
+    P.out = reinterpret_cast<double*>(b + out_off);
+    P.info = reinterpret_cast<int*>(b + out_off + 16);
+    P.status = P.info + 1;
+    P.counter = reinterpret_cast<unsigned*>(b + out_off + 128);
+    P.given_n = n;
+    const int team = pick_team(tc ? 1 : 0, 1, n);
+    if (tc ? tc64_run(P, 1, team, n, b + img_off, nullptr)
+           : launch_teams(k_engine_fp64, 1, team, NT, smem_bytes(), (cudaStream_t) nullptr, P))
+        return set_err(MSGPU_E_CUDA, std::string("tracelog_matrix: ") + cudaGetErrorString(cudaGetLastError()));
+    g_launches++;
+    double h[3];
+    CK(cudaMemcpy(h, b + out_off, sizeof(h), cudaMemcpyDeviceToHost));
+    int st[2];
+    std::memcpy(st, &h[2], sizeof(st));
+    if (st[1] & MSGPU_S_TIMEOUT) return set_err(MSGPU_E_CUDA, "tracelog_matrix: a device wait ran out");
+    out[0] = h[0];
+    out[1] = h[1];
+    if (info) *info = st[0];
     return 0;
 }
 

@@ -31,6 +31,8 @@ struct EngineParams {
     double* amps;         // kinds 2, 4: a (or the eigenvector) per item (2 * n_i doubles each) or nullptr
     const long long* amp_off;  // kind 2: offset (in complex elements) of item i in amps
     int wide_ok;          // mixed engine: the launch has the shared memory for six-way slicing
+    int given_n;          // > 0: one item, the caller's matrix of given_n rows, already in the first slot
+    int* info;            // given matrix: 1-based index of the first zero pivot, or 0
     int warm;             // kind 4: start each inverse iteration from the item's vector in amps
 };
 

@@ -96,11 +96,19 @@ static __device__ void run_items_fp64(const EngineParams& P, S& s, const Cluster
         tm.sync();
         const int q = s.item;
         if (q >= P.nitem) break;
-        const int it = P.order[q];
-        const MedDev md = P.media[P.item_med[it]];
-        const zc k = mk(P.ks[2 * it], P.ks[2 * it + 1]);
+        int it = 0;
+        MedDev md{0, P.given_n, nullptr, {}};
+        zc k = mk(0.0);
         EntryRange rg;
-        assemble(A, P.kind == 1 ? B : nullptr, md.n, md.d, md.pos, md.model, k, s, tm, rg);
+        if (P.given_n > 0) {
+            const size_t nn = (size_t)md.n * md.n;
+            for (size_t e = (size_t)tm.rank * S::NTH + tid; e < nn; e += (size_t)tm.size * S::NTH) rg.add(A[e]);
+        } else {
+            it = P.order[q];
+            md = P.media[P.item_med[it]];
+            k = mk(P.ks[2 * it], P.ks[2 * it + 1]);
+            assemble(A, P.kind == 1 ? B : nullptr, md.n, md.d, md.pos, md.model, k, s, tm, rg);
+        }
         up.begin(rg, md.n, s, tm);
         zc res = mk(0.0);
         int conv = 1;
@@ -158,8 +166,9 @@ static __device__ void run_items_fp64(const EngineParams& P, S& s, const Cluster
             if (!isfinite(res.re) || !isfinite(res.im)) st |= MSGPU_S_NONFINITE;
             if (!conv) st |= MSGPU_S_NOCONV;
             P.status[it] = st;
+            if (P.given_n > 0) *P.info = s.info;
             // a run given up: every item not yet taken is marked, none keeps a stale result
-            if (bad)
+            if (bad && P.given_n <= 0)
                 for (unsigned u = atomicAdd(P.counter, 1u); u < P.counter[1] && (int)u < P.nitem;
                      u = atomicAdd(P.counter, 1u)) {
                     P.out[2 * P.order[u]] = P.out[2 * P.order[u] + 1] = nan("");

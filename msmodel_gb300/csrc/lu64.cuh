@@ -36,6 +36,11 @@ MSG_D zc zfms(zc a, zc l, zc u) {
     return a;
 }
 
+// a b with the products' roundings fixed, so that every inlined copy gives the same bits
+MSG_D zc zmulf(zc a, zc b) {
+    return mk(fma(a.re, b.re, -__dmul_rn(a.im, b.im)), fma(a.re, b.im, __dmul_rn(a.im, b.re)));
+}
+
 // The CTAs that factor one matrix together.  Solo: one CTA, the barrier is
 // __syncthreads.  ClusterTeam: the CTAs of a thread-block cluster; its barrier
 // (release / acquire at cluster scope) orders their global-memory accesses.
@@ -45,7 +50,7 @@ struct Solo {
 };
 // A batch that leaves SMs idle gives each matrix several CTAs: the 32 targets of
 // one resonance search at n = 100 take 45 ms against 83 ms with one CTA each
-// (the panel's share included), one dlogf at d = 2, n = 50 1.7 against 2.5 ms.
+// (FP64-pipe updates, panel included), one dlogf at d = 2, n = 50 1.7 against 2.5.
 struct ClusterTeam {
     int rank, size;
     __device__ __forceinline__ void sync() const {
@@ -145,30 +150,39 @@ MSG_D long long pivot_key(zc a) {
     return b > 0x7FF0000000000000LL ? -1LL : b;
 }
 
+// row of the warp's largest key, the smallest row on ties: three warp reductions
+__device__ __forceinline__ void warp_pivot(long long& key, int& row) {
+    const unsigned FULL = 0xffffffffu;
+    const int hi = (int)(key >> 32);
+    const int mh = __reduce_max_sync(FULL, hi);
+    const unsigned lo = hi == mh ? (unsigned)key : 0u;
+    const unsigned ml = __reduce_max_sync(FULL, lo);
+    row = __reduce_min_sync(FULL, hi == mh && lo == ml ? row : 0x7fffffff);
+    key = ((long long)mh << 32) | ml;
+}
+
 // row of the CTA's largest key (smallest row on ties), in every thread; one
 // barrier: the warps' candidates are double-buffered by `par`
 template <class S>
 __device__ __forceinline__ int block_pivot(long long key, int row, int par, S& s) {
     constexpr int NW = S::NTH / 32;
-    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const long long k2 = __shfl_xor_sync(FULL, key, off);
-        const int r2 = __shfl_xor_sync(FULL, row, off);
-        if (k2 > key || (k2 == key && r2 < row)) { key = k2; row = r2; }
-    }
+    warp_pivot(key, row);
     if (lane == 0) { s.red_k[par][warp] = key; s.red_p[par][warp] = row; }
     __syncthreads();
     key = s.red_k[par][lane & (NW - 1)];
     row = s.red_p[par][lane & (NW - 1)];
-#pragma unroll
-    for (int off = NW / 2; off > 0; off >>= 1) {
-        const long long k2 = __shfl_xor_sync(FULL, key, off);
-        const int r2 = __shfl_xor_sync(FULL, row, off);
-        if (k2 > key || (k2 == key && r2 < row)) { key = k2; row = r2; }
-    }
+    warp_pivot(key, row);
     return row;
+}
+
+// 1 / b by one reciprocal of |b|^2 where the squares stay well inside the
+// exponent range (one division on the panel's serial chain, zrecip has two)
+__device__ __forceinline__ zc pivot_recip(zc b) {
+    const int e = max(__double2hiint(b.re) & 0x7fffffff, __double2hiint(b.im) & 0x7fffffff) >> 20;
+    if (e < 1023 - 500 || e > 1023 + 500) return zrecip(b);
+    const double rd = 1.0 / fma(b.re, b.re, b.im * b.im);
+    return mk(b.re * rd, -b.im * rd);
 }
 
 // Factor the panel A[j0:n, j0:j0+jb) in place by one CTA; interchanges inside
@@ -180,7 +194,9 @@ __device__ __forceinline__ int block_pivot(long long key, int row, int par, S& s
 // one lane's work (256 threads each doing the hypot and the divisions held
 // the FP64 pipe, 2 lanes a clock, for ~10k cycles a column) and there are two
 // barriers.  4096 ln det at n = 64 (d = 3): 19.6 ms with the full-width rank-1
-// form and a reciprocal per thread, 11.6 ms now.
+// form and a reciprocal per thread; 11.6 ms with one reciprocal; 6.8 ms with the
+// columns of few rows spread over the warps, warp reductions in the pivot search
+// and the small update tiles (11k -> 6k cycles a column at n = 100).
 constexpr int SWP = 4;
 template <class S>
 static __device__ __noinline__ void panel_factor(zc* A, int n, int j0, int jb, int* ipiv, S& s) {
@@ -216,10 +232,12 @@ static __device__ __noinline__ void panel_factor(zc* A, int n, int j0, int jb, i
                 if (tid == c - j0) {
                     ipiv[c] = p;
                     if (!nz && s.info == 0) s.info = c + 1;
-                    const bool recip = nz && zabs(b) >= DBL_MIN;
+                    // |b| >= DBL_MIN, by the exponents where they decide it
+                    const int hb = max(__double2hiint(b.re) & 0x7fffffff, __double2hiint(b.im) & 0x7fffffff);
+                    const bool recip = nz && (hb >= 0x00100000 || zabs(b) >= DBL_MIN);
                     s.nz = nz ? (recip ? 1 : 2) : 0;
                     s.piv = b;
-                    s.rpiv = recip ? zrecip(b) : mk(0.0);
+                    s.rpiv = recip ? pivot_recip(b) : mk(0.0);
                 }
             }
             __syncthreads();
@@ -230,7 +248,7 @@ static __device__ __noinline__ void panel_factor(zc* A, int n, int j0, int jb, i
             if (nz) {
                 for (int i = c + 1 + tid; i < n; i += NTH) {
                     zc l = A[i + (size_t)c * n];
-                    l = nz == 1 ? l * r : l / s.piv;
+                    l = nz == 1 ? zmulf(l, r) : l / s.piv;
                     A[i + (size_t)c * n] = l;
                     if (c + 1 < sw) {
                         const zc a = zfms(A[i + (size_t)(c + 1) * n], l, s.urow[c + 1 - j0]);
@@ -272,23 +290,30 @@ static __device__ __noinline__ void panel_factor(zc* A, int n, int j0, int jb, i
             __syncthreads();
             bk = -1;
             bi = n;
-            for (int i = sw + tid; i < n; i += NTH) {
-                zc l[SWP];
+            // a warp takes 32 rows; where the rows do not fill the CTA several warps share
+            // them, each with every G-th column (a thread alone on a row would leave the
+            // other warps' share of the FP64 pipe idle for 28 columns)
+            const int nrb = (n - sw + 31) / 32, G = max(1, (NTH / 32) / max(nrb, 1));
+            const int g = nrb < NTH / 32 ? (tid >> 5) / nrb : 0;
+            const int i0 = sw + (nrb < NTH / 32 ? ((tid >> 5) % nrb) * 32 + (tid & 31) : tid);
+            if (g < G)
+                for (int i = i0; i < n; i += NTH) {
+                    zc l[SWP];
 #pragma unroll
-                for (int q = 0; q < SWP; ++q) l[q] = q < cw ? A[i + (size_t)(c0 + q) * n] : mk(0.0);
-                for (int t = 0; t < rem; ++t) {
-                    zc* q = A + i + (size_t)(sw + t) * n;
-                    zc a = *q;
+                    for (int q = 0; q < SWP; ++q) l[q] = q < cw ? A[i + (size_t)(c0 + q) * n] : mk(0.0);
+                    for (int t = g; t < rem; t += G) {
+                        zc* q = A + i + (size_t)(sw + t) * n;
+                        zc a = *q;
 #pragma unroll
-                    for (int e = 0; e < SWP; ++e)
-                        if (e < cw) a = zfms(a, l[e], s.T[e][t]);
-                    *q = a;
-                    if (t == 0) {
-                        const long long k = pivot_key(a);
-                        if (k > bk) { bk = k; bi = i; }
+                        for (int e = 0; e < SWP; ++e)
+                            if (e < cw) a = zfms(a, l[e], s.T[e][t]);
+                        *q = a;
+                        if (t == 0) {
+                            const long long k = pivot_key(a);
+                            if (k > bk) { bk = k; bi = i; }
+                        }
                     }
                 }
-            }
         }
     }
     __syncthreads();
@@ -326,7 +351,7 @@ __device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, cons
         zc y[CH];
 #pragma unroll
         for (int r = 0; r < CH; ++r) y[r] = (rb + r < jb) ? b[rb + r] : mk(0.0);
-        for (int q = rb + CH; q < jb; ++q) {
+        for (int q = jb - 1; q >= rb + CH; --q) {
             const zc xq = b[q];
 #pragma unroll
             for (int r = 0; r < CH; ++r) y[r] = zfms(y[r], T[rb + r][q], xq);
@@ -336,8 +361,9 @@ __device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, cons
             if (rb + r < jb) {
                 zc acc = y[r];
 #pragma unroll
-                for (int q = r + 1; q < CH; ++q) acc = zfms(acc, T[rb + r][rb + q], y[q]);
-                y[r] = acc * T[rb + r][rb + r];
+                for (int q = CH - 1; q > r; --q)
+                    if (rb + q < jb) acc = zfms(acc, T[rb + r][rb + q], y[q]);
+                y[r] = zmulf(acc, T[rb + r][rb + r]);
             }
         }
 #pragma unroll
@@ -346,12 +372,82 @@ __device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, cons
     }
 }
 
-// first column and stride of this thread when a team deals columns in blocks
-// of 32 (one per warp), CTA by CTA, so that few columns still spread over it
-template <class S, class Team>
-__device__ __forceinline__ void team_columns(const Team& tm, int& first, int& step) {
-    first = ((threadIdx.x >> 5) * tm.size + tm.rank) * 32 + (threadIdx.x & 31);
-    step = S::NTH * tm.size;
+// The same solves with one row a lane, for a warp per column: where a CTA has few
+// columns, one thread per column would put them on a warp or two, a quarter of
+// the FP64 pipe each, for jb^2/2 steps.  Every element takes its updates in the
+// order of the column solves, so the results are the same bits.
+__device__ __forceinline__ zc row_solve_lower_unit(zc x, int jb, const zc (*T)[NB + 1]) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    for (int q = 0; q + 1 < jb; ++q) {
+        const zc xq = mk(__shfl_sync(FULL, x.re, q), __shfl_sync(FULL, x.im, q));
+        if (lane > q && lane < jb) x = zfms(x, T[lane][q], xq);
+    }
+    return x;
+}
+__device__ __forceinline__ zc row_solve_upper(zc x, int jb, const zc (*T)[NB + 1]) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    for (int q = jb - 1; q >= 0; --q) {
+        if (lane == q) x = zmulf(x, T[q][q]);
+        const zc xq = mk(__shfl_sync(FULL, x.re, q), __shfl_sync(FULL, x.im, q));
+        if (lane < q) x = zfms(x, T[lane][q], xq);
+    }
+    return x;
+}
+
+// Columns go to the team in blocks of 32, block b to CTA b % size: the columns
+// of this CTA below ncol
+template <class Team>
+__device__ __forceinline__ int cta_columns(int ncol, const Team& tm) {
+    const int nb = (ncol + 31) / 32, mine = (nb - tm.rank + tm.size - 1) / tm.size;
+    return mine * 32;
+}
+// ... and the x-th of them (may be >= ncol in the last block)
+template <class Team>
+__device__ __forceinline__ int cta_column(int x, const Team& tm) { return ((x >> 5) * tm.size + tm.rank) * 32 + (x & 31); }
+// few columns: a warp for each column and a lane for each row is the faster solve
+// (~2k cycles a column on the whole SM, against ~127k for up to 128 columns with
+// a thread each: 166k -> 59k cycles a panel at n = 100)
+__device__ __forceinline__ bool few_columns(int cols) { return cols <= 64; }
+
+// The net effect of a panel's interchanges, worked out by every warp for
+// itself: row j0 + lane receives row `inner`, and row `orow` (-1: none), one of
+// the rows below the panel that took part, receives row `ocur`.  One load and
+// one store per moved row then replace the chain of up to 32 exchanges.
+__device__ __forceinline__ void panel_moves(const int* ipiv, int j0, int jb, int& inner, int& orow, int& ocur) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int pv = lane < jb ? ipiv[j0 + lane] : j0 + lane;
+    inner = j0 + lane;
+    orow = -1;
+    ocur = -1;
+    int used = 0;
+    for (int c = 0; c < jb; ++c) {
+        const int p = __shfl_sync(FULL, pv, c);
+        if (p == j0 + c) continue;
+        const int ic = __shfl_sync(FULL, inner, c);
+        if (p < j0 + jb) {
+            const int ip = __shfl_sync(FULL, inner, p - j0);
+            if (lane == c) inner = ip;
+            if (lane == p - j0) inner = ic;
+        } else {
+            const unsigned hit = __ballot_sync(FULL, orow == p);
+            const int u = hit ? __ffs(hit) - 1 : used++;
+            const int cur = hit ? __shfl_sync(FULL, ocur, u) : p;
+            if (lane == u) { orow = p; ocur = ic; }
+            if (lane == c) inner = cur;
+        }
+    }
+}
+
+template <class S>
+static __device__ void load_lower(const zc* A, int n, int j0, int jb, S& s) {
+    for (int e = threadIdx.x; e < NB * NB; e += S::NTH) {
+        int r = e % NB, q = e / NB;
+        s.T[r][q] = (r < jb && q < r) ? A[(j0 + r) + (size_t)(j0 + q) * n] : mk(0.0);
+    }
+    __syncthreads();
 }
 
 // Apply the panel's interchanges to every other column and compute
@@ -359,24 +455,45 @@ __device__ __forceinline__ void team_columns(const Team& tm, int& first, int& st
 // columns left of the panel alone: a ln det reads only U's diagonal and the
 // pivots afterwards.
 template <class S, class Team>
-static __device__ void panel_swaps_trsm(zc* A, int n, int j0, int jb, const int* ipiv, bool keep_l,
-                                        S& s, const Team& tm) {
-    for (int e = threadIdx.x; e < NB * NB; e += S::NTH) {
-        int r = e % NB, q = e / NB;
-        s.T[r][q] = (r < jb && q < r) ? A[(j0 + r) + (size_t)(j0 + q) * n] : mk(0.0);
-    }
-    __syncthreads();
-    int first, step;
-    team_columns<S>(tm, first, step);
-    const int base = keep_l ? 0 : j0 + jb;
-    for (int col = base + first; col < n; col += step) {
-        if (col >= j0 && col < j0 + jb) continue;
-        zc* a = A + (size_t)col * n;
-        for (int c = j0; c < j0 + jb; ++c) {
-            int p = ipiv[c];
-            if (p != c) { zc t = a[c]; a[c] = a[p]; a[p] = t; }
+static __device__ void panel_swaps_trsm(zc* A, int n, int j0, int jb, const int* ipiv, bool keep_l, S& s, const Team& tm) {
+    constexpr int NW = S::NTH / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    load_lower(A, n, j0, jb, s);
+    int inner, orow, ocur;
+    panel_moves(ipiv, j0, jb, inner, orow, ocur);
+    const bool moves = __any_sync(0xffffffffu, inner != j0 + lane);
+    const int right = j0 + jb, nr = cta_columns(n - right, tm);
+    const bool few = few_columns(nr);
+    if (keep_l && moves) {
+        const int nl = cta_columns(j0, tm);
+        for (int x = warp; x < nl; x += NW) {
+            const int col = cta_column(x, tm);
+            if (col >= j0) continue;
+            zc* a = A + (size_t)col * n;
+            const zc v = lane < jb ? a[inner] : mk(0.0), w = orow >= 0 ? a[ocur] : mk(0.0);
+            __syncwarp();
+            if (lane < jb) a[j0 + lane] = v;
+            if (orow >= 0) a[orow] = w;
         }
-        if (col >= j0 + jb) col_solve_lower_unit(a + j0, jb, s.T);
+    }
+    if (few || moves)
+        for (int x = warp; x < nr; x += NW) {
+            const int col = right + cta_column(x, tm);
+            if (col >= n) continue;
+            zc* a = A + (size_t)col * n;
+            zc v = lane < jb ? a[inner] : mk(0.0);
+            const zc w = orow >= 0 ? a[ocur] : mk(0.0);
+            __syncwarp();
+            if (few) v = row_solve_lower_unit(v, jb, s.T);
+            if (lane < jb) a[j0 + lane] = v;
+            if (orow >= 0) a[orow] = w;
+        }
+    if (!few) {
+        __syncthreads();
+        for (int x = tid; x < nr; x += S::NTH) {
+            const int col = right + cta_column(x, tm);
+            if (col < n) col_solve_lower_unit(A + (size_t)col * n + j0, jb, s.T);
+        }
     }
     tm.sync();
 }
@@ -384,10 +501,13 @@ static __device__ void panel_swaps_trsm(zc* A, int n, int j0, int jb, const int*
 // C[m x nn] -= Ablk[m x kk] * Bblk[kk x nn] (all column-major); kk <= NB.
 // tri != 0: only tiles that hold some element with row >= col are updated.
 // The team deals the tiles round robin; the caller's barrier ends the update.
-template <class S, class Team>
-static __device__ void gemm_sub(zc* C, int ldc, const zc* Ab, int lda, const zc* Bb,
-                         int ldb, int m, int nn, int kk, S& s, const Team& tm, int tri = 0) {
-    constexpr int NTH = S::NTH, TNC = S::TNC, CST = NTH / 16;
+// A thread holds R x R elements: R = 4 (64 x 64 tiles for 256 threads), or R = 2
+// for blocks of at most 32 rows or columns, most of whose larger tile would be
+// work on padding.
+template <int R, class S, class Team>
+static __device__ void gemm_sub_r(zc* C, int ldc, const zc* Ab, int lda, const zc* Bb,
+                           int ldb, int m, int nn, int kk, S& s, const Team& tm, int tri) {
+    constexpr int NTH = S::NTH, TM = 16 * R, TNC = NTH / 16 * R, CST = NTH / 16;
     if (m <= 0 || nn <= 0 || kk <= 0) return;
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
@@ -413,36 +533,43 @@ static __device__ void gemm_sub(zc* C, int ldc, const zc* Ab, int lda, const zc*
                 s.Bs[k][c] = v;
             }
             __syncthreads();
-            zc acc[4][4];
+            zc acc[R][R];
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < R; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
+                for (int b = 0; b < R; ++b) {
                     int r = ti + tx + 16 * a, c = tj + ty + CST * b;
                     acc[a][b] = (r < m && c < nn) ? C[r + (size_t)c * ldc] : mk(0.0);
                 }
 #pragma unroll 2
             for (int k = 0; k < kk; ++k) {
-                zc av[4], bw[4];
+                zc av[R], bw[R];
 #pragma unroll
-                for (int a = 0; a < 4; ++a) av[a] = s.As[k][tx + 16 * a];
+                for (int a = 0; a < R; ++a) av[a] = s.As[k][tx + 16 * a];
 #pragma unroll
-                for (int b = 0; b < 4; ++b) bw[b] = s.Bs[k][ty + CST * b];
+                for (int b = 0; b < R; ++b) bw[b] = s.Bs[k][ty + CST * b];
 #pragma unroll
-                for (int a = 0; a < 4; ++a)
+                for (int a = 0; a < R; ++a)
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) acc[a][b] = zfms(acc[a][b], av[a], bw[b]);
+                    for (int b = 0; b < R; ++b) acc[a][b] = zfms(acc[a][b], av[a], bw[b]);
             }
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < R; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
+                for (int b = 0; b < R; ++b) {
                     int r = ti + tx + 16 * a, c = tj + ty + CST * b;
                     if (r < m && c < nn) C[r + (size_t)c * ldc] = acc[a][b];
                 }
             __syncthreads();
         }
     }
+}
+
+template <class S, class Team>
+static __device__ void gemm_sub(zc* C, int ldc, const zc* Ab, int lda, const zc* Bb, int ldb, int m, int nn, int kk, S& s,
+                         const Team& tm, int tri = 0) {
+    if (m <= 32 || nn <= 32) gemm_sub_r<2>(C, ldc, Ab, lda, Bb, ldb, m, nn, kk, s, tm, tri);
+    else gemm_sub_r<4>(C, ldc, Ab, lda, Bb, ldb, m, nn, kk, s, tm, tri);
 }
 
 // the trailing update on the FP64 pipe (DFMA); another kernel may pass its own
@@ -497,27 +624,45 @@ static __device__ zc lu_tracelog(const zc* A, int n, const int* ipiv, S& s) {
 template <class S, class Team, class Update>
 static __device__ zc lu_trace_solve(const zc* A, zc* B, int n, const int* ipiv,
                              S& s, const Team& tm, const Update& update) {
-    constexpr int NTH = S::NTH;
-    const int tid = threadIdx.x;
-    int first, step;
-    team_columns<S>(tm, first, step);
-    for (int col = first; col < n; col += step) {
-        zc* b = B + (size_t)col * n;
-        for (int i = 0; i < n; ++i) {
-            int p = ipiv[i];
-            if (p != i) { zc t = b[i]; b[i] = b[p]; b[p] = t; }
+    constexpr int NTH = S::NTH, NW = NTH / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int mine = cta_columns(n, tm);
+    // P B: each warp takes its columns through every panel's interchanges
+    for (int j0 = 0; j0 < n; j0 += NB) {
+        const int jb = min(NB, n - j0);
+        int inner, orow, ocur;
+        panel_moves(ipiv, j0, jb, inner, orow, ocur);
+        if (!__any_sync(0xffffffffu, inner != j0 + lane)) continue;
+        for (int x = warp; x < mine; x += NW) {
+            const int col = cta_column(x, tm);
+            if (col >= n) continue;
+            zc* b = B + (size_t)col * n;
+            const zc v = lane < jb ? b[inner] : mk(0.0), w = orow >= 0 ? b[ocur] : mk(0.0);
+            __syncwarp();
+            if (lane < jb) b[j0 + lane] = v;
+            if (orow >= 0) b[orow] = w;
+            __syncwarp();
         }
     }
-    tm.sync();
+    __syncthreads();
     // forward: L X = P B
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
-        for (int e = tid; e < NB * NB; e += NTH) {
-            int r = e % NB, q = e / NB;
-            s.T[r][q] = (r < jb && q < r) ? A[(j0 + r) + (size_t)(j0 + q) * n] : mk(0.0);
+        load_lower(A, n, j0, jb, s);
+        if (few_columns(mine)) {
+            for (int x = warp; x < mine; x += NW) {
+                const int col = cta_column(x, tm);
+                if (col >= n) continue;
+                zc* b = B + (size_t)col * n + j0;
+                const zc v = row_solve_lower_unit(lane < jb ? b[lane] : mk(0.0), jb, s.T);
+                if (lane < jb) b[lane] = v;
+            }
+        } else {
+            for (int x = tid; x < mine; x += NTH) {
+                const int col = cta_column(x, tm);
+                if (col < n) col_solve_lower_unit(B + (size_t)col * n + j0, jb, s.T);
+            }
         }
-        __syncthreads();
-        for (int col = first; col < n; col += step) col_solve_lower_unit(B + (size_t)col * n + j0, jb, s.T);
         tm.sync();
         const int r0 = j0 + jb;
         update(B + r0, n, A + r0 + (size_t)j0 * n, n, B + j0, n, n - r0, n, jb, 0, s, tm);
@@ -537,7 +682,21 @@ static __device__ zc lu_trace_solve(const zc* A, zc* B, int n, const int* ipiv,
             s.T[r][q] = v;
         }
         __syncthreads();
-        for (int col = first; col < ncol; col += step) col_solve_upper(B + (size_t)col * n + j0, jb, s.T);
+        const int cols = cta_columns(ncol, tm);
+        if (few_columns(cols)) {
+            for (int x = warp; x < cols; x += NW) {
+                const int col = cta_column(x, tm);
+                if (col >= ncol) continue;
+                zc* b = B + (size_t)col * n + j0;
+                const zc v = row_solve_upper(lane < jb ? b[lane] : mk(0.0), jb, s.T);
+                if (lane < jb) b[lane] = v;
+            }
+        } else {
+            for (int x = tid; x < cols; x += NTH) {
+                const int col = cta_column(x, tm);
+                if (col < ncol) col_solve_upper(B + (size_t)col * n + j0, jb, s.T);
+            }
+        }
         tm.sync();
         // Y[0:j0, 0:ncol] -= U[0:j0, j0:j0+jb] X[j0:j0+jb, 0:ncol]   (rows >= cols only)
         update(B, n, A + (size_t)j0 * n, n, B + j0, n, j0, ncol, jb, 1, s, tm);

@@ -152,7 +152,7 @@ __device__ __forceinline__ int tc_row_exp(int e) { return e == 0x7ff ? TC_BAD : 
 struct TcState {
     uint8_t* img;      // the team's B image: ceil(nmax / 32) tiles of TC_BTILE
     uint32_t tmem;
-    uint32_t ph_b[2], ph_mma;
+    uint32_t ph_b, ph_mma;  // phases of bar_b (a bit each) and bar_mma
     bool use;          // the item's updates run on the tensor cores
 };
 
@@ -197,28 +197,30 @@ static __device__ void tc_slice_b(const zc* Bp, int ldb, int nn, int K, uint8_t*
     }
 }
 
-__device__ __forceinline__ void tc_issue_tile(uint32_t a0, uint32_t b0, uint64_t* bar, uint32_t tmem) {
+// the products of one tile, issued by warp 0 (lead: its elected lane)
+__device__ __forceinline__ void tc_issue_tile(uint32_t a0, uint32_t b0, uint64_t* bar, uint32_t tmem, uint32_t lead) {
     const uint32_t idp = idesc_bf16(TC_M, TC_N, false, false), idn = idesc_bf16(TC_M, TC_N, false, true);
-#pragma unroll 1
+    const uint64_t da0 = sdesc(a0, TC_M * 16, 128), db0 = sdesc(b0, TC_N * 16, 128);
+#pragma unroll
     for (int ks = 0; ks < 2; ++ks) {
-        const uint32_t ak = a0 + ks * (TC_M * 32), bk = b0 + ks * (TC_N * 32);
-        auto dA = [&](int i, int c) { return sdesc(ak + (2 * i + c) * TC_ASUB, TC_M * 16, 128); };
-        auto dB = [&](int j, int c) { return sdesc(bk + (2 * j + c) * TC_BSUB, TC_N * 16, 128); };
-#pragma unroll 1
+        // a descriptor's start address counts 16-byte units
+        auto dA = [&](int i, int c) { return da0 + (ks * (TC_M * 32) + (2 * i + c) * TC_ASUB) / 16; };
+        auto dB = [&](int j, int c) { return db0 + (ks * (TC_N * 32) + (2 * j + c) * TC_BSUB) / 16; };
+#pragma unroll
         for (int l = 0; l < TC_NS; ++l) {
             const uint32_t tre = tmem + 2 * TC_N * l, tim = tre + TC_N;
-#pragma unroll 1
+#pragma unroll
             for (int i = 0; i <= l; ++i) {
                 const int j = l - i;
                 const uint32_t acc = (ks == 0 && i == 0) ? 0u : 1u;
-                umma_bf16(tre, dA(i, 0), dB(j, 0), idp, acc);
-                umma_bf16(tre, dA(i, 1), dB(j, 1), idn, 1);
-                umma_bf16(tim, dA(i, 0), dB(j, 1), idp, acc);
-                umma_bf16(tim, dA(i, 1), dB(j, 0), idp, 1);
+                umma_bf16_lead(tre, dA(i, 0), dB(j, 0), idp, acc, lead);
+                umma_bf16_lead(tre, dA(i, 1), dB(j, 1), idn, 1, lead);
+                umma_bf16_lead(tim, dA(i, 0), dB(j, 1), idp, acc, lead);
+                umma_bf16_lead(tim, dA(i, 1), dB(j, 0), idp, 1, lead);
             }
         }
     }
-    umma_commit(bar);
+    umma_commit_lead(bar, lead);
 }
 
 // sum of the levels, weight 2^(39 - 9 l), in units of 2^-55 (rowmax x colmax scale)
@@ -236,12 +238,17 @@ __device__ __forceinline__ long long tc_levels(const float* L) {
     return v;
 }
 
-// c - v 2^xe
-__device__ __forceinline__ double tc_sub(double c, long long v, int xe) {
-    double d = __ll2double_rn(v);
-    int hi = __double2hiint(d);
-    if (v != 0) hi += xe << 20;
-    return c - __hiloint2double(hi, __double2loint(d));
+// v 2^xe, rounded to the nearest double (halves away from zero) in integer
+// arithmetic: a conversion instruction would take the FP64 pipe as long as the
+// one addition the update needs
+__device__ __forceinline__ double tc_double(long long v, int xe) {
+    unsigned long long u = v < 0 ? -v : v;
+    const int lz = __clzll(u);
+    u <<= lz & 63;
+    const int e = xe + 1023 + 63 - lz;
+    long long b = ((long long)(e - 1) << 52) + (long long)((u >> 11) + ((u >> 10) & 1));
+    if (e < 1 || v == 0) b = 0;  // nothing to subtract, or below the normal range
+    return __longlong_as_double(b | (v & (long long)0x8000000000000000ULL));
 }
 
 // C[m x nn] -= Ap[m x K] Bp[K x nn], all column-major; tri: only tiles holding
@@ -252,7 +259,10 @@ template <class Team>
 static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int lda, const zc* Bp,
                                  int ldb, int m, int nn, int K, int tri, Tc64Smem& s, Team tm, TcState& t) {
     if (m <= 0 || nn <= 0 || K <= 0) return;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform, so is the branch around the MMAs
+    const uint32_t tmem = __shfl_sync(0xffffffffu, t.tmem, 0);
+    uint32_t ph_b = t.ph_b;
     tc_slice_b(Bp, ldb, nn, K, t.img, tm);
     fence_proxy_async_all();
     tm.sync();
@@ -287,17 +297,18 @@ static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int 
             __syncthreads();
             band = bi;
         }
-        if (tid == 0) {
-            const bool ok = !s.err && mbar_wait(&s.bar_b[buf], t.ph_b[buf]);
-            if (!s.err) t.ph_b[buf] ^= 1;
-            if (ok) {
+        if (warp == 0) {
+            const bool ok = !s.err && mbar_wait(&s.bar_b[buf], (ph_b >> buf) & 1);
+            ph_b ^= 1u << buf;
+            if (__all_sync(0xffffffffu, ok)) {
                 tc_fence_after();
-                tc_issue_tile(smem_u32(s.g.a), smem_u32(s.g.b[buf]), &s.bar_mma, t.tmem);
-                if (todo > 1) load_b(buf ^ 1, bj2);
-            } else {
+                tc_issue_tile(smem_u32(s.g.a), smem_u32(s.g.b[buf]), &s.bar_mma, tmem, elect_lane());
+                if (lane == 0 && todo > 1) load_b(buf ^ 1, bj2);
+            } else if (lane == 0) {
                 s.err = 1;
                 mbar_arrive(&s.bar_mma);
             }
+            __syncwarp();
         }
         // this thread's row and 8 columns of C, on their way while the tensor core works
         const int row = bi * TC_M + rloc, col0 = bj * TC_N + 8 * cg;
@@ -318,7 +329,7 @@ static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int 
 #pragma unroll
         for (int j0 = 0; j0 < 8; j0 += 2) {
             float g[2][2 * TC_NS];
-            const uint32_t base = t.tmem + ((uint32_t)(32 * q) << 16) + 8 * cg + j0;
+            const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + 8 * cg + j0;
 #pragma unroll
             for (int a = 0; a < 2 * TC_NS; ++a) tmem_ld2(base + TC_N * a, g[0][a], g[1][a]);
             tmem_wait_ld();
@@ -337,8 +348,8 @@ static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int 
                     if (ea + eb[j0 + j] >= TC_BAD) {
                         c = mk(nan(""), nan(""));
                     } else {
-                        c.re = tc_sub(c.re, tc_levels(lr), xe);
-                        c.im = tc_sub(c.im, tc_levels(li), xe);
+                        c.re -= tc_double(tc_levels(lr), xe);
+                        c.im -= tc_double(tc_levels(li), xe);
                     }
                     cp[(size_t)(j0 + j) * ldc] = c;
                 }
@@ -351,9 +362,10 @@ static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int 
         bj = bj2;
         --todo;
     }
+    t.ph_b = ph_b;
     // a failed wait may leave a B copy in flight: let it land before the buffer changes hands
     if (s.err && tid == 0)
-        for (int b = 0; b < 2; ++b) mbar_wait(&s.bar_b[b], t.ph_b[b], 1 << 16);
+        for (int b = 0; b < 2; ++b) mbar_wait(&s.bar_b[b], (ph_b >> b) & 1, 1 << 16);
     __syncthreads();
 }
 
