@@ -145,17 +145,69 @@ int init_locked(int device) {
     return 0;
 }
 
+void pool_trim();
+
 int ensure_ws(size_t bytes, void** p) {
     if (bytes > g_ws_bytes) {
         if (g_ws) cudaFree(g_ws);
         g_ws = nullptr;
         g_ws_bytes = 0;
         ++g_ws_gen;
-        CK(cudaMalloc(&g_ws, bytes));
+        if (cudaMalloc(&g_ws, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            pool_trim();
+            CK(cudaMalloc(&g_ws, bytes));
+        }
         g_ws_bytes = bytes;
     }
     *p = g_ws;
     return 0;
+}
+
+// Device blocks of finished jobs, kept for the next ones: a job's arrays are one
+// block, and cudaMalloc / cudaFree of a dozen of them took 0.8 of the 1.4 ms of
+// a one-item call at n = 50.  At most POOL_BLOCKS blocks and POOL_BYTES in all;
+// a block goes back to the driver when the pool is full or an allocation fails.
+// Blocks change hands under g_mu, and only after the job's runs have completed.
+struct PoolBlock {
+    void* p;
+    size_t bytes;
+};
+constexpr size_t POOL_BLOCKS = 8, POOL_BYTES = (size_t)64 << 20;
+std::vector<PoolBlock> g_pool;
+
+void pool_trim() {
+    for (auto& b : g_pool) cudaFree(b.p);
+    g_pool.clear();
+}
+
+// a block of at least `bytes` (rounded up in place); nullptr if the device has none
+void* pool_get(size_t& bytes) {
+    size_t want = (size_t)64 << 10;
+    while (want < bytes && want < POOL_BYTES) want <<= 1;
+    if (want < bytes) want = bytes;
+    bytes = want;
+    for (size_t i = 0; i < g_pool.size(); ++i)
+        if (g_pool[i].bytes == want) {
+            void* p = g_pool[i].p;
+            g_pool.erase(g_pool.begin() + i);
+            return p;
+        }
+    void* p = nullptr;
+    if (cudaMalloc(&p, want) == cudaSuccess) return p;
+    cudaGetLastError();
+    pool_trim();
+    if (cudaMalloc(&p, want) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+
+void pool_put(void* p, size_t bytes) {
+    if (!p) return;
+    size_t held = bytes;
+    for (auto& b : g_pool) held += b.bytes;
+    if (g_pool.size() >= POOL_BLOCKS || held > POOL_BYTES) cudaFree(p);
+    else g_pool.push_back({p, bytes});
 }
 
 }  // namespace
@@ -210,8 +262,13 @@ struct msgpu_job {
     bool wide = false;       // some item may need six-way slicing (sticky: captured graphs keep it)
     bool warm = false;       // kind 4: inverse iterations start from the vectors set by msgpu_job_set_vectors
     bool d3only = true;      // every medium has d = 3
+    // the job's device arrays, all in one block
+    void* block = nullptr;
+    size_t block_bytes = 0;
+    bool ran = false;        // a run may still be on the device
     MedDev* d_media = nullptr;
     double* d_pos = nullptr;
+    size_t items_b = 0;      // bytes from d_ks to the live count: the item arrays at full capacity
     double* d_ks = nullptr;
     int* d_item_med = nullptr;
     int* d_order = nullptr;
@@ -413,21 +470,38 @@ static int set_items_locked(msgpu_job* J, int nitem, const int* item_med, const 
     std::vector<int> order(nitem);
     for (int i = 0; i < nitem; i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return J->med_n[med_of[a]] > J->med_n[med_of[b]]; });
-    CK(cudaMemcpy(J->d_ks, ks, sizeof(double) * 2 * nitem, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(J->d_item_med, med_of.data(), sizeof(int) * nitem, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(J->d_order, order.data(), sizeof(int) * nitem, cudaMemcpyHostToDevice));
-    if ((J->kind == 2 || J->kind == 4) && J->d_amp_off) {
-        std::vector<long long> off(nitem);
+    std::vector<long long> off;
+    if (J->d_amp_off) {
+        off.resize(nitem);
         long long acc = 0;
         for (int i = 0; i < nitem; i++) { off[i] = acc; acc += J->med_n[med_of[i]]; }
-        CK(cudaMemcpy(J->d_amp_off, off.data(), sizeof(long long) * nitem, cudaMemcpyHostToDevice));
     }
-    const unsigned live = (unsigned)nitem;
-    CK(cudaMemcpy(J->d_counter + 1, &live, sizeof(unsigned), cudaMemcpyHostToDevice));
+    const unsigned queue[2] = {0u, (unsigned)nitem};
+    // small jobs: the item arrays (and the queue words behind them) in one copy
+    std::vector<char> all(J->items_b <= ((size_t)64 << 10) ? J->items_b : 0);
+    auto put = [&](void* dst, const void* src, size_t bytes) -> bool {
+        if (bytes == 0) return true;
+        if (all.empty()) return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+        std::memcpy(all.data() + ((char*)dst - (char*)J->d_ks), src, bytes);
+        return true;
+    };
+    bool ok = put(J->d_ks, ks, sizeof(double) * 2 * nitem) && put(J->d_item_med, med_of.data(), sizeof(int) * nitem) &&
+              put(J->d_order, order.data(), sizeof(int) * nitem) &&
+              put(J->d_amp_off, off.data(), sizeof(long long) * off.size()) && put(J->d_counter, queue, sizeof(queue));
+    if (ok && !all.empty()) ok = cudaMemcpy(J->d_ks, all.data(), all.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+    if (!ok) return set_err(MSGPU_E_CUDA, std::string("job: copy of the items: ") + cudaGetErrorString(cudaGetLastError()));
     J->nitem = nitem;
     J->flops = flops;
     J->amp_total = amp_total;
     return 0;
+}
+
+static void destroy_locked(msgpu_job* J) {
+    if (J->gexec) cudaGraphExecDestroy(J->gexec);
+    if (J->cap_stream) cudaStreamDestroy(J->cap_stream);
+    if (J->ran) cudaDeviceSynchronize();  // the block may be another job's next
+    pool_put(J->block, J->block_bytes);
+    delete J;
 }
 
 msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int nitem, const int* item_med,
@@ -468,7 +542,7 @@ msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int n
     // pair-distance range of every d = 3 "maximum" medium (mixed jobs: the entry span of M(k))
     J->med_rmin.assign(nmed, -1.0);
     J->med_rmax.assign(nmed, -1.0);
-    if (J->precision == MSGPU_MIXED && kind <= 2)
+    if (J->precision == MSGPU_MIXED && (kind == 0 || kind == 2))  // dlogf jobs are wide whatever the span
         for (int i = 0; i < nmed; i++) {
             const msgpu_medium& m = media[i];
             if (m.d != 3 || m.model.type != MSGPU_MAXIMUM || m.n < 2) continue;
@@ -486,40 +560,10 @@ msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int n
         }
     auto fail = [&](const char* what) -> msgpu_job* {
         set_err(MSGPU_E_CUDA, std::string("job: ") + what);
-        msgpu_job_destroy(J);
+        destroy_locked(J);
         return nullptr;
     };
-    if (cudaMalloc(&J->d_media, sizeof(MedDev) * nmed) != cudaSuccess) return fail("alloc media");
-    if (cudaMalloc(&J->d_pos, sizeof(double) * npos) != cudaSuccess) return fail("alloc pos");
-    if (cudaMalloc(&J->d_ks, sizeof(double) * 2 * nitem) != cudaSuccess) return fail("alloc ks");
-    if (cudaMalloc(&J->d_item_med, sizeof(int) * nitem) != cudaSuccess) return fail("alloc items");
-    if (cudaMalloc(&J->d_order, sizeof(int) * nitem) != cudaSuccess) return fail("alloc order");
-    if (cudaMalloc(&J->d_out, sizeof(double) * 2 * nitem) != cudaSuccess) return fail("alloc out");
-    if (cudaMalloc(&J->d_status, sizeof(int) * nitem) != cudaSuccess) return fail("alloc status");
-    if (cudaMalloc(&J->d_counter, 256) != cudaSuccess) return fail("alloc counter");
-    if (cudaMemset(J->d_counter, 0, 256) != cudaSuccess) return fail("clear counter");
-    if (kind == 2 || kind == 4) {
-        // capacity for the amplitudes (eigenvectors) of nitem items of the largest medium
-        J->amp_cap = (long long)nitem * J->nmax;
-        if (cudaMalloc(&J->d_amps, sizeof(double) * 2 * (size_t)J->amp_cap) != cudaSuccess) return fail("alloc amps");
-        if (cudaMalloc(&J->d_amp_off, sizeof(long long) * nitem) != cudaSuccess) return fail("alloc amp_off");
-    }
-    size_t off = 0;
-    for (int i = 0; i < nmed; i++) {
-        const msgpu_medium& m = media[i];
-        size_t cnt = (size_t)m.n * m.d;
-        if (cudaMemcpy(J->d_pos + off, m.pos, sizeof(double) * cnt, cudaMemcpyHostToDevice) != cudaSuccess)
-            return fail("copy pos");
-        hm[i] = MedDev{m.d, m.n, J->d_pos + off, m.model};
-        off += cnt;
-    }
-    if (cudaMemcpy(J->d_media, hm.data(), sizeof(MedDev) * nmed, cudaMemcpyHostToDevice) != cudaSuccess)
-        return fail("copy media");
-    if (set_items_locked(J, nitem, item_med, ks)) {
-        msgpu_job_destroy(J);
-        return nullptr;
-    }
-    // per-CTA slots
+    // launch: the team, and as many slots as the device and the memory hold
     J->slot = (size_t)J->nmax * J->nmax;
     const bool fp64 = J->precision == MSGPU_FP64;
     J->tc = fp64 && J->nmax >= TC_NMIN;
@@ -529,15 +573,61 @@ msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int n
     const int ctas = te.ctas ? std::min(te.ctas, g_ctas_fp64) : g_ctas_fp64;
     if (fp64) J->team = pick_team(J->tc ? 1 : 0, nitem, J->nmax);
     int grid = std::min(nitem, J->team > 1 ? g_teams[J->tc][ilog2(J->team)] : J->tc ? g_sms : g_sms * ctas);
-    size_t budget = ws_budget();
-    while (grid > 1 && (size_t)grid * per_cta > budget) grid--;
+    if ((size_t)grid * per_cta + 128 > g_ws_bytes) {  // else the workspace that is there holds them
+        const size_t budget = ws_budget();
+        while (grid > 1 && (size_t)grid * per_cta > budget) grid--;
+    }
     J->grid = grid;
     J->img_off = ((size_t)grid * slot_b + 127) / 128 * 128;
     J->ws_bytes = J->img_off + (size_t)grid * img_b;
-    if (cudaMalloc(&J->d_piv, sizeof(int) * (size_t)grid * J->nmax) != cudaSuccess) return fail("alloc piv");
+    // one block: media, positions, then the item arrays, results, pivots, amplitudes
+    const bool vecs = kind == 2 || kind == 4;
+    if (vecs) J->amp_cap = (long long)nitem * J->nmax;  // nitem items of the largest medium
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at = (at + bytes + 255) / 256 * 256;
+        return o;
+    };
+    const size_t o_media = take(sizeof(MedDev) * nmed), o_pos = take(sizeof(double) * npos);
+    const size_t o_ks = take(sizeof(double) * 2 * nitem), o_med = take(sizeof(int) * nitem), o_order = take(sizeof(int) * nitem);
+    const size_t o_off = take(vecs ? sizeof(long long) * nitem : 0), o_counter = take(sizeof(unsigned) * 2);
+    const size_t o_out = take(sizeof(double) * 2 * nitem), o_status = take(sizeof(int) * nitem);
+    const size_t o_piv = take(sizeof(int) * (size_t)grid * J->nmax);
+    const size_t o_amps = take(vecs ? sizeof(double) * 2 * (size_t)J->amp_cap : 0);
+    J->block_bytes = at;
+    char* base = static_cast<char*>(J->block = pool_get(J->block_bytes));
+    if (!base) return fail("device allocation");
+    J->d_media = reinterpret_cast<MedDev*>(base + o_media);
+    J->d_pos = reinterpret_cast<double*>(base + o_pos);
+    J->d_ks = reinterpret_cast<double*>(base + o_ks);
+    J->d_item_med = reinterpret_cast<int*>(base + o_med);
+    J->d_order = reinterpret_cast<int*>(base + o_order);
+    J->d_amp_off = vecs ? reinterpret_cast<long long*>(base + o_off) : nullptr;
+    J->d_counter = reinterpret_cast<unsigned*>(base + o_counter);
+    J->items_b = o_counter + 2 * sizeof(unsigned) - o_ks;
+    J->d_out = reinterpret_cast<double*>(base + o_out);
+    J->d_status = reinterpret_cast<int*>(base + o_status);
+    J->d_piv = reinterpret_cast<int*>(base + o_piv);
+    J->d_amps = vecs ? reinterpret_cast<double*>(base + o_amps) : nullptr;
+    std::vector<char> head(o_ks);
+    size_t off = 0;
+    for (int i = 0; i < nmed; i++) {
+        const msgpu_medium& m = media[i];
+        const size_t cnt = (size_t)m.n * m.d;
+        std::memcpy(head.data() + o_pos + sizeof(double) * off, m.pos, sizeof(double) * cnt);
+        hm[i] = MedDev{m.d, m.n, J->d_pos + off, m.model};
+        off += cnt;
+    }
+    std::memcpy(head.data() + o_media, hm.data(), sizeof(MedDev) * nmed);
+    if (cudaMemcpy(base, head.data(), head.size(), cudaMemcpyHostToDevice) != cudaSuccess) return fail("copy media");
+    if (set_items_locked(J, nitem, item_med, ks)) {
+        destroy_locked(J);
+        return nullptr;
+    }
     void* ws = nullptr;
     if (ensure_ws(J->ws_bytes, &ws)) {
-        msgpu_job_destroy(J);
+        destroy_locked(J);
         return nullptr;
     }
     return J;
@@ -640,6 +730,7 @@ int msgpu_job_run(msgpu_job* J, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     void* ws = nullptr;
     if (int e = ensure_ws(J->ws_bytes, &ws)) return e;
+    J->ran = true;
     if (!J->use_graph) {
         if (int e = launch_locked(J, ws, st)) return e;
         g_launches++;
@@ -682,6 +773,7 @@ double msgpu_job_flops(const msgpu_job* J) { return J ? J->flops : 0.0; }
 int msgpu_job_results(msgpu_job* J, double* out, int* status) {
     if (!J) return set_err(MSGPU_E_ARG, "null job");
     CK(cudaDeviceSynchronize());
+    J->ran = false;
     if (out) CK(cudaMemcpy(out, J->d_out, sizeof(double) * 2 * J->nitem, cudaMemcpyDeviceToHost));
     if (status) CK(cudaMemcpy(status, J->d_status, sizeof(int) * J->nitem, cudaMemcpyDeviceToHost));
     return 0;
@@ -706,20 +798,8 @@ int msgpu_job_set_vectors(msgpu_job* J, const double* vecs) {
 
 void msgpu_job_destroy(msgpu_job* J) {
     if (!J) return;
-    if (J->gexec) cudaGraphExecDestroy(J->gexec);
-    if (J->cap_stream) cudaStreamDestroy(J->cap_stream);
-    cudaFree(J->d_media);
-    cudaFree(J->d_pos);
-    cudaFree(J->d_ks);
-    cudaFree(J->d_item_med);
-    cudaFree(J->d_order);
-    cudaFree(J->d_out);
-    cudaFree(J->d_status);
-    cudaFree(J->d_counter);
-    cudaFree(J->d_piv);
-    cudaFree(J->d_amps);
-    cudaFree(J->d_amp_off);
-    delete J;
+    std::lock_guard<std::mutex> lk(g_mu);
+    destroy_locked(J);
 }
 
 int msgpu_tune_set(int kind, int precision, int n, int engine, int ctas_per_sm) {
