@@ -30,8 +30,9 @@
 //    ~1.4e-9 of FP64, while at d = 2, Im k = -0.3, N = 2048 (span 2^19, the
 //    exponential growth e^{|Im k| r} over a disk of radius 25) they leave
 //    ~1e-5 and six slices are needed;
-//  * complex = 4 real products, Re uses the negate-B bit of the instruction
-//    descriptor; the accumulators use 2 NG TN TMEM columns (192 or 128);
+//  * complex = 3 MMAs: A_re (Re B, Im B) together, A_im Im B with the negate-B bit of
+//    the instruction descriptor, A_im Re B; the accumulators use 2 NG TN TMEM
+//    columns (192 or 128);
 //  * epilogue: C (double-float, global) -= 2^(ea+eb-16) (sum of the levels).
 // Operand slices are written to global images in the tensor core's
 // core-matrix layout and moved to shared memory by bulk copies (TMA engine).
@@ -62,8 +63,14 @@ template <int NS> struct SliceCfg;
 template <> struct SliceCfg<4> { static constexpr int TN = 32, NG = 3; };
 template <> struct SliceCfg<6> { static constexpr int TN = 16, NG = 4; };
 template <int NS> __host__ __device__ constexpr int a_band() { return 2 * NS * A_SUB; }  // NS slices x {Re, Im}
-template <int NS> __host__ __device__ constexpr int b_sub() { return SliceCfg<NS>::TN * NB * 2; }
-template <int NS> __host__ __device__ constexpr int b_band() { return 2 * NS * b_sub<NS>(); }
+// A B tile's operand rows, per slice: Re, Im of its columns, so that A_re times
+// (Re, Im) is one MMA of N = 2 TN: three MMAs a complex product.  304 ln det at
+// d = 2, n = 2048: 647 ms with four, 605 with three; 512 dlogf 10% less.  (A third block of
+// rows, -Im, makes it two, but the shared memory comes out of the L1 cache: 2% slower
+// at n = 64, and no room for two CTAs per SM with six slices.)
+template <int NS> __host__ __device__ constexpr int b_rows() { return 2 * SliceCfg<NS>::TN; }
+template <int NS> __host__ __device__ constexpr int b_sub() { return b_rows<NS>() * NB * 2; }
+template <int NS> __host__ __device__ constexpr int b_band() { return NS * b_sub<NS>(); }
 // shared-memory operand buffer: A band then B band (NS = 4: 64 + 16 KB; NS = 6: 96 + 12 KB)
 constexpr int GEMM_BYTES = a_band<6>() + b_band<6>() > a_band<4>() + b_band<4>() ? a_band<6>() + b_band<6>()
                                                                                    : a_band<4>() + b_band<4>();
@@ -181,17 +188,16 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// One operand row of K <= 32 complex values (stride `st` in float4) -> the
-// 2 NS sub-tiles (slice k, Re/Im) of a band of R rows, row r; exponent returned.
-template <int R, int NS>
-__device__ __forceinline__ int slice_operand_row(const float4* __restrict__ src, size_t st, int K, uint8_t* band, int r) {
+// One operand row of K <= 32 complex values (stride `st` in float4) -> put(slice,
+// 0 Re / 1 Im, first k, 8 bf16); exponent returned.
+template <int NS, class Put>
+__device__ __forceinline__ int slice_operand_row(const float4* __restrict__ src, size_t st, int K, Put put) {
     float mx = 0.0f;
     for (int kk = 0; kk < K; ++kk) {
         float4 v = src[kk * st];
         mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.z)));
     }
     const int e = row_exponent(mx);
-    constexpr int SUB = R * NB * 2;
     for (int kb = 0; kb < NB / 8; ++kb) {
         uint32_t w[2 * NS][4];
 #pragma unroll
@@ -215,10 +221,9 @@ __device__ __forceinline__ int slice_operand_row(const float4* __restrict__ src,
                 w[2 * sl + 1][q] = pack2(im[0][sl], im[1][sl]);
             }
         }
-        const uint32_t off = cm_offset(r, kb * 8, R);
 #pragma unroll
         for (int sub = 0; sub < 2 * NS; ++sub)
-            *reinterpret_cast<uint4*>(band + sub * SUB + off) = make_uint4(w[sub][0], w[sub][1], w[sub][2], w[sub][3]);
+            put(sub >> 1, sub & 1, kb * 8, make_uint4(w[sub][0], w[sub][1], w[sub][2], w[sub][3]));
     }
     return e;
 }
@@ -232,7 +237,9 @@ static __device__ void slice_panel_rows(const float4* __restrict__ P, int ld, in
         uint8_t* band = img + (size_t)(i / MT_M) * a_band<NS>();
         const int r = i % MT_M;
         if (i < m) {
-            ea[i] = ldexpf(1.0f, slice_operand_row<MT_M, NS>(P + i, (size_t)ld, K, band, r) - 8);
+            ea[i] = ldexpf(1.0f, slice_operand_row<NS>(P + i, (size_t)ld, K, [&](int sl, int c, int k, uint4 w) {
+                               *reinterpret_cast<uint4*>(band + (2 * sl + c) * A_SUB + cm_offset(r, k, MT_M)) = w;
+                           }) - 8);
         } else {
             ea[i] = 0.0f;
             for (int kb = 0; kb < NB / 8; ++kb)
@@ -250,14 +257,16 @@ static __device__ void slice_block_cols(const float4* __restrict__ Bp, int ld, i
     for (int j = threadIdx.x; j < np; j += NT) {
         uint8_t* band = img + (size_t)(j / TN) * b_band<NS>();
         const int r = j % TN;
+        auto put = [&](int sl, int c, int k, uint4 w) {
+            *reinterpret_cast<uint4*>(band + sl * b_sub<NS>() + cm_offset(c * TN + r, k, b_rows<NS>())) = w;
+        };
         if (j < nn) {
-            eb[j] = ldexpf(1.0f, slice_operand_row<TN, NS>(Bp + (size_t)j * ld, 1, K, band, r) - 8);
+            eb[j] = ldexpf(1.0f, slice_operand_row<NS>(Bp + (size_t)j * ld, 1, K, put) - 8);
         } else {
             eb[j] = 0.0f;
-            for (int kb = 0; kb < NB / 8; ++kb)
-                for (int sub = 0; sub < 2 * NS; ++sub)
-                    *reinterpret_cast<uint4*>(band + sub * b_sub<NS>() + cm_offset(r, kb * 8, TN)) =
-                        make_uint4(0, 0, 0, 0);
+            for (int k = 0; k < NB; k += 8)
+                for (int sl = 0; sl < NS; ++sl)
+                    for (int c = 0; c < 2; ++c) put(sl, c, k, make_uint4(0, 0, 0, 0));
         }
     }
 }
@@ -272,13 +281,13 @@ static __device__ void slice_block_cols(const float4* __restrict__ Bp, int ld, i
 // 512 dlogf of n = 100..600 55.5 against 62.1, 300 ln det at d = 3, n = 1024 10% less.
 template <int NS>
 __device__ __forceinline__ void issue_tile_mmas(uint32_t a0, uint32_t b0, uint64_t* bar, uint32_t tmem, uint32_t lead) {
-    constexpr int TN = SliceCfg<NS>::TN, NG = SliceCfg<NS>::NG, BSUB = b_sub<NS>();
-    const uint32_t idp = idesc_bf16(MT_M, TN, false, false), idn = idesc_bf16(MT_M, TN, false, true);
+    constexpr int TN = SliceCfg<NS>::TN, NG = SliceCfg<NS>::NG;
+    const uint32_t id2 = idesc_bf16(MT_M, 2 * TN), idp = idesc_bf16(MT_M, TN), idn = idesc_bf16(MT_M, TN, false, true);
     // core-matrix strides: K direction (LBO) R/8*128, row direction (SBO) 128; a K step of 16 is
     // R*32 bytes; a descriptor's start address counts 16-byte units
-    const uint64_t da0 = sdesc(a0, MT_M * 16, 128), db0 = sdesc(b0, TN * 16, 128);
+    const uint64_t da0 = sdesc(a0, MT_M * 16, 128), db0 = sdesc(b0, b_rows<NS>() * 16, 128);
     auto dA = [&](int k, int c, int ks) { return da0 + ((k * 2 + c) * A_SUB + ks * (MT_M * 32)) / 16; };
-    auto dB = [&](int k, int c, int ks) { return db0 + ((k * 2 + c) * BSUB + ks * (TN * 32)) / 16; };
+    auto dB = [&](int k, int row, int ks) { return db0 + (k * b_sub<NS>() + ks * (b_rows<NS>() * 32) + row * 16) / 16; };
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks) {
 #pragma unroll
@@ -289,9 +298,8 @@ __device__ __forceinline__ void issue_tile_mmas(uint32_t a0, uint32_t b0, uint64
                 const int j = l - i;
                 const uint32_t acc = (ks == 0 && i == 0 && l == g) ? 0u : 1u;  // first product of group g
                 const uint32_t tre = tmem + 2 * TN * g, tim = tre + TN;
-                umma_bf16_lead(tre, dA(i, 0, ks), dB(j, 0, ks), idp, acc, lead);
-                umma_bf16_lead(tre, dA(i, 1, ks), dB(j, 1, ks), idn, 1, lead);
-                umma_bf16_lead(tim, dA(i, 0, ks), dB(j, 1, ks), idp, acc, lead);
+                umma_bf16_lead(tre, dA(i, 0, ks), dB(j, 0, ks), id2, acc, lead);
+                umma_bf16_lead(tre, dA(i, 1, ks), dB(j, TN, ks), idn, 1, lead);
                 umma_bf16_lead(tim, dA(i, 1, ks), dB(j, 0, ks), idp, 1, lead);
             }
         }

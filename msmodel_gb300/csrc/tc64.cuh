@@ -23,7 +23,11 @@
 //
 // One CTA of 512 threads per SM: A band 128 rows x 32 (7 digits x Re/Im, 112 KB),
 // two B buffers of 32 columns (28 KB each), 7 levels x Re/Im x 32 = 448 TMEM
-// columns.  A is sliced straight into shared memory, B once per update into a
+// columns.  B's rows are stacked Re, Im, so that A_re times (Re, Im) is one MMA of
+// N = 64: three MMAs a complex product, 83 cycles for the wide and 57 for each
+// narrow one.  (A third block of rows, -Im, makes it two wide MMAs, but the 28 KB
+// it takes from the L1 cache cost the panel and the TRSM as much at n = 1024 and
+// 5% of the call at n = 100.)  A is sliced straight into shared memory, B once per update into a
 // global image that bulk copies (TMA engine) bring in a tile ahead.
 #pragma once
 #include <cuda_bf16.h>
@@ -38,9 +42,10 @@ constexpr int TC_M = 128;   // tile rows = TMEM lanes
 constexpr int TC_N = 32;    // tile columns
 constexpr int TC_NS = 7;    // digits = levels
 constexpr int TC_ASUB = TC_M * NB * 2;           // one digit of Re or Im of an A band: 8 KB
-constexpr int TC_BSUB = TC_N * NB * 2;           // the same of a B tile: 2 KB
+constexpr int TC_BROWS = 2 * TC_N;               // a B tile's operand rows: Re, Im of its columns
+constexpr int TC_BSUB = TC_BROWS * NB * 2;       // one digit of them: 4 KB
 constexpr int TC_ABAND = 2 * TC_NS * TC_ASUB;    // 112 KB
-constexpr int TC_BDIG = 2 * TC_NS * TC_BSUB;     // 28 KB
+constexpr int TC_BDIG = TC_NS * TC_BSUB;         // 28 KB
 constexpr int TC_BTILE = TC_BDIG + TC_N * 4;     // digits, then the columns' exponents
 constexpr uint32_t TC_TMEM = 512;
 // Items whose entries span more than 2^TC_SPAN_LOG2 stay on the FP64 pipe.  Up to
@@ -113,10 +118,9 @@ __device__ __forceinline__ uint32_t tc_pack(int a, int b) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// digits of 8 consecutive k of one row (all Re, then all Im) into a band of R
-// rows at core-matrix offset `off`
-template <int R>
-__device__ __forceinline__ void tc_store_digits(const zc* v, int E, uint8_t* band, uint32_t off) {
+// digits of 8 consecutive k of one row: put(digit, 0 Re / 1 Im, 8 bf16)
+template <class Put>
+__device__ __forceinline__ void tc_store_digits(const zc* v, int E, Put put) {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         long long x[8];
@@ -127,12 +131,10 @@ __device__ __forceinline__ void tc_store_digits(const zc* v, int E, uint8_t* ban
             int d[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) d[k] = tc_digit(x[k]);
-            *reinterpret_cast<uint4*>(band + (2 * s + c) * (R * NB * 2) + off) =
-                make_uint4(tc_pack(d[0], d[1]), tc_pack(d[2], d[3]), tc_pack(d[4], d[5]), tc_pack(d[6], d[7]));
+            put(s, c, make_uint4(tc_pack(d[0], d[1]), tc_pack(d[2], d[3]), tc_pack(d[4], d[5]), tc_pack(d[6], d[7])));
         }
-        *reinterpret_cast<uint4*>(band + c * (R * NB * 2) + off) =
-            make_uint4(tc_pack((int)x[0], (int)x[1]), tc_pack((int)x[2], (int)x[3]), tc_pack((int)x[4], (int)x[5]),
-                       tc_pack((int)x[6], (int)x[7]));
+        put(0, c, make_uint4(tc_pack((int)x[0], (int)x[1]), tc_pack((int)x[2], (int)x[3]), tc_pack((int)x[4], (int)x[5]),
+                             tc_pack((int)x[6], (int)x[7])));
     }
 }
 
@@ -171,7 +173,8 @@ static __device__ void tc_slice_a(const zc* Ap, int lda, int r0, int m, int K, T
     __syncthreads();
     const int E = tc_row_exp(s.emax[r]);
     if (kb == 0) s.ea[r] = E;
-    tc_store_digits<TC_M>(v, E, s.g.a, cm_offset(r, 8 * kb, TC_M));
+    uint8_t* dst = s.g.a + cm_offset(r, 8 * kb, TC_M);
+    tc_store_digits(v, E, [&](int d, int c, uint4 w) { *reinterpret_cast<uint4*>(dst + (2 * d + c) * TC_ASUB) = w; });
 }
 
 // B image: columns [0, nn) of the K x nn block, four threads a column
@@ -193,30 +196,29 @@ static __device__ void tc_slice_b(const zc* Bp, int ldb, int nn, int K, uint8_t*
         e = max(e, __shfl_xor_sync(grp, e, 2));
         const int E = tc_row_exp(e);
         if (kb == 0) *reinterpret_cast<int*>(tile + TC_BDIG + 4 * r) = E;
-        tc_store_digits<TC_N>(v, E, tile, cm_offset(r, 8 * kb, TC_N));
+        tc_store_digits(v, E, [&](int d, int c, uint4 w) {
+            *reinterpret_cast<uint4*>(tile + d * TC_BSUB + cm_offset(c * TC_N + r, 8 * kb, TC_BROWS)) = w;
+        });
     }
 }
 
 // the products of one tile, issued by warp 0 (lead: its elected lane)
 __device__ __forceinline__ void tc_issue_tile(uint32_t a0, uint32_t b0, uint64_t* bar, uint32_t tmem, uint32_t lead) {
-    const uint32_t idp = idesc_bf16(TC_M, TC_N, false, false), idn = idesc_bf16(TC_M, TC_N, false, true);
-    const uint64_t da0 = sdesc(a0, TC_M * 16, 128), db0 = sdesc(b0, TC_N * 16, 128);
+    const uint32_t id2 = idesc_bf16(TC_M, 2 * TC_N), idp = idesc_bf16(TC_M, TC_N), idn = idesc_bf16(TC_M, TC_N, false, true);
+    const uint64_t da0 = sdesc(a0, TC_M * 16, 128), db0 = sdesc(b0, TC_BROWS * 16, 128);
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks) {
-        // a descriptor's start address counts 16-byte units
+        // a descriptor's start address counts 16-byte units, a K step of 16 is two core-matrix columns
         auto dA = [&](int i, int c) { return da0 + (ks * (TC_M * 32) + (2 * i + c) * TC_ASUB) / 16; };
-        auto dB = [&](int j, int c) { return db0 + (ks * (TC_N * 32) + (2 * j + c) * TC_BSUB) / 16; };
+        auto dB = [&](int j, int row) { return db0 + (ks * (TC_BROWS * 32) + j * TC_BSUB + row * 16) / 16; };
 #pragma unroll
         for (int l = 0; l < TC_NS; ++l) {
-            const uint32_t tre = tmem + 2 * TC_N * l, tim = tre + TC_N;
+            const uint32_t t = tmem + 2 * TC_N * l;
 #pragma unroll
             for (int i = 0; i <= l; ++i) {
-                const int j = l - i;
-                const uint32_t acc = (ks == 0 && i == 0) ? 0u : 1u;
-                umma_bf16_lead(tre, dA(i, 0), dB(j, 0), idp, acc, lead);
-                umma_bf16_lead(tre, dA(i, 1), dB(j, 1), idn, 1, lead);
-                umma_bf16_lead(tim, dA(i, 0), dB(j, 1), idp, acc, lead);
-                umma_bf16_lead(tim, dA(i, 1), dB(j, 0), idp, 1, lead);
+                umma_bf16_lead(t, dA(i, 0), dB(l - i, 0), id2, (ks == 0 && i == 0) ? 0u : 1u, lead);
+                umma_bf16_lead(t, dA(i, 1), dB(l - i, TC_N), idn, 1, lead);
+                umma_bf16_lead(t + TC_N, dA(i, 1), dB(l - i, 0), idp, 1, lead);
             }
         }
     }
