@@ -71,7 +71,7 @@ def build(force=False, verbose=False):
         if force or _stale(out, [src] + deps):
             jobs.append((["gcc", "-O2", "-std=gnu11", "-fPIC", "-I", INC, "-c", src, "-o", out], out))
     if jobs:
-        with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
+        with cf.ThreadPoolExecutor(max_workers=min(os.cpu_count() or 8, len(jobs))) as ex:
             for out in ex.map(_compile, jobs):
                 if verbose:
                     print("built", out)

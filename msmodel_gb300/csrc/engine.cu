@@ -230,24 +230,24 @@ static int ilog2(int v) {
 // CTAs per matrix: the team size whose estimated time is least.  A matrix
 // takes a part s of its time in steps one CTA does (the panels) and 1 - s in
 // steps the team shares; the items go in waves of as many teams as the device
-// holds at once.
-static int pick_team(int tc, int nitem, int nmax) {
-    const double s = tc ? 0.2 : 0.3;
+// holds at once (teams[j] of 2^j CTAs), CTAs that share an SM `share` slower.
+static int pick_team(const int* teams, double s, double share, int nitem, int nmax) {
     int best = 1;
     double t_best = 0.0;
     for (int j = 0; j < 5; ++j) {
-        const int team = 1 << j, teams = g_teams[tc][j];
-        if (teams < 1 || (team > 1 && nmax < 16 * team)) break;
-        // CTAs of the FP64-pipe kernel that share an SM share its FP64 pipe
-        const double waves = (nitem + teams - 1) / teams;
-        const double share = (double)std::min(nitem, teams) * team > g_sms ? (tc ? 1.0 : 1.6) : 1.0;
-        const double t = waves * share * (s + (1.0 - s) / team);
+        const int team = 1 << j, held = teams[j];
+        if (held < 1 || (team > 1 && nmax < 16 * team)) break;
+        const double waves = (nitem + held - 1) / held;
+        const double t = waves * ((double)std::min(nitem, held) * team > g_sms ? share : 1.0) * (s + (1.0 - s) / team);
         if (j == 0 || t < 0.95 * t_best) {
             best = team;
             t_best = t;
         }
     }
     return best;
+}
+static int pick_team_fp64(bool tc, int nitem, int nmax) {
+    return pick_team(g_teams[tc], tc ? 0.2 : 0.3, tc ? 1.0 : 1.6, nitem, nmax);
 }
 
 struct msgpu_job {
@@ -279,7 +279,7 @@ struct msgpu_job {
     size_t slot = 0;
     size_t ws_bytes = 0;
     bool tc = false;         // FP64: the kernel whose trailing updates run on the tensor cores
-    int team = 1;            // FP64: CTAs that share one matrix
+    int team = 1;            // CTAs that share one matrix
     size_t img_off = 0;      // tc: offset of the operand images in the workspace
     long long amp_total = 0, amp_cap = 0;
     double* d_amps = nullptr;
@@ -571,8 +571,18 @@ msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int n
     const size_t img_b = J->tc ? (tc64_image_bytes(J->nmax) + 127) / 128 * 128 : 0;
     const size_t per_cta = slot_b + img_b;
     const int ctas = te.ctas ? std::min(te.ctas, g_ctas_fp64) : g_ctas_fp64;
-    if (fp64) J->team = pick_team(J->tc ? 1 : 0, nitem, J->nmax);
-    int grid = std::min(nitem, J->team > 1 ? g_teams[J->tc][ilog2(J->team)] : J->tc ? g_sms : g_sms * ctas);
+    int held = J->tc ? g_sms : g_sms * ctas;  // matrices on the device at once
+    if (fp64) {
+        J->team = pick_team_fp64(J->tc, nitem, J->nmax);
+        if (J->team > 1) held = g_teams[J->tc][ilog2(J->team)];
+    } else if (nitem < held && te.ctas == 0) {
+        // a mixed job may turn wide with later points: count the teams of the wide launch
+        int teams[5] = {held, 0, 0, 0, 0};
+        for (int j = 1; j < 5; ++j) teams[j] = mixed_max_teams(kind, J->d3only, 1 << j, true);
+        J->team = pick_team(teams, 0.25, 1.6, nitem, J->nmax);
+        held = teams[ilog2(J->team)];
+    }
+    int grid = std::min(nitem, held);
     if ((size_t)grid * per_cta + 128 > g_ws_bytes) {  // else the workspace that is there holds them
         const size_t budget = ws_budget();
         while (grid > 1 && (size_t)grid * per_cta > budget) grid--;
@@ -670,7 +680,7 @@ static int launch_locked(msgpu_job* J, void* ws, cudaStream_t st) {
     P.amps = J->d_amps;
     P.amp_off = J->d_amp_off;
     if (J->precision == MSGPU_MIXED) {
-        int e = mixed_run(P, J->grid, J->nmax, J->d3only, st);
+        int e = mixed_run(P, J->grid, J->team, J->nmax, J->d3only, st);
         if (e) return set_err(e, "mixed engine launch failed");
         return 0;
     }
@@ -708,7 +718,7 @@ int msgpu_tracelog_matrix(int n, const double* mat, double* out, int* info) {
     P.status = P.info + 1;
     P.counter = reinterpret_cast<unsigned*>(b + out_off + 128);
     P.given_n = n;
-    const int team = pick_team(tc ? 1 : 0, 1, n);
+    const int team = pick_team_fp64(tc, 1, n);
     if (tc ? tc64_run(P, 1, team, n, b + img_off, nullptr)
            : launch_teams(k_engine_fp64, 1, team, NT, smem_bytes(), (cudaStream_t) nullptr, P))
         return set_err(MSGPU_E_CUDA, std::string("tracelog_matrix: ") + cudaGetErrorString(cudaGetLastError()));

@@ -93,9 +93,12 @@ constexpr int TC_NMIN = 97;
 // Mixed-precision engine (mixed.cu).  Returns 0 when it ran the job, a
 // negative MSGPU_E* code on error.
 // d3only: every medium of the job has d = 3 (selects the d = 3 kernel instantiation);
-// P.wide_ok: launch with the shared memory for six-way slicing.
-int mixed_run(const EngineParams& P, int grid, int nmax, bool d3only, cudaStream_t st);
-// Allocates the mixed engine's scratch for `grid` CTAs and matrices up to nmax
+// P.wide_ok: launch with the shared memory for six-way slicing; grid matrices at a time,
+// `team` CTAs on each.
+int mixed_run(const EngineParams& P, int grid, int team, int nmax, bool d3only, cudaStream_t st);
+// clusters of `team` CTAs of that variant the device holds at once (0: none of that size)
+int mixed_max_teams(int kind, bool d3only, int team, bool wide);
+// Allocates the mixed engine's scratch for `grid` matrices up to nmax
 // (mixed_run does so itself; called before a stream capture, which must not allocate).
 int mixed_prepare(int grid, int nmax);
 // Changes whenever the mixed engine's scratch is reallocated (captured graphs hold its address).

@@ -75,6 +75,12 @@ __device__ __forceinline__ void cluster_store(int* p, int rank, int v) {
     asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void cluster_store(double* p, int rank, double v) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
 // shared memory of a CTA of NTH threads: NTH / 16 x 4 = TNC columns per DFMA tile
 template <int NTHREADS>
 struct __align__(16) LuSmemT {
@@ -721,10 +727,16 @@ static __device__ void lu_solve_vec(const zc* A, zc* x, int n, const int* ipiv,
                              S& s) {
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
-    if (tid == 0)
-        for (int i = 0; i < n; ++i) {
-            int p = ipiv[i];
-            if (p != i) { zc t = x[i]; x[i] = x[p]; x[p] = t; }
+    if (tid < 32)
+        for (int j0 = 0; j0 < n; j0 += NB) {
+            const int jb = min(NB, n - j0);
+            int inner, orow, ocur;
+            panel_moves(ipiv, j0, jb, inner, orow, ocur);
+            const zc v = lane < jb ? x[inner] : mk(0.0), w = orow >= 0 ? x[ocur] : mk(0.0);
+            __syncwarp();
+            if (lane < jb) x[j0 + lane] = v;
+            if (orow >= 0) x[orow] = w;
+            __syncwarp();
         }
     __syncthreads();
     for (int j0 = 0; j0 < n; j0 += NB) {

@@ -17,24 +17,20 @@ unsigned long long* g_stats = nullptr;
 int g_first_wait = WAIT_LIMIT;
 }  // namespace
 
-// the operand buffers need 16-byte alignment (no-swizzle layout); 128 is kept
-static size_t mixed_smem() { return MIX_SMEM_WIDE; }
-
-using Variant = int (*)(const EngineParams&, const MixScratch&, int, size_t, cudaStream_t, bool);
-const Variant kVariants[6] = {mixed_variant_0_d3, mixed_variant_1_d3, mixed_variant_2_d3,
-                              mixed_variant_0_any, mixed_variant_1_any, mixed_variant_2_any};
+using Variant = int (*)(const EngineParams&, const MixScratch&, const MixLaunch&);
+// kinds 0..2 for media all of d = 3, then for any dimension; one CTA per matrix, then clusters
+const Variant kVariants[2][6] = {{mixed_variant_0_d3, mixed_variant_1_d3, mixed_variant_2_d3, mixed_variant_0_any,
+                                  mixed_variant_1_any, mixed_variant_2_any},
+                                 {mixed_team_0_d3, mixed_team_1_d3, mixed_team_2_d3, mixed_team_0_any, mixed_team_1_any,
+                                  mixed_team_2_any}};
+static Variant variant(int kind, bool d3only, int team) {
+    return kVariants[team > 1][(d3only ? 0 : 3) + (kind < 0 ? 0 : kind > 2 ? 2 : kind)];
+}
 
 unsigned long long g_mix_gen = 1;
 
 // scratch layout for `grid` CTAs and matrices up to nmax; allocates when it grows
 static int prepare_locked(int grid, int nmax, MixScratch& X) {
-    static bool attr = false;
-    if (!attr) {
-        const int sm = (int)mixed_smem();
-        for (auto f : kVariants)
-            if (f(EngineParams{}, MixScratch{}, 0, (size_t)sm, nullptr, true)) return MSGPU_E_CUDA;
-        attr = true;
-    }
     // images sized for the larger of the two slice configurations
     const int nbA = (nmax + MT_M - 1) / MT_M, ncB = (nmax + 31) / 32 * 32;
     X.a_stride = (size_t)nbA * A_IMG_BAND;
@@ -78,15 +74,18 @@ unsigned long long mixed_generation() {
     return g_mix_gen;
 }
 
-int mixed_run(const EngineParams& P, int grid, int nmax, bool d3only, cudaStream_t st) {
+int mixed_max_teams(int kind, bool d3only, int team, bool wide) {
+    return variant(kind, d3only, team)(EngineParams{}, MixScratch{},
+                                       {0, team, wide ? MIX_SMEM_WIDE : MIX_SMEM_NARROW, nullptr, true});
+}
+
+int mixed_run(const EngineParams& P, int grid, int team, int nmax, bool d3only, cudaStream_t st) {
     std::lock_guard<std::mutex> lk(g_mx);
     MixScratch X;
     if (int e = prepare_locked(grid, nmax, X)) return e;
     if (X.stats) cudaMemsetAsync(X.stats, 0, sizeof(unsigned long long) * PH_N, st);
     if (cudaMemsetAsync(P.counter, 0, sizeof(unsigned), st) != cudaSuccess) return MSGPU_E_CUDA;
-    // variants: kinds 0..2 for media all of d = 3, then for any dimension
-    const int v = (d3only ? 0 : 3) + (P.kind < 0 ? 0 : P.kind > 2 ? 2 : P.kind);
-    return kVariants[v](P, X, grid, P.wide_ok ? MIX_SMEM_WIDE : MIX_SMEM_NARROW, st, false);
+    return variant(P.kind, d3only, team)(P, X, {grid, team, P.wide_ok ? MIX_SMEM_WIDE : MIX_SMEM_NARROW, st, false});
 }
 
 int mixed_stats(double* out, int n) {

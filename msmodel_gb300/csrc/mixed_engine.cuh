@@ -108,10 +108,15 @@ struct MixSmem {
     uint32_t tmem;
     int err;
     int mma_stuck;        // an MMA completion wait ran out: 1 + the parity it waited on
-    zc diag[2];
+    zc diag[3];
     double red_v[NT / 32];
     int red_i[NT / 32];
-    float red_f[NT / 32];
+    int red_k[2][NT / 32], red_p[2][NT / 32];
+    float4 rpiv;          // reciprocal of the panel's pivot
+    int nz;
+    int rng[2];           // the item's entry range, this CTA's part (float bits), and every CTA's of the team
+    int team_rng[16][2];
+    double team_max[16];
     double red_s[3][NT / 32];
     int info, bcast_i, item;
     unsigned long long stat[PH_N];
@@ -119,13 +124,13 @@ struct MixSmem {
     union alignas(128) {
         MixGemm g;
         MixPanel p;
+        LuSmem lu;  // the FP64 assembly of the refinement's copy of M
     } u;
 };
 // dynamic shared memory of a launch with and without room for six slices
 constexpr size_t MIX_SMEM_WIDE = sizeof(MixSmem) + 128;
 constexpr size_t MIX_SMEM_NARROW =
-    offsetof(MixSmem, u) + (sizeof(MixPanel) > (size_t)(a_band<4>() + b_band<4>()) ? sizeof(MixPanel)
-                                                                                     : (size_t)(a_band<4>() + b_band<4>())) + 128;
+    offsetof(MixSmem, u) + std::max({(size_t)(a_band<4>() + b_band<4>()), sizeof(MixPanel), sizeof(LuSmem)}) + 128;
 
 __device__ __forceinline__ void stat_start(MixSmem& s) {
     if (threadIdx.x == 0) s.t0 = clock64();
@@ -191,7 +196,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // One operand row of K <= 32 complex values (stride `st` in float4) -> put(slice,
 // 0 Re / 1 Im, first k, 8 bf16); exponent returned.
 template <int NS, class Put>
-__device__ __forceinline__ int slice_operand_row(const float4* __restrict__ src, size_t st, int K, Put put) {
+__device__ __forceinline__ int slice_operand_row(const float4* src, size_t st, int K, Put put) {
     float mx = 0.0f;
     for (int kk = 0; kk < K; ++kk) {
         float4 v = src[kk * st];
@@ -230,10 +235,10 @@ __device__ __forceinline__ int slice_operand_row(const float4* __restrict__ src,
 
 // A operand: rows [0, m) of the m x K panel P (column-major, ld), all bands;
 // ea[i] = 2^(e_i - 8), the row's scale
-template <int NS>
-static __device__ void slice_panel_rows(const float4* __restrict__ P, int ld, int m, int K, uint8_t* img, float* ea) {
+template <int NS, class Team>
+static __device__ void slice_panel_rows(const float4* P, int ld, int m, int K, uint8_t* img, float* ea, const Team& tm) {
     const int mp = (m + MT_M - 1) / MT_M * MT_M;
-    for (int i = threadIdx.x; i < mp; i += NT) {
+    for (int i = tm.rank * NT + threadIdx.x; i < mp; i += NT * tm.size) {
         uint8_t* band = img + (size_t)(i / MT_M) * a_band<NS>();
         const int r = i % MT_M;
         if (i < m) {
@@ -250,11 +255,11 @@ static __device__ void slice_panel_rows(const float4* __restrict__ P, int ld, in
 }
 
 // B operand: columns [0, nn) of the K x nn block Bp (column-major, ld); eb[j] = 2^(e_j - 8)
-template <int NS>
-static __device__ void slice_block_cols(const float4* __restrict__ Bp, int ld, int nn, int K, uint8_t* img, float* eb) {
+template <int NS, class Team>
+static __device__ void slice_block_cols(const float4* Bp, int ld, int nn, int K, uint8_t* img, float* eb, const Team& tm) {
     constexpr int TN = SliceCfg<NS>::TN;
     const int np = (nn + TN - 1) / TN * TN;
-    for (int j = threadIdx.x; j < np; j += NT) {
+    for (int j = tm.rank * NT + threadIdx.x; j < np; j += NT * tm.size) {
         uint8_t* band = img + (size_t)(j / TN) * b_band<NS>();
         const int r = j % TN;
         auto put = [&](int sl, int c, int k, uint4 w) {
@@ -324,54 +329,60 @@ __device__ __forceinline__ df df_sub_levels(df c, const float* lv) {
 }
 
 // C[m x nn] -= Ap[m x K] * Bp[K x nn]; all double-float complex, column-major.
-// tri != 0: only tiles holding an element with row >= column are updated.
-// Returns false if a wait timed out (the engine then stops).
-template <int NS>
-static __device__ bool mixed_gemm_sub(float4* __restrict__ C, int ldc, const float4* __restrict__ Ap, int lda,
-                               const float4* __restrict__ Bp, int ldb, int m, int nn, int K, int tri, MixSmem& s,
-                               const MixScratch& X, uint32_t tmem, Phases& ph) {
+// tri != 0: only tiles holding an element with row >= column are updated.  The
+// team slices the operands together and deals out the tiles in row-band order,
+// in contiguous runs.  A wait that ran out sets s.err: the CTA then issues no
+// more copies or MMAs but keeps to the barriers, and its items are marked.
+template <int NS, class Team>
+static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const float4* Ap, int lda, const float4* Bp, int ldb,
+                               int m, int nn, int K, int tri, MixSmem& s, const MixScratch& X, uint32_t tmem, Phases& ph,
+                               const Team& tm) {
     constexpr int TN = SliceCfg<NS>::TN, NG = SliceCfg<NS>::NG, AB = a_band<NS>(), BB = b_band<NS>();
     constexpr int CW = TN / 2;  // columns of a tile per thread (two warps per TMEM lane quadrant)
-    if (m <= 0 || nn <= 0 || K <= 0) return true;
+    if (m <= 0 || nn <= 0 || K <= 0) return;
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform, so is the branch around the MMAs
-    uint8_t* imgA = X.imgA + (size_t)blockIdx.x * X.a_stride;
-    uint8_t* imgB = X.imgB + (size_t)blockIdx.x * X.b_stride;
-    float* gea = X.ea + (size_t)blockIdx.x * X.e_stride;
-    float* geb = X.eb + (size_t)blockIdx.x * X.e_stride;
+    const size_t team = blockIdx.x / tm.size;
+    uint8_t* imgA = X.imgA + team * X.a_stride;
+    uint8_t* imgB = X.imgB + team * X.b_stride;
+    float* gea = X.ea + team * X.e_stride;
+    float* geb = X.eb + team * X.e_stride;
     uint8_t* sA = s.u.g.buf;
     uint8_t* sB = s.u.g.buf + AB;
     stat_start(s);
-    slice_panel_rows<NS>(Ap, lda, m, K, imgA, gea);
-    slice_block_cols<NS>(Bp, ldb, nn, K, imgB, geb);
+    slice_panel_rows<NS>(Ap, lda, m, K, imgA, gea, tm);
+    slice_block_cols<NS>(Bp, ldb, nn, K, imgB, geb, tm);
     fence_proxy_async_all();
-    __syncthreads();
+    tm.sync();
+    if (tm.size > 1) fence_proxy_async_all();
     stat_add(s, PH_SLICE);
     const int nbi = (m + MT_M - 1) / MT_M, nbj = (nn + TN - 1) / TN;
-    // tile list in row-band order, skipping tiles wholly above the diagonal when tri
-    auto tile_ok = [&](int bi, int bj) { return !tri || bi * MT_M + MT_M - 1 >= bj * TN; };
-    auto next_tile = [&](int& bi, int& bj) {
-        do {
-            if (++bj >= nbj) { bj = 0; ++bi; }
-        } while (bi < nbi && !tile_ok(bi, bj));
-    };
+    // tile list in row-band order: band bi holds the tiles of columns [0, width(bi))
+    auto width = [&](int bi) { return tri ? min(nbj, (bi * MT_M + MT_M - 1) / TN + 1) : nbj; };
+    int todo = 0;
+    for (int b = 0; b < nbi; ++b) todo += width(b);
     int bi = 0, bj = 0;
-    if (!tile_ok(bi, bj)) next_tile(bi, bj);
-    if (bi >= nbi) return true;
-    if (tid == 0) {
+    if (tm.size > 1) {
+        const int total = todo;
+        bj = (int)((long long)total * tm.rank / tm.size);
+        todo = (int)((long long)total * (tm.rank + 1) / tm.size) - bj;
+        while (bi < nbi && bj >= width(bi)) bj -= width(bi++);
+    }
+    bool pend = todo > 0 && !s.err;  // warp 0: this tile's operand copies were issued
+    pend = __shfl_sync(0xffffffffu, pend, 0);
+    if (tid == 0 && pend) {
         mbar_arrive_expect_tx(&s.bar_a, AB);
         bulk_g2s(sA, imgA + (size_t)bi * AB, AB / 2, &s.bar_a);
         bulk_g2s(sA + AB / 2, imgA + (size_t)bi * AB + AB / 2, AB / 2, &s.bar_a);
         mbar_arrive_expect_tx(&s.bar_b, BB);
         bulk_g2s(sB, imgB + (size_t)bj * BB, BB, &s.bar_b);
     }
-    bool ok = true;
     bool new_band = true, first = true;
     const int q = warp & 3, hcol = warp >> 2;  // TMEM lane quadrant, column half of this warp
     const int rloc = 32 * q + lane;
-    while (bi < nbi) {
-        int nbi2 = bi, nbj2 = bj;
-        next_tile(nbi2, nbj2);
+    while (todo > 0) {
+        int nbi2 = bi, nbj2 = bj + 1;
+        if (nbj2 >= width(bi)) { nbj2 = 0; ++nbi2; }
         // this thread's row and CW columns of C, and its row scale, fetched before
         // the MMAs complete so the memory latency hides behind the tensor core
         const int row = bi * MT_M + rloc;
@@ -384,20 +395,22 @@ static __device__ bool mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
             cpre[j] = (row_ok && col < nn) ? C[row + (size_t)col * ldc] : make_float4(0, 0, 0, 0);
         }
         if (warp == 0) {
-            bool w = true;
-            if (new_band) {
-                w = mbar_wait(&s.bar_a, ph.a, first ? X.first_wait : WAIT_LIMIT);
-                if (!w) mbar_wait(&s.bar_a, ph.a);  // let the copy in flight land before moving on
-                ph.a ^= 1;
+            bool ok = pend;
+            if (pend) {
+                if (new_band) {
+                    ok = mbar_wait(&s.bar_a, ph.a, first ? X.first_wait : WAIT_LIMIT);
+                    if (!ok) mbar_wait(&s.bar_a, ph.a);  // let the copy in flight land before moving on
+                    ph.a ^= 1;
+                }
+                ok = mbar_wait(&s.bar_b, ph.b) && ok;
+                ph.b ^= 1;
             }
-            const bool wb = mbar_wait(&s.bar_b, ph.b);
-            ph.b ^= 1;
-            if (__all_sync(0xffffffffu, w && wb)) {
+            if (__all_sync(0xffffffffu, ok)) {
                 tc_fence_after();
                 issue_tile_mmas<NS>(smem_u32(sA), smem_u32(sB), &s.bar_mma, tmem, elect_lane());
             } else if (lane == 0) {
-                s.err = 1;                // operands missing: no MMA is issued, the CTA stops
-                mbar_arrive(&s.bar_mma);  // after this tile; release its MMA wait at once
+                s.err = 1;                // operands missing: no MMA is issued;
+                mbar_arrive(&s.bar_mma);  // release this tile's MMA wait at once
             }
             __syncwarp();
         }
@@ -409,14 +422,17 @@ static __device__ bool mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
         }
         ph.mma ^= 1;
         // operands of the next tile: smem is free once the MMAs completed (none after a failed wait)
-        if (tid == 0 && nbi2 < nbi && !s.err) {
-            if (nbi2 != bi) {
-                mbar_arrive_expect_tx(&s.bar_a, AB);
-                bulk_g2s(sA, imgA + (size_t)nbi2 * AB, AB / 2, &s.bar_a);
-                bulk_g2s(sA + AB / 2, imgA + (size_t)nbi2 * AB + AB / 2, AB / 2, &s.bar_a);
+        if (warp == 0) {
+            pend = __shfl_sync(0xffffffffu, todo > 1 && !s.err, 0);
+            if (lane == 0 && pend) {
+                if (nbi2 != bi) {
+                    mbar_arrive_expect_tx(&s.bar_a, AB);
+                    bulk_g2s(sA, imgA + (size_t)nbi2 * AB, AB / 2, &s.bar_a);
+                    bulk_g2s(sA + AB / 2, imgA + (size_t)nbi2 * AB + AB / 2, AB / 2, &s.bar_a);
+                }
+                mbar_arrive_expect_tx(&s.bar_b, BB);
+                bulk_g2s(sB, imgB + (size_t)nbj2 * BB, BB, &s.bar_b);
             }
-            mbar_arrive_expect_tx(&s.bar_b, BB);
-            bulk_g2s(sB, imgB + (size_t)nbj2 * BB, BB, &s.bar_b);
         }
         tc_fence_after();
         // epilogue: TMEM lanes 32(w%4).. (rows), columns CW(w/4)..+CW-1
@@ -432,7 +448,7 @@ static __device__ bool mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
                 for (int j = 0; j < 4; ++j) {
                     const int col = bj * TN + CW * hcol + cc + j;
                     if (col < nn) {
-                        const float sc = ea_r * __ldg(geb + col);  // 2^(ea+eb-16), exact
+                        const float sc = ea_r * geb[col];  // 2^(ea+eb-16), exact
                         const float4 cv = cpre[cc + j];
                         dfc c = dfc{df{cv.x, cv.y}, df{cv.z, cv.w}};
                         float lr[NG], li[NG];
@@ -453,41 +469,28 @@ static __device__ bool mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
         new_band = (nbi2 != bi);
         bi = nbi2;
         bj = nbj2;
-        if (s.err) {
-            ok = false;
-            break;
-        }
+        --todo;
     }
     stat_add(s, PH_TILES);
-    return ok;
 }
 
 // ---------------------------------------------------------------- double-float panel, TRSM, solves
-// arg max of v over the CTA (smallest index on ties), in FP32: the FP64 pipe
-// (1/64 of the FP32 rate on GB300) stays out of the panel's per-column steps
-__device__ __forceinline__ int block_argmaxf(float v, int i, MixSmem& s) {
+// row of the CTA's largest v >= 0 (smallest row on ties; v = -1: no row), in
+// every thread: the FP32 bit patterns order like the values, so the search is
+// two warp reductions, and one barrier (candidates double-buffered by `par`)
+__device__ __forceinline__ int block_pivotf(float v, int row, int par, MixSmem& s) {
+    constexpr int NW = NT / 32;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const float v2 = __shfl_down_sync(FULL, v, off);
-        const int i2 = __shfl_down_sync(FULL, i, off);
-        if (v2 > v || (v2 == v && i2 < i)) { v = v2; i = i2; }
-    }
-    if (lane == 0) { s.red_f[warp] = v; s.red_i[warp] = i; }
+    int k = v < 0.0f ? -1 : __float_as_int(v);
+    int m = __reduce_max_sync(FULL, k);
+    row = __reduce_min_sync(FULL, k == m ? row : 0x7fffffff);
+    if (lane == 0) { s.red_k[par][warp] = m; s.red_p[par][warp] = row; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float bv = s.red_f[0];
-        int bi = s.red_i[0];
-        for (int w = 1; w < NT / 32; w++) {
-            const float v2 = s.red_f[w];
-            const int i2 = s.red_i[w];
-            if (v2 > bv || (v2 == bv && i2 < bi)) { bv = v2; bi = i2; }
-        }
-        s.bcast_i = bi;
-    }
-    __syncthreads();
-    return s.bcast_i;
+    k = s.red_k[par][lane & (NW - 1)];
+    row = s.red_p[par][lane & (NW - 1)];
+    m = __reduce_max_sync(FULL, k);
+    return __reduce_min_sync(FULL, k == m ? row : 0x7fffffff);
 }
 
 // 1 / b in double-float, with b scaled by a power of two first so that its
@@ -508,14 +511,16 @@ __device__ __forceinline__ dfc dfc_recip_pow2(dfc b) {
 // matrix does not stay in L2 across 304 resident CTAs, so this cuts its
 // memory traffic (the full-width rank-1 form re-reads and re-writes the whole
 // remaining panel once per column) by about 2.4x at the same arithmetic.
-// The pivot's reciprocal is a double-float one that every thread computes
-// (the FP64 division by one thread, on a pipe at 1/64 of the FP32 rate, held
-// the whole CTA at the next barrier).
+// One warp takes the interchange, the pivot row and the pivot's double-float
+// reciprocal (an FP64 division, on a pipe at 1/64 of the FP32 rate, held the
+// whole CTA at the next barrier): two barriers a column.  4096 ln det at n = 64:
+// 4.95 ms with three barriers, every thread's own reciprocal and a thread per row
+// of the rank-4 update, 3.49 now.
 // Not inlined: its registers are then allocated apart from the engine's
 // tensor-core epilogue, which holds the kernel at the 128-register cap.
 constexpr int SW = 4;
 
-static __device__ __noinline__ void df_panel(float4* __restrict__ A, int n, int j0, int jb, int* __restrict__ ipiv, MixSmem& s) {
+static __device__ __noinline__ void df_panel(float4* A, int n, int j0, int jb, int* ipiv, MixSmem& s) {
     const int tid = threadIdx.x;
     const int cend = j0 + jb;
     float bv = -1.0f;
@@ -527,25 +532,34 @@ static __device__ __noinline__ void df_panel(float4* __restrict__ A, int n, int 
     for (int c0 = j0; c0 < cend; c0 += SW) {
         const int sw = min(c0 + SW, cend);  // sub-panel columns [c0, sw)
         for (int c = c0; c < sw; ++c) {
-            int p = block_argmaxf(bv, bi, s);
+            int p = block_pivotf(bv, bi, c & 1, s);
             if (p >= n) p = c;
-            const dfc piv = dfc_load(A + p + (size_t)c * n);
-            const bool nz = !dfc_is_zero(piv);
-            if (tid == 0) {
-                ipiv[c] = p;
-                if (!nz && s.info == 0) s.info = c + 1;
-            }
-            const dfc r = nz ? dfc_recip_pow2(piv) : dfc{df{0, 0}, df{0, 0}};
-            __syncthreads();  // every thread holds the pivot before row p is swapped away
-            if (nz && p != c && tid < jb) {
+            if (tid < 32) {
                 const size_t col = (size_t)(j0 + tid) * n;
-                float4 t = A[c + col];
-                A[c + col] = A[p + col];
-                A[p + col] = t;
+                float4 a = make_float4(0, 0, 0, 0), t = a;
+                if (tid < jb) {
+                    a = A[c + col];
+                    t = p != c ? A[p + col] : a;
+                }
+                const bool piv0 = t.x == 0.0f && t.z == 0.0f;
+                const bool nz = !__shfl_sync(0xffffffffu, (int)piv0, c - j0);
+                if (tid < jb) {
+                    if (nz && p != c) {
+                        A[c + col] = t;
+                        A[p + col] = a;
+                    }
+                    s.u.p.urow[tid] = nz ? t : a;
+                }
+                if (tid == c - j0) {
+                    ipiv[c] = p;
+                    if (!nz && s.info == 0) s.info = c + 1;
+                    s.nz = nz;
+                    if (nz) dfc_store(&s.rpiv, dfc_recip_pow2(dfc{df{t.x, t.y}, df{t.z, t.w}}));
+                }
             }
             __syncthreads();
-            if (tid < jb && j0 + tid > c && j0 + tid < sw) s.u.p.urow[tid] = A[c + (size_t)(j0 + tid) * n];
-            __syncthreads();
+            const bool nz = s.nz != 0;
+            const dfc r = dfc_load(&s.rpiv);
             bv = -1.0f;
             bi = n;
             if (nz) {
@@ -598,27 +612,33 @@ static __device__ __noinline__ void df_panel(float4* __restrict__ A, int n, int 
                 }
             }
             __syncthreads();
-            // rank-cw update of rows >= sw; argmax of column sw on the way
+            // rank-cw update of rows >= sw; argmax of column sw on the way.  A warp takes 32
+            // rows; where the rows do not fill the CTA several warps share them, each with
+            // every G-th column.
             bv = -1.0f;
             bi = n;
-            for (int i = sw + tid; i < n; i += NT) {
-                dfc l[SW];
-#pragma unroll
-                for (int q = 0; q < SW; ++q)
-                    if (q < cw) l[q] = dfc_load(A + i + (size_t)(c0 + q) * n);
-                for (int t = 0; t < rem; ++t) {
-                    float4* qp = A + i + (size_t)(sw + t) * n;
-                    dfc a = dfc_load(qp);
+            const int nrb = (n - sw + 31) / 32, G = max(1, (NT / 32) / nrb);
+            const int g = nrb < NT / 32 ? (tid >> 5) / nrb : 0;
+            const int i0 = sw + (nrb < NT / 32 ? ((tid >> 5) % nrb) * 32 + (tid & 31) : tid);
+            if (g < G)
+                for (int i = i0; i < n; i += NT) {
+                    dfc l[SW];
 #pragma unroll
                     for (int q = 0; q < SW; ++q)
-                        if (q < cw) a = dfc_fms(a, l[q], dfc_load(&s.u.p.T[q][t]));
-                    dfc_store(qp, a);
-                    if (t == 0) {
-                        const float v = dfc_abs1(a);
-                        if (v > bv) { bv = v; bi = i; }
+                        if (q < cw) l[q] = dfc_load(A + i + (size_t)(c0 + q) * n);
+                    for (int t = g; t < rem; t += G) {
+                        float4* qp = A + i + (size_t)(sw + t) * n;
+                        dfc a = dfc_load(qp);
+#pragma unroll
+                        for (int q = 0; q < SW; ++q)
+                            if (q < cw) a = dfc_fms(a, l[q], dfc_load(&s.u.p.T[q][t]));
+                        dfc_store(qp, a);
+                        if (t == 0) {
+                            const float v = dfc_abs1(a);
+                            if (v > bv) { bv = v; bi = i; }
+                        }
                     }
                 }
-            }
         }
     }
     __syncthreads();
@@ -650,7 +670,7 @@ __device__ __forceinline__ void dcol_upper(float4* __restrict__ b, int jb, const
         dfc y[CH];
 #pragma unroll
         for (int r = 0; r < CH; ++r) y[r] = (rb + r < jb) ? dfc_load(b + rb + r) : dfc{df{0, 0}, df{0, 0}};
-        for (int q = rb + CH; q < jb; ++q) {
+        for (int q = jb - 1; q >= rb + CH; --q) {
             const dfc xq = dfc_load(b + q);
 #pragma unroll
             for (int r = 0; r < CH; ++r) y[r] = dfc_fms(y[r], dfc_load(&T[rb + r][q]), xq);
@@ -660,7 +680,8 @@ __device__ __forceinline__ void dcol_upper(float4* __restrict__ b, int jb, const
             if (rb + r < jb) {
                 dfc acc = y[r];
 #pragma unroll
-                for (int q = r + 1; q < CH; ++q) acc = dfc_fms(acc, dfc_load(&T[rb + r][rb + q]), y[q]);
+                for (int q = CH - 1; q > r; --q)
+                    if (rb + q < jb) acc = dfc_fms(acc, dfc_load(&T[rb + r][rb + q]), y[q]);
                 y[r] = dfc_mul(acc, dfc_load(&T[rb + r][rb + r]));
             }
         }
@@ -668,6 +689,31 @@ __device__ __forceinline__ void dcol_upper(float4* __restrict__ b, int jb, const
         for (int r = 0; r < CH; ++r)
             if (rb + r < jb) dfc_store(b + rb + r, y[r]);
     }
+}
+
+// The same solves with one row a lane, for a warp per column (few columns); every
+// element takes its updates in the order of the column solves.
+__device__ __forceinline__ dfc dfc_shfl(dfc v, int src) {
+    const unsigned FULL = 0xffffffffu;
+    return dfc{df{__shfl_sync(FULL, v.re.h, src), __shfl_sync(FULL, v.re.l, src)},
+               df{__shfl_sync(FULL, v.im.h, src), __shfl_sync(FULL, v.im.l, src)}};
+}
+__device__ __forceinline__ dfc drow_lower_unit(dfc x, int jb, const float4 (*T)[NB + 1]) {
+    const int lane = threadIdx.x & 31;
+    for (int q = 0; q + 1 < jb; ++q) {
+        const dfc xq = dfc_shfl(x, q);
+        if (lane > q && lane < jb) x = dfc_fms(x, dfc_load(&T[lane][q]), xq);
+    }
+    return x;
+}
+__device__ __forceinline__ dfc drow_upper(dfc x, int jb, const float4 (*T)[NB + 1]) {
+    const int lane = threadIdx.x & 31;
+    for (int q = jb - 1; q >= 0; --q) {
+        if (lane == q) x = dfc_mul(x, dfc_load(&T[q][q]));
+        const dfc xq = dfc_shfl(x, q);
+        if (lane < q) x = dfc_fms(x, dfc_load(&T[lane][q]), xq);
+    }
+    return x;
 }
 
 static __device__ void load_lower_block(const float4* A, int n, int j0, int jb, MixSmem& s) {
@@ -698,72 +744,142 @@ static __device__ void load_upper_block(const float4* A, int n, int j0, int jb, 
     __syncthreads();
 }
 
+// one column through a panel's interchanges (panel_moves), one load and one store a lane
+__device__ __forceinline__ void move_rows(float4* a, int j0, int jb, int inner, int orow, int ocur) {
+    const int lane = threadIdx.x & 31;
+    const float4 z = make_float4(0, 0, 0, 0);
+    const float4 v = lane < jb ? a[inner] : z, w = orow >= 0 ? a[ocur] : z;
+    __syncwarp();
+    if (lane < jb) a[j0 + lane] = v;
+    if (orow >= 0) a[orow] = w;
+}
+
 // The panel's row interchanges on the columns outside it, then the TRSM
 // U12 = L11^-1 A12 of the columns right of it.  keep_l = false leaves the columns
 // left of the panel alone: a ln det reads only U's diagonal and the pivots.
-static __device__ void df_swaps_trsm(float4* __restrict__ A, int n, int j0, int jb, const int* __restrict__ ipiv,
-                                     MixSmem& s, bool keep_l) {
+template <class Team>
+static __device__ void df_swaps_trsm(float4* A, int n, int j0, int jb, const int* ipiv, MixSmem& s, bool keep_l, const Team& tm) {
+    constexpr int NW = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     load_lower_block(A, n, j0, jb, s);
-    for (int col = keep_l ? threadIdx.x : j0 + threadIdx.x; col < n; col += NT) {
-        if (col >= j0 && col < j0 + jb) continue;
-        float4* a = A + (size_t)col * n;
-        for (int c = j0; c < j0 + jb; ++c) {
-            int p = ipiv[c];
-            if (p != c) { float4 t = a[c]; a[c] = a[p]; a[p] = t; }
+    int inner, orow, ocur;
+    panel_moves(ipiv, j0, jb, inner, orow, ocur);
+    const bool moves = __any_sync(0xffffffffu, inner != j0 + lane);
+    const int right = j0 + jb, nr = cta_columns(n - right, tm);
+    const bool few = few_columns(nr);
+    if (keep_l && moves) {
+        const int nl = cta_columns(j0, tm);
+        for (int x = warp; x < nl; x += NW) {
+            const int col = cta_column(x, tm);
+            if (col < j0) move_rows(A + (size_t)col * n, j0, jb, inner, orow, ocur);
         }
-        if (col >= j0 + jb) dcol_lower_unit(a + j0, jb, s.u.p.T);
     }
-    __syncthreads();
+    if (moves)
+        for (int x = warp; x < nr; x += NW) {
+            const int col = right + cta_column(x, tm);
+            if (col < n) move_rows(A + (size_t)col * n, j0, jb, inner, orow, ocur);
+        }
+    if (few) {
+        __syncwarp();  // a warp solves the columns it moved
+        for (int x = warp; x < nr; x += NW) {
+            const int col = right + cta_column(x, tm);
+            if (col >= n) continue;
+            float4* a = A + (size_t)col * n + j0;
+            const dfc v = drow_lower_unit(lane < jb ? dfc_load(a + lane) : dfc{df{0, 0}, df{0, 0}}, jb, s.u.p.T);
+            if (lane < jb) dfc_store(a + lane, v);
+        }
+    } else {
+        __syncthreads();
+        for (int x = tid; x < nr; x += NT) {
+            const int col = right + cta_column(x, tm);
+            if (col < n) dcol_lower_unit(A + (size_t)col * n + j0, jb, s.u.p.T);
+        }
+    }
+    tm.sync();
 }
 
-template <int NS>
-static __device__ bool lu_mixed(float4* __restrict__ A, int n, int* __restrict__ ipiv, bool keep_l, MixSmem& s,
-                                const MixScratch& X, uint32_t tmem, Phases& ph) {
+template <int NS, class Team>
+static __device__ void lu_mixed(float4* A, int n, int* ipiv, bool keep_l, MixSmem& s, const MixScratch& X, uint32_t tmem,
+                                Phases& ph, const Team& tm) {
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
         stat_start(s);
-        df_panel(A, n, j0, jb, ipiv, s);
+        if (tm.rank == 0) df_panel(A, n, j0, jb, ipiv, s);
+        if (tm.size > 1) tm.sync();
         stat_add(s, PH_PANEL);
-        df_swaps_trsm(A, n, j0, jb, ipiv, s, keep_l);
+        df_swaps_trsm(A, n, j0, jb, ipiv, s, keep_l, tm);
         stat_add(s, PH_TRSM);
         const int r0 = j0 + jb;
-        if (!mixed_gemm_sub<NS>(A + r0 + (size_t)r0 * n, n, A + r0 + (size_t)j0 * n, n, A + j0 + (size_t)r0 * n, n,
-                            n - r0, n - r0, jb, 0, s, X, tmem, ph))
-            return false;
+        mixed_gemm_sub<NS>(A + r0 + (size_t)r0 * n, n, A + r0 + (size_t)j0 * n, n, A + j0 + (size_t)r0 * n, n, n - r0, n - r0,
+                           jb, 0, s, X, tmem, ph, tm);
+        if (tm.size > 1) tm.sync();
     }
-    return true;
 }
 
 // tr(A^-1 B) from the mixed LU of A; B (double-float, n x n) is destroyed
-template <int NS>
-static __device__ bool trace_solve_mixed(const float4* __restrict__ A, float4* __restrict__ B, int n,
-                                  const int* __restrict__ ipiv, MixSmem& s, const MixScratch& X, uint32_t tmem,
-                                  Phases& ph, zc& out) {
-    const int tid = threadIdx.x;
-    for (int col = tid; col < n; col += NT) {
-        float4* b = B + (size_t)col * n;
-        for (int i = 0; i < n; ++i) {
-            int p = ipiv[i];
-            if (p != i) { float4 t = b[i]; b[i] = b[p]; b[p] = t; }
+template <int NS, class Team>
+static __device__ zc trace_solve_mixed(const float4* A, float4* B, int n, const int* ipiv, MixSmem& s, const MixScratch& X,
+                                  uint32_t tmem, Phases& ph, const Team& tm) {
+    constexpr int NW = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int mine = cta_columns(n, tm);
+    const dfc zero{df{0, 0}, df{0, 0}};
+    for (int j0 = 0; j0 < n; j0 += NB) {
+        const int jb = min(NB, n - j0);
+        int inner, orow, ocur;
+        panel_moves(ipiv, j0, jb, inner, orow, ocur);
+        if (!__any_sync(0xffffffffu, inner != j0 + lane)) continue;
+        for (int x = warp; x < mine; x += NW) {
+            const int col = cta_column(x, tm);
+            if (col < n) move_rows(B + (size_t)col * n, j0, jb, inner, orow, ocur);
         }
+        __syncwarp();
     }
     __syncthreads();
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
         load_lower_block(A, n, j0, jb, s);
-        for (int col = tid; col < n; col += NT) dcol_lower_unit(B + (size_t)col * n + j0, jb, s.u.p.T);
-        __syncthreads();
+        if (few_columns(mine)) {
+            for (int x = warp; x < mine; x += NW) {
+                const int col = cta_column(x, tm);
+                if (col >= n) continue;
+                float4* b = B + (size_t)col * n + j0;
+                const dfc v = drow_lower_unit(lane < jb ? dfc_load(b + lane) : zero, jb, s.u.p.T);
+                if (lane < jb) dfc_store(b + lane, v);
+            }
+        } else {
+            for (int x = tid; x < mine; x += NT) {
+                const int col = cta_column(x, tm);
+                if (col < n) dcol_lower_unit(B + (size_t)col * n + j0, jb, s.u.p.T);
+            }
+        }
+        tm.sync();
         const int r0 = j0 + jb;
-        if (!mixed_gemm_sub<NS>(B + r0, n, A + r0 + (size_t)j0 * n, n, B + j0, n, n - r0, n, jb, 0, s, X, tmem, ph))
-            return false;
+        mixed_gemm_sub<NS>(B + r0, n, A + r0 + (size_t)j0 * n, n, B + j0, n, n - r0, n, jb, 0, s, X, tmem, ph, tm);
+        if (tm.size > 1) tm.sync();
     }
     const int nblk = (n + NB - 1) / NB;
     for (int kb = nblk - 1; kb >= 0; --kb) {
         const int j0 = kb * NB, jb = min(NB, n - j0), ncol = j0 + jb;
         load_upper_block(A, n, j0, jb, s);
-        for (int col = tid; col < ncol; col += NT) dcol_upper(B + (size_t)col * n + j0, jb, s.u.p.T);
-        __syncthreads();
-        if (!mixed_gemm_sub<NS>(B, n, A + (size_t)j0 * n, n, B + j0, n, j0, ncol, jb, 1, s, X, tmem, ph)) return false;
+        const int cols = cta_columns(ncol, tm);
+        if (few_columns(cols)) {
+            for (int x = warp; x < cols; x += NW) {
+                const int col = cta_column(x, tm);
+                if (col >= ncol) continue;
+                float4* b = B + (size_t)col * n + j0;
+                const dfc v = drow_upper(lane < jb ? dfc_load(b + lane) : zero, jb, s.u.p.T);
+                if (lane < jb) dfc_store(b + lane, v);
+            }
+        } else {
+            for (int x = tid; x < cols; x += NT) {
+                const int col = cta_column(x, tm);
+                if (col < ncol) dcol_upper(B + (size_t)col * n + j0, jb, s.u.p.T);
+            }
+        }
+        tm.sync();
+        mixed_gemm_sub<NS>(B, n, A + (size_t)j0 * n, n, B + j0, n, j0, ncol, jb, 1, s, X, tmem, ph, tm);
+        if (tm.size > 1) tm.sync();
     }
     double tr = 0.0, ti = 0.0, z = 0.0;
     for (int i = tid; i < n; i += NT) {
@@ -772,8 +888,7 @@ static __device__ bool trace_solve_mixed(const float4* __restrict__ A, float4* _
         ti += df_to_double(v.im);
     }
     block_sum3(tr, ti, z, s);
-    out = mk(tr, ti);
-    return true;
+    return mk(tr, ti);
 }
 
 // (largest, smallest non-zero) of max(|Re|, |Im|) over the entries seen, with v added
@@ -899,16 +1014,16 @@ static __device__ __noinline__ float2 assemble_tile_grouped_df2(float4* __restri
 
 // Assembly of M(k) (and dM/dk into B) as double-floats; returns the largest
 // and the smallest non-zero max(|Re|, |Im|) over the entries this thread stored.
-template <bool D3ONLY>
+template <bool D3ONLY, class Team>
 __device__ float2 assemble_df(float4* __restrict__ A, float4* __restrict__ B, int n, int d,
-                             const double* __restrict__ pos, const msgpu_model& mdl, zc k, MixSmem& s) {
+                             const double* __restrict__ pos, const msgpu_model& mdl, zc k, MixSmem& s, const Team& tm) {
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        s.diag[0] = invf(mdl, d, k);
-        if (B) s.diag[1] = dk_invf(mdl, d, k);
-    }
+    // F^-1 and the two sides of its central difference (dk_invf), one thread of three warps
+    if (tid == 0) s.diag[0] = invf(mdl, d, k);
+    if (B && tid == 32) s.diag[1] = invf(mdl, d, k + DK_INVF_STEP);
+    if (B && tid == 64) s.diag[2] = invf(mdl, d, k - DK_INVF_STEP);
     __syncthreads();
-    const zc dg0 = s.diag[0], dg1 = s.diag[1];
+    const zc dg0 = s.diag[0], dg1 = B ? (s.diag[1] - s.diag[2]) / (2.0 * DK_INVF_STEP) : mk(0.0);
     const bool d3 = D3ONLY || d == 3;
     const df kr = df_from_double(k.re), ki = df_from_double(k.im);
     const bool grow = k.im != 0.0;
@@ -924,8 +1039,10 @@ __device__ float2 assemble_df(float4* __restrict__ A, float4* __restrict__ B, in
         return make_float4(a.h, a.l, b.h, b.l);
     };
     const int nt = (n + 31) / 32;
+    int tile = 0;
     for (int J = 0; J < nt; ++J) {
         for (int I = 0; I <= J; ++I) {
+            if (tm.size > 1 && tile++ % tm.size != tm.rank) continue;
             if (d3 || d2) {
                 // the tile's atoms as double-floats: rows I*32.., columns J*32..
                 if (tid < 64) {
@@ -1007,6 +1124,34 @@ __device__ float2 assemble_df(float4* __restrict__ A, float4* __restrict__ B, in
     return rg;
 }
 
+// The range of an item's entries over its team: FP32 bit patterns of non-negative
+// values order like the values, so integer reductions serve.
+template <class Team>
+__device__ __forceinline__ float2 team_range(float2 rg, MixSmem& s, const Team& tm) {
+    const int tid = threadIdx.x;
+    if (tid == 0) { s.rng[0] = 0; s.rng[1] = 0x7f800000; }
+    __syncthreads();
+    const int h = __reduce_max_sync(0xffffffffu, __float_as_int(rg.x)), l = __reduce_min_sync(0xffffffffu, __float_as_int(rg.y));
+    if ((tid & 31) == 0) {
+        atomicMax(&s.rng[0], h);
+        atomicMin(&s.rng[1], l);
+    }
+    __syncthreads();
+    int hi = s.rng[0], lo = s.rng[1];
+    if (tm.size > 1) {
+        if (tid < tm.size) {
+            cluster_store(&s.team_rng[tm.rank][0], tid, hi);
+            cluster_store(&s.team_rng[tm.rank][1], tid, lo);
+        }
+        tm.sync();
+        for (int r = 0; r < tm.size; ++r) {
+            hi = max(hi, s.team_rng[r][0]);
+            lo = min(lo, s.team_rng[r][1]);
+        }
+    }
+    return make_float2(__int_as_float(hi), __int_as_float(lo));
+}
+
 // after block_argmax: the CTA-wide maximum (thread 0 folded the warp maxima into red_v)
 __device__ __forceinline__ double block_max_value(MixSmem& s) {
     double m = s.red_v[0];
@@ -1031,14 +1176,15 @@ static __device__ zc tracelog_df(const float4* __restrict__ A, int n, const int*
 // x <- (LU)^-1 x, one right-hand side, double-float (LAPACK-layout LU): the
 // interchanges, then blocked substitution; each block's triangle by warp 0
 // (one row per lane), the rectangular part by all threads (one row each)
-static __device__ void df_solve_vec(const float4* __restrict__ A, float4* __restrict__ x, int n,
-                             const int* __restrict__ ipiv, MixSmem& s) {
+static __device__ void df_solve_vec(const float4* A, float4* x, int n, const int* ipiv, MixSmem& s) {
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
-    if (tid == 0)
-        for (int i = 0; i < n; ++i) {
-            int p = ipiv[i];
-            if (p != i) { float4 t = x[i]; x[i] = x[p]; x[p] = t; }
+    if (tid < 32)
+        for (int j0 = 0; j0 < n; j0 += NB) {
+            int inner, orow, ocur;
+            panel_moves(ipiv, j0, min(NB, n - j0), inner, orow, ocur);
+            move_rows(x, j0, min(NB, n - j0), inner, orow, ocur);
+            __syncwarp();
         }
     __syncthreads();
     auto shfl4 = [&](float4 v, int src) {
@@ -1099,42 +1245,30 @@ static __device__ void df_solve_vec(const float4* __restrict__ A, float4* __rest
     }
 }
 
-// a = M^-1 phi by the mixed LU plus iterative refinement: r = phi - M a with
-// M in FP64 for the refinement residual: every element evaluated as the FP64
-// engine does (each pair on its own, so the writes stay coalesced)
-static __device__ void assemble_fp64_copy(zc* __restrict__ M, const MedDev& md, zc k, MixSmem& s) {
-    const int n = md.n;
-    const zc dg = s.diag[0];
-    for (size_t e = threadIdx.x; e < (size_t)n * n; e += NT) {
-        const int i = (int)(e % n), j = (int)(e / n);
-        zc m = dg, dm;
-        if (i != j) pair_elements(md.d, k, atom_distance(md.d, md.pos, min(i, j), max(i, j)), false, m, dm);
-        M[e] = m;
-    }
-    __syncthreads();
-}
-
 // a = M^-1 phi from the mixed LU with iterative refinement: r = phi - M a in
 // FP64 against the FP64 copy of M, a += (LU)^-1 r (correction in double-float,
 // a kept in FP64), until |r| <= 1e-14 |phi| (max norms), the residual stops
 // halving, or 8 corrections.  Returns sigma = -Im(conj(phi).a)/k (the optical
 // theorem of total_cross_section, ms_matrix_util.c:361).
-static __device__ zc refine_solve(const float4* __restrict__ LU, const zc* __restrict__ M, const zc* __restrict__ phi,
-                           zc* __restrict__ x, float4* __restrict__ r, float4* __restrict__ t, const MedDev& md,
-                           zc k, const int* __restrict__ ipiv, MixSmem& s) {
+// The team shares the residuals (a row a thread), its first CTA takes the solves.
+template <class Team>
+static __device__ zc refine_solve(const float4* LU, const zc* M, const zc* phi, zc* x, float4* r, float4* t, const MedDev& md,
+                           zc k, const int* ipiv, MixSmem& s, const Team& tm) {
     const int n = md.n, tid = threadIdx.x;
     auto to4 = [](zc v) {
         const df a = df_from_double(v.re), b = df_from_double(v.im);
         return make_float4(a.h, a.l, b.h, b.l);
     };
-    for (int i = tid; i < n; i += NT) t[i] = to4(phi[i]);
-    __syncthreads();
-    df_solve_vec(LU, t, n, ipiv, s);
-    for (int i = tid; i < n; i += NT) {
-        const dfc v = dfc_load(t + i);
-        x[i] = mk(df_to_double(v.re), df_to_double(v.im));
+    if (tm.rank == 0) {
+        for (int i = tid; i < n; i += NT) t[i] = to4(phi[i]);
+        __syncthreads();
+        df_solve_vec(LU, t, n, ipiv, s);
+        for (int i = tid; i < n; i += NT) {
+            const dfc v = dfc_load(t + i);
+            x[i] = mk(df_to_double(v.re), df_to_double(v.im));
+        }
     }
-    __syncthreads();
+    tm.sync();
     double pmax = 0.0;
     for (int i = tid; i < n; i += NT) pmax = fmax(pmax, zabs(phi[i]));
     int dummy;
@@ -1145,7 +1279,7 @@ static __device__ zc refine_solve(const float4* __restrict__ LU, const zc* __res
     for (int it = 0; it < 8; ++it) {
         // r = phi - M x in FP64, rows over threads (coalesced columns of M)
         double rmax = 0.0;
-        for (int i = tid; i < n; i += NT) {
+        for (int i = tm.rank * NT + tid; i < n; i += NT * tm.size) {
             zc acc = phi[i];
             for (int j = 0; j < n; ++j) {
                 const zc mv = M[i + (size_t)j * n], xv = x[j];
@@ -1158,14 +1292,21 @@ static __device__ zc refine_solve(const float4* __restrict__ LU, const zc* __res
         block_argmax(rmax, tid, s, dummy);
         rmax = block_max_value(s);
         __syncthreads();
+        if (tm.size > 1) {
+            if (tid < tm.size) cluster_store(&s.team_max[tm.rank], tid, rmax);
+            tm.sync();  // and every part of r is there
+            for (int q = 0; q < tm.size; ++q) rmax = fmax(rmax, s.team_max[q]);
+        }
         if (!(rmax > 1e-14 * pmax) || !(rmax < 0.5 * prev)) break;
         prev = rmax;
-        df_solve_vec(LU, r, n, ipiv, s);
-        for (int i = tid; i < n; i += NT) {
-            const dfc v = dfc_load(r + i);
-            x[i] = x[i] + mk(df_to_double(v.re), df_to_double(v.im));
+        if (tm.rank == 0) {
+            df_solve_vec(LU, r, n, ipiv, s);
+            for (int i = tid; i < n; i += NT) {
+                const dfc v = dfc_load(r + i);
+                x[i] = x[i] + mk(df_to_double(v.re), df_to_double(v.im));
+            }
         }
-        __syncthreads();
+        tm.sync();
     }
     double dr = 0.0, di = 0.0, z = 0.0;
     for (int i = tid; i < n; i += NT) {
@@ -1182,17 +1323,35 @@ static __device__ zc refine_solve(const float4* __restrict__ LU, const zc* __res
 // only its own reduction, solve and Green function, so a kernel's registers
 // are not shaped by code it never runs (a never-taken call to the d != 3 tile
 // cost the d = 3 ln det kernel 5 %).
-// host entries of the six variants (mixed_k*.cu): set the shared-memory limit
-// (attr_only) or launch
-int mixed_variant_0_d3(const EngineParams&, const MixScratch&, int, size_t, cudaStream_t, bool);
-int mixed_variant_1_d3(const EngineParams&, const MixScratch&, int, size_t, cudaStream_t, bool);
-int mixed_variant_2_d3(const EngineParams&, const MixScratch&, int, size_t, cudaStream_t, bool);
-int mixed_variant_0_any(const EngineParams&, const MixScratch&, int, size_t, cudaStream_t, bool);
-int mixed_variant_1_any(const EngineParams&, const MixScratch&, int, size_t, cudaStream_t, bool);
-int mixed_variant_2_any(const EngineParams&, const MixScratch&, int, size_t, cudaStream_t, bool);
+// Each comes for one CTA per matrix (Solo) and for a cluster of them (ClusterTeam),
+// which a batch that leaves SMs idle takes: one wavefunction at n = 1024, 512 x 512
+// pixels, 74 ms with one CTA, 31 with a cluster of 16.
+// host entries of the variants (mixed_k*.cu, mixed_t*.cu): the largest number of
+// clusters resident (query), or launch
+struct MixLaunch {
+    int teams, team;  // matrices at a time, CTAs on each
+    size_t smem;
+    cudaStream_t st;
+    bool query;
+};
+int mixed_variant_0_d3(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_variant_1_d3(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_variant_2_d3(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_variant_0_any(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_variant_1_any(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_variant_2_any(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_team_0_d3(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_team_1_d3(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_team_2_d3(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_team_0_any(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_team_1_any(const EngineParams&, const MixScratch&, const MixLaunch&);
+int mixed_team_2_any(const EngineParams&, const MixScratch&, const MixLaunch&);
 
 #ifdef MSG_MIXED_KERNEL_BODY
-template <int KIND, bool D3ONLY>
+__device__ __forceinline__ void make_team(Solo&) {}
+__device__ __forceinline__ void make_team(ClusterTeam& t) { t = this_team(); }
+
+template <int KIND, bool D3ONLY, class Team>
 __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScratch X)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -1216,10 +1375,12 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s.tmem;
+    Team tm;
+    make_team(tm);
     Phases ph{0, 0, 0};
-    const size_t vec = (((size_t)P.piv_stride + 15) / 16) * 16;
+    const size_t vec = (((size_t)P.piv_stride + 15) / 16) * 16, team = blockIdx.x / tm.size;
     const size_t slot_all = KIND == 0 ? P.slot : (KIND == 1 ? 2 * P.slot : 2 * P.slot + 4 * vec);
-    float4* A = reinterpret_cast<float4*>(P.ws) + (size_t)blockIdx.x * slot_all;
+    float4* A = reinterpret_cast<float4*>(P.ws) + team * slot_all;
     float4* B = (KIND == 1) ? A + P.slot : nullptr;
     // kind 2: copy of M, right-hand side phi, solution, residual, correction
     zc* Mc = reinterpret_cast<zc*>(A + P.slot);  // kind 2: M in FP64 for the refinement
@@ -1227,30 +1388,28 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
     zc* vx = vphi + vec;
     float4* vr = reinterpret_cast<float4*>(vx + vec);
     float4* vt = vr + vec;
-    int* ipiv = P.piv + (size_t)blockIdx.x * P.piv_stride;
+    int* ipiv = P.piv + team * P.piv_stride;
+    if (tm.size > 1) tm.sync();  // every CTA of the cluster is there before its shared memory is written
     bool alive = true;
     while (alive) {
-        if (tid == 0) {
+        if (tm.rank == 0 && tid == 0) {
             const unsigned q = atomicAdd(P.counter, 1u);
-            s.item = q < P.counter[1] ? (int)q : P.nitem;
+            const int item = q < P.counter[1] ? (int)q : P.nitem;
+            s.item = item;
+            for (int r = 1; r < tm.size; ++r) cluster_store(&s.item, r, item);
             s.info = 0;
         }
-        __syncthreads();
+        tm.sync();
         const int q = s.item;
         if (q >= P.nitem) break;
         const int it = P.order[q];
         const MedDev md = P.media[P.item_med[it]];
         const zc k = mk(P.ks[2 * it], P.ks[2 * it + 1]);
         stat_start(s);
-        const float2 rg = assemble_df<D3ONLY>(A, B, md.n, md.d, md.pos, md.model, k, s);
+        float2 rg = assemble_df<D3ONLY>(A, B, md.n, md.d, md.pos, md.model, k, s, tm);
         stat_add(s, PH_ASSEMBLE);
-        int dummy;
-        block_argmax((double)rg.x, tid, s, dummy);
-        const double mxd = block_max_value(s);
-        __syncthreads();  // red_v is reused by the next reduction
-        block_argmax(-(double)rg.y, tid, s, dummy);
-        const double mnd = -block_max_value(s);
-        __syncthreads();
+        rg = team_range(rg, s, tm);
+        const double mxd = rg.x, mnd = rg.y;
         // six slices when the entries span more than SPAN_WIDE (SPAN_WIDE_REFINED for amplitude
         // items) or an entry is zero / non-finite, and for every dlogf item (near a root the condition number of M magnifies the LU's
         // error in tr(M^-1 dM/dk)), if this launch has the shared memory for them; else four,
@@ -1265,34 +1424,45 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
             res = mk(nan(""), nan(""));
         } else {
             if (KIND == 2) {
-                // keep M for the residual; incident plane wave along +x (incident_wave_util.c:76)
-                assemble_fp64_copy(Mc, md, k, s);
-                for (int i = tid; i < md.n; i += NT) vphi[i] = zexp(mk(0.0, 1.0) * k * md.pos[i * md.d]);
+                // M in FP64 for the residual, every element as the FP64 engine assembles it;
+                // incident plane wave along +x (incident_wave_util.c:76)
+                EntryRange er;
                 __syncthreads();
+                assemble(Mc, nullptr, md.n, md.d, md.pos, md.model, k, s.u.lu, tm, er);
+                if (tm.rank == 0)
+                    for (int i = tid; i < md.n; i += NT) vphi[i] = zexp(mk(0.0, 1.0) * k * md.pos[i * md.d]);
             }
-            if (!(wide ? lu_mixed<6>(A, md.n, ipiv, KIND != 0, s, X, tmem, ph)
-                       : lu_mixed<4>(A, md.n, ipiv, KIND != 0, s, X, tmem, ph))) {
-                alive = false;
-            } else if (KIND == 0) {
-                res = tracelog_df(A, md.n, ipiv, s);
+            tm.sync();
+            if (wide) lu_mixed<6>(A, md.n, ipiv, KIND != 0, s, X, tmem, ph, tm);
+            else lu_mixed<4>(A, md.n, ipiv, KIND != 0, s, X, tmem, ph, tm);
+            if (KIND == 0) {
+                if (tm.rank == 0) res = tracelog_df(A, md.n, ipiv, s);
             } else if (KIND == 1) {
-                if (!(wide ? trace_solve_mixed<6>(A, B, md.n, ipiv, s, X, tmem, ph, res)
-                           : trace_solve_mixed<4>(A, B, md.n, ipiv, s, X, tmem, ph, res)))
-                    alive = false;
+                res = wide ? trace_solve_mixed<6>(A, B, md.n, ipiv, s, X, tmem, ph, tm)
+                           : trace_solve_mixed<4>(A, B, md.n, ipiv, s, X, tmem, ph, tm);
             } else {
-                res = refine_solve(A, Mc, vphi, vx, vr, vt, md, k, ipiv, s);
-                if (P.amps)
+                res = refine_solve(A, Mc, vphi, vx, vr, vt, md, k, ipiv, s, tm);
+                if (P.amps && tm.rank == 0)
                     for (int i = tid; i < md.n; i += NT) {
                         P.amps[2 * (P.amp_off[it] + i)] = vx[i].re;
                         P.amps[2 * (P.amp_off[it] + i) + 1] = vx[i].im;
                     }
             }
         }
-        if (!alive) {
+        // a wait that ran out in some CTA: the team agrees to stop
+        __syncthreads();
+        int bad = s.err;
+        if (tm.size > 1) {
+            if (tid < tm.size) cluster_store(&s.team_rng[tm.rank][0], tid, bad);
+            tm.sync();
+            for (int r = 0; r < tm.size; ++r) bad |= s.team_rng[r][0];
+        }
+        if (bad) {
+            alive = false;
             st |= MSGPU_S_TIMEOUT;
             res = mk(nan(""), nan(""));
         }
-        if (tid == 0) {
+        if (tm.rank == 0 && tid == 0) {
             s.stat[PH_ITEMS] += 1;
             if (span_wide && !wide) st |= MSGPU_S_SPAN;
             P.out[2 * it] = res.re;
@@ -1301,9 +1471,9 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
             if (!isfinite(res.re) || !isfinite(res.im)) st |= MSGPU_S_NONFINITE;
             P.status[it] = st;
         }
-        __syncthreads();
+        tm.sync();
     }
-    if (s.err && tid == 0) {
+    if (!alive && tm.rank == 0 && tid == 0) {
         atomicExch(X.err, 1);
         // the run is abandoned: every item not yet taken is marked, none keeps a stale result
         for (unsigned q = atomicAdd(P.counter, 1u); q < P.counter[1] && (int)q < P.nitem;
@@ -1320,6 +1490,23 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
+}
+
+// launch or query of one variant
+template <int KIND, bool D3ONLY, class Team>
+static int mixed_variant(const EngineParams& P, const MixScratch& X, const MixLaunch& L) {
+    auto* kern = k_engine_mixed<KIND, D3ONLY, Team>;
+    static bool done[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return MSGPU_E_CUDA;
+    if (dev >= 64 || !done[dev]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MIX_SMEM_WIDE) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            return MSGPU_E_CUDA;
+        if (dev < 64) done[dev] = true;
+    }
+    if (L.query) return max_teams(kern, L.team, NT, L.smem);
+    return launch_teams(kern, L.teams, L.team, NT, L.smem, L.st, P, X);
 }
 #endif
 

@@ -1,0 +1,10 @@
+// One variant of the mixed-precision engine: job kind 0 (ln det), media of any dimension,
+// a cluster of CTAs per matrix.
+#define MSG_MIXED_KERNEL_BODY
+#include "mixed_engine.cuh"
+
+namespace msg {
+int mixed_team_0_any(const EngineParams& P, const MixScratch& X, const MixLaunch& L) {
+    return mixed_variant<0, false, ClusterTeam>(P, X, L);
+}
+}  // namespace msg
