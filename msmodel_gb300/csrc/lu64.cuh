@@ -81,6 +81,26 @@ __device__ __forceinline__ void cluster_store(double* p, int rank, double v) {
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
+// a 16-byte shared-memory variable of CTA `rank` of the cluster
+template <class E>
+__device__ __forceinline__ E cluster_load(const E* p, int rank) {
+    static_assert(sizeof(E) == 16, "one 128-bit load");
+    uint32_t a;
+    E v;
+    uint32_t* w = reinterpret_cast<uint32_t*>(&v);
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                 : "r"(a)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_store(long long* p, int rank, long long v) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+
 // shared memory of a CTA of NTH threads: NTH / 16 x 4 = TNC columns per DFMA tile
 template <int NTHREADS>
 struct __align__(16) LuSmemT {
@@ -88,6 +108,9 @@ struct __align__(16) LuSmemT {
     static constexpr int TNC = NTHREADS / 4;  // trailing-update tile columns (64 for 256 threads)
     zc As[NB][TM];       // 32 KB  L21 tile  (k-major)
     zc Bs[NB][TNC];      // U12 tile  (k-major)
+    // the two tiles' space holds a panel between updates
+    __device__ __forceinline__ void* panel_buf() { return &As[0][0]; }
+    static constexpr size_t PANEL_BYTES = sizeof(zc) * NB * (TM + TNC);
     zc T[NB][NB + 1];    // 16.5 KB diagonal block / assembly transpose
     zc urow[NB];         // pivot row of the panel
     zc piv, rpiv;        // the pivot and its reciprocal
@@ -592,6 +615,30 @@ struct DfmaUpdate {
     }
 };
 
+// A team's panels short enough are factored in shared memory (panel.cuh), by all
+// of it above PANEL_SOLO rows (below, a barrier a column costs more than the rows
+// it takes off the first CTA): one ln det at n = 1024 16.6 -> 8.7 ms, n = 300
+// 2.28 -> 1.69.  Longer ones, and those of a CTA alone, whose columns the FP64 pipe
+// bounds either way (n = 100: 708k cycles out of global memory, 742k in shared),
+// take panel_factor.
+constexpr int PANEL_SOLO = 64;
+struct PanelFp64;
+template <class E>
+__device__ __forceinline__ bool panel_fits(int m, int size, size_t bytes);
+template <class Ar, int NTH, class Team>
+static __device__ __noinline__ void panel_smem(typename Ar::E* A, int n, int j0, int jb, int* ipiv, void* buf, int& info,
+                                               Team tm);
+template <class S, class Team>
+__device__ __forceinline__ void factor_panel(zc* A, int n, int j0, int jb, int* ipiv, S& s, const Team& tm) {
+    const int m = n - j0;
+    if (tm.size > 1 && m > PANEL_SOLO && panel_fits<zc>(m, tm.size, S::PANEL_BYTES))
+        panel_smem<PanelFp64, S::NTH>(A, n, j0, jb, ipiv, s.panel_buf(), s.info, tm);
+    else if (tm.rank != 0) return;
+    else if (tm.size > 1 && panel_fits<zc>(m, 1, S::PANEL_BYTES))
+        panel_smem<PanelFp64, S::NTH>(A, n, j0, jb, ipiv, s.panel_buf(), s.info, Solo{});
+    else panel_factor(A, n, j0, jb, ipiv, s);
+}
+
 // In-place LU of A (n x n, ld n).  ipiv 0-based.  Sets s.info of the team's
 // first CTA (1-based first zero pivot).
 template <class S, class Team, class Update>
@@ -599,7 +646,7 @@ static __device__ void lu_factor(zc* A, int n, int* ipiv, bool keep_l, S& s, con
                                  const Update& update) {
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
-        if (tm.rank == 0) panel_factor(A, n, j0, jb, ipiv, s);
+        factor_panel(A, n, j0, jb, ipiv, s, tm);
         if (tm.size > 1) tm.sync();
         panel_swaps_trsm(A, n, j0, jb, ipiv, keep_l, s, tm);
         const int r0 = j0 + jb;
@@ -935,3 +982,5 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
 }
 
 }  // namespace msg
+
+#include "panel.cuh"
