@@ -236,7 +236,7 @@ static int pick_team(const int* teams, double s, double share, int nitem, int nm
     double t_best = 0.0;
     for (int j = 0; j < 5; ++j) {
         const int team = 1 << j, held = teams[j];
-        if (held < 1 || (team > 1 && nmax < 16 * team)) break;
+        if (held < 1 || (team > 1 && nmax < 6 * team)) break;
         const double waves = (nitem + held - 1) / held;
         const double t = waves * ((double)std::min(nitem, held) * team > g_sms ? share : 1.0) * (s + (1.0 - s) / team);
         if (j == 0 || t < 0.95 * t_best) {

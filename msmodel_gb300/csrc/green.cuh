@@ -139,6 +139,21 @@ MSG_D zc bessel_k_int(int nu, zc z) {
     return zsqrt(0.5 * PI / z) * zexp(-z) * bk_miller(nu, z);
 }
 
+// K_0(z) and K_1(z): the two integer orders of the d = 2 elements, with the
+// square root and the exponential in front of two of the regimes taken once
+MSG_D void bessel_k01(zc z, zc& k0, zc& k1) {
+    const double x = z.re, y = z.im;
+    const bool asym = x * x + y * y > 256.0;
+    if (!asym && x < 3.0 - y * y / 12.0) {
+        k0 = bk_series(0, z);
+        k1 = bk_series(1, z);
+        return;
+    }
+    const zc f = zsqrt(0.5 * PI / z) * zexp(-z);
+    k0 = f * (asym ? bk_asym(0, z) : bk_miller(0, z));
+    k1 = f * (asym ? bk_asym(1, z) : bk_miller(1, z));
+}
+
 // K_{twonu/2}(z); half-integer orders by the terminating expansion (DLMF 10.49.12),
 // integer orders >= 2 by forward recurrence from K_0, K_1.
 MSG_D zc bessel_k(int twonu, zc z) {

@@ -835,6 +835,15 @@ __device__ __forceinline__ void pair_elements(int d, zc k, double r, bool want_d
         if (want_deriv) dm = mk(-e.im, e.re) / FOURPI;
         return;
     }
+    if (d == 2 && want_deriv) {
+        // M = K_0(z) / (2 pi), dM/dk = -(k / 2 pi) G_0 = i r K_1(z) / (2 pi), z = -i k r (the general
+        // G_0 = -(-ik / (2 pi r))^-1 K_-1 / (2 pi) raises a complex power for every pair)
+        zc k0, k1;
+        bessel_k01(-(mk(-k.im, k.re) * r), k0, k1);
+        m = k0 / TWOPI;
+        dm = (r / TWOPI) * mk(-k1.im, k1.re);
+        return;
+    }
     m = -free_green(d, k, r);
     if (want_deriv) dm = -dk_free_green(d, k, r);
 }
@@ -857,10 +866,10 @@ __device__ __forceinline__ int k_regime(zc k, double r) {
 // fixed order, but every element is a function of (k, r) alone.
 template <int NTH, class Put>
 __device__ __forceinline__ void tile_pairs_grouped(int I, int J, int n, int d, const double* __restrict__ pos, zc k,
-                                                   bool want_deriv, unsigned short* list, int* cnt, Put put) {
+                                                   bool want_deriv, unsigned short* list, int* cnt, Put put, int q0 = 0,
+                                                   int q1 = 1024 / NTH) {
     const int tid = threadIdx.x;
-#pragma unroll
-    for (int q = 0; q < 1024 / NTH; ++q) {
+    for (int q = q0; q < q1; ++q) {
         const int p = tid + NTH * q, ii = p & 31, jj = p >> 5;
         const int i = I * 32 + ii, j = J * 32 + jj;
         if (i < n && j < n && i < j) {
@@ -895,7 +904,8 @@ struct EntryRange {
 // Assemble M(k) into A and, if B != nullptr, dM/dk into B (ld n, column-major).
 // Tiles of 32 x 32 pairs above the diagonal are evaluated once and written to
 // both triangles, the mirrored tile through shared memory to keep stores
-// coalesced; a team deals the tiles round robin.
+// coalesced.  A team deals out strips of a tile (NTH / 32 of its columns), round
+// robin: one dlogf at d = 2, n = 50 has three tiles, of which K_nu is the most work.
 template <class S, class Team>
 static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, int d, const double* __restrict__ pos,
                          const msgpu_model& mdl, zc k, S& s, const Team& tm, EntryRange& rg) {
@@ -919,10 +929,13 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
     if (grouped && tid < 3) cnt[tid] = 0;
     __syncthreads();
     const int nt = (n + 31) / 32;
-    int tile = 0;
-    for (int J = 0; J < nt; ++J) {
-        for (int I = 0; I <= J; ++I) {
-            if (tm.size > 1 && tile++ % tm.size != tm.rank) continue;
+    const int strips = tm.size > 1 ? NQ : 1, units = nt * (nt + 1) / 2 * strips;
+    int I = 0, J = 0, at = 0;  // tile of unit `at`
+    for (int u = tm.rank; u < units; u += tm.size) {
+        for (; at < u / strips; ++at)
+            if (++I > J) { I = 0; ++J; }
+        const int q0 = tm.size > 1 ? u % strips : 0, q1 = tm.size > 1 ? q0 + 1 : NQ;
+        {
             if (grouped) {
                 tile_pairs_grouped<NTH>(I, J, n, d, pos, k, B != nullptr, list, cnt, [&](int ii, int jj, zc m, zc dm) {
                     s.T[jj][ii] = m;
@@ -931,9 +944,8 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
                         T2[jj][ii] = dm;
                         rg.add(dm);
                     }
-                });
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
+                }, q0, q1);
+                for (int q = q0; q < q1; ++q) {
                     const int ii = tid & 31, jj = (tid >> 5) + RQ * q;
                     const int i = I * 32 + ii, j = J * 32 + jj;
                     if (i < n && j < n && i <= j) {
@@ -942,8 +954,7 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
                     }
                 }
             } else {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
+            for (int q = q0; q < q1; ++q) {
                 const int ii = tid & 31, jj = (tid >> 5) + RQ * q;
                 const int i = I * 32 + ii, j = J * 32 + jj;
                 if (i < n && j < n && i <= j) {
@@ -966,15 +977,16 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
             }
             }
             __syncthreads();
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const int jj = tid & 31, ii = (tid >> 5) + RQ * q;
-                const int i = I * 32 + ii, j = J * 32 + jj;
-                if (j < n && i < j) {
-                    A[j + (size_t)i * n] = s.T[jj][ii];
-                    if (B) B[j + (size_t)i * n] = T2[jj][ii];
+            // the mirrored elements: a lane takes a column j, of this unit's strip
+            const int jj = tid & 31, j = J * 32 + jj;
+            if (j < n && jj >= RQ * q0 && jj < RQ * q1)
+                for (int ii = tid >> 5; ii < 32; ii += RQ) {
+                    const int i = I * 32 + ii;
+                    if (i < j) {
+                        A[j + (size_t)i * n] = s.T[jj][ii];
+                        if (B) B[j + (size_t)i * n] = T2[jj][ii];
+                    }
                 }
-            }
             __syncthreads();
         }
     }
