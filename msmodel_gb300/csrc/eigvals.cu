@@ -18,8 +18,9 @@
 //      subdiagonals, the Ahues-Kressner deflation test, Wilkinson shifts with
 //      exceptional shifts every 10 iterations without deflation, the search
 //      for two consecutive small subdiagonals, 2 x 2 reflectors chasing the
-//      bulge through the active block): thread 0 takes the scalar chain of
-//      each bulge step, the CTA splits the step's row and column updates.
+//      bulge through the active block): warp 0 chases the bulge through a window
+//      of up to 30 steps on its diagonal block, the CTA takes the columns and
+//      rows outside it through the window's reflectors.
 // zgeev also balances the matrix first (zgebal); this path does not: M(k)'s
 // entries do not span the magnitudes balancing is for, and the eigenvalues
 // agree with the reference's to ~1e-13 of the largest.  Eigenvalues come out
@@ -114,35 +115,84 @@ static __device__ void hessenberg(zc* __restrict__ A, int n, LuSmem& s) {
 }
 
 // zlarfg for n = 2: on return a = beta (real), x scaled, the reflector
-// I - tau (1, x)(1, x)^H.  On the bulge-chasing chain of every QR step, so it
-// takes two divisions and one square root (zlarfg's dlapy3 scaling guards
-// against overflow of |a|^2 + |x|^2, far beyond M(k)'s entries)
+// I - tau (1, x)(1, x)^H.  On the bulge-chasing chain of every QR step: one square
+// root, then two independent divisions (zlarfg's dlapy3 scaling guards against
+// overflow of |a|^2 + |x|^2, far beyond M(k)'s entries)
 __device__ __forceinline__ zc larfg2(zc& a, zc& x) {
     const double x2 = zabs2(x);
     if (x2 == 0.0 && a.im == 0.0) return mk(0.0);
     const double beta = -copysign(sqrt(a.re * a.re + a.im * a.im + x2), a.re);
     const double rb = 1.0 / beta;
+    const zc d = a - beta;
+    const double rd = 1.0 / zabs2(d);
     const zc tau = mk((beta - a.re) * rb, -a.im * rb);
-    x = x * zrecip(a - beta);
+    x = x * mk(d.re * rd, -d.im * rd);
     a = mk(beta);
     return tau;
 }
 
-// the QR iteration's scalars, computed by thread 0 and read by the CTA
+// reflectors a bulge-chase window makes, and its rows and columns
+constexpr int HQR_W = 30, HQR_D = HQR_W + 2;
+
+// what the CTA shares in the QR iteration
 struct HqrShared {
-    zc t1, v2, temp;
-    double t2;
+    zc temp;
+    zc t1[2][HQR_W], v2[2][HQR_W];  // reflectors of the last two windows
+    double t2[2][HQR_W];
+    zc win[HQR_D][HQR_D + 1];       // the diagonal block of the window being chased
     int l, m, flag;
 };
 
+// One reflector (t1, v2, t2) on the pair (a, b) of a column, from the left
+__device__ __forceinline__ void hqr_left(zc t1, zc v2, double t2, zc& a, zc& b) {
+    const zc sum = conjz(t1) * a + t2 * b;
+    a -= sum;
+    b -= sum * v2;
+}
+// ... and on the pair (a, b) of a row, from the right
+__device__ __forceinline__ void hqr_right(zc t1, zc v2, double t2, zc& a, zc& b) {
+    const zc sum = t1 * a + t2 * b;
+    a -= sum;
+    b -= sum * conjz(v2);
+}
+
+// A window's ns reflectors (rows and columns lo..lo+ns) on columns [c0, c1] from the
+// left and on rows [r0, r1] from the right, a lane a column or row, 32 of them at a
+// time for warp w of nw.
+static __device__ void hqr_far(zc* __restrict__ H, int n, const HqrShared& q, int par, int lo, int ns, int c0, int c1, int r0,
+                               int r1, int w, int nw) {
+    const int lane = threadIdx.x & 31;
+    const int bc = c1 >= c0 ? (c1 - c0 + 32) / 32 : 0, br = r1 >= r0 ? (r1 - r0 + 32) / 32 : 0;
+    for (int b = w; b < bc + br; b += nw) {
+        const bool left = b < bc;
+        const int x = left ? c0 + 32 * b + lane : r0 + 32 * (b - bc) + lane;
+        if (x > (left ? c1 : r1)) continue;
+        zc* p = left ? H + lo + (size_t)x * n : H + x + (size_t)lo * n;
+        const size_t st = left ? 1 : n;
+        zc a = p[0];
+        for (int s = 0; s < ns; ++s) {
+            zc v = p[(s + 1) * st];
+            if (left) hqr_left(q.t1[par][s], q.v2[par][s], q.t2[par][s], a, v);
+            else hqr_right(q.t1[par][s], q.v2[par][s], q.t2[par][s], a, v);
+            p[s * st] = a;
+            a = v;
+        }
+        p[ns * st] = a;
+    }
+}
+
 // Eigenvalues of the upper Hessenberg H (n x n, ld n) into w by zlahqr's
-// single-shift QR (wantt = wantz = false).  Thread 0 takes every scalar step
-// (the deflation and shift searches, each 2 x 2 reflector) and the CTA splits
-// each step's row and column updates, three barriers a bulge step.  (Letting
-// thread 0 update the next reflector's two rows itself and start on it while
-// the CTA finishes the step saves a barrier but measured 10-16% slower.)  Returns 0,
-// or i + 1 if eigenvalue i and above did not converge within 30 max(10, n)
-// iterations (zlahqr's info).
+// single-shift QR (wantt = wantz = false).  A sweep is chased in windows of up to
+// HQR_W steps: warp 0 makes the reflectors on the window's diagonal block in
+// shared memory, every lane with the scalar chain to itself, a column or row of
+// the block each; then the CTA takes each column right of the block and each row
+// above it through all of the window's reflectors, a thread a column or row, the
+// next window's columns first and the rest beside the next window's chase.  (A
+// step at a time across the CTA, three barriers and three global round trips each,
+// took 8k cycles a step at n = 256: 415 ms for 64 matrices on as many SMs.)  The
+// deflation test and the search for the sweep's start look at 32 rows at once.
+// Returns 0, or i + 1 if eigenvalue i and above did not converge within
+// 30 max(10, n) iterations (zlahqr's info).
 static __device__ int hqr_cta(zc* __restrict__ H, int n, zc* __restrict__ w, HqrShared& q) {
     const int tid = threadIdx.x;
     auto h = [&](int r, int c) -> zc& { return H[r + (size_t)c * n]; };
@@ -178,33 +228,42 @@ static __device__ int hqr_cta(zc* __restrict__ H, int n, zc* __restrict__ w, Hqr
     constexpr int KEXSH = 10;
     int kdefl = 0;
     int i = ihi;
-    zc v0 = mk(0.0), v1 = mk(0.0);  // thread 0's reflector vector
+    zc v0 = mk(0.0), v1 = mk(0.0);  // warp 0's reflector vector
     while (i >= ilo) {
         int l = ilo;
         bool done = false;
         for (int its = 0; its <= itmax; ++its) {
-            if (tid == 0) {
-                // a single small subdiagonal element
-                int k;
-                for (k = i; k > l; --k) {
+            if (tid < 32) {
+                // a single small subdiagonal element: the largest k in (l, i] that has one, else l
+                auto small = [&](int k) {
                     const zc hkk1 = h(k, k - 1);
-                    if (abs1(hkk1) <= smlnum) break;
+                    if (abs1(hkk1) <= smlnum) return true;
                     double tst = abs1(h(k - 1, k - 1)) + abs1(h(k, k));
                     if (tst == 0.0) {
                         if (k - 2 >= ilo) tst += fabs(h(k - 1, k - 2).re);
                         if (k + 1 <= ihi) tst += fabs(h(k + 1, k).re);
                     }
-                    if (fabs(hkk1.re) <= ulp * tst) {
-                        const double a1 = abs1(hkk1), a2 = abs1(h(k - 1, k));
-                        const double ab = fmax(a1, a2), ba = fmin(a1, a2);
-                        const double b1 = abs1(h(k, k)), b2 = abs1(h(k - 1, k - 1) - h(k, k));
-                        const double aa = fmax(b1, b2), bb = fmin(b1, b2);
-                        const double sab = aa + ab;
-                        if (ba * (ab / sab) <= fmax(smlnum, ulp * (bb * (aa / sab)))) break;
+                    if (fabs(hkk1.re) > ulp * tst) return false;
+                    const double a1 = abs1(hkk1), a2 = abs1(h(k - 1, k));
+                    const double ab = fmax(a1, a2), ba = fmin(a1, a2);
+                    const double b1 = abs1(h(k, k)), b2 = abs1(h(k - 1, k - 1) - h(k, k));
+                    const double aa = fmax(b1, b2), bb = fmin(b1, b2);
+                    const double sab = aa + ab;
+                    return ba * (ab / sab) <= fmax(smlnum, ulp * (bb * (aa / sab)));
+                };
+                int k = l;
+                for (int top = i; top > l; top -= 32) {
+                    const unsigned hit = __ballot_sync(0xffffffffu, top - tid > l && small(top - tid));
+                    if (hit) {
+                        k = top - (__ffs(hit) - 1);
+                        break;
                     }
                 }
-                if (k > ilo) h(k, k - 1) = mk(0.0);
-                q.l = k;
+                __syncwarp();
+                if (tid == 0) {
+                    if (k > ilo) h(k, k - 1) = mk(0.0);
+                    q.l = k;
+                }
                 if (k < i) {
                     const int kd = kdefl + 1;
                     zc t;
@@ -229,28 +288,32 @@ static __device__ int hqr_cta(zc* __restrict__ H, int n, zc* __restrict__ w, Hqr
                             t = t - u * (u / (x + y));
                         }
                     }
-                    // two consecutive small subdiagonal elements: start the sweep at row m
-                    int m;
-                    for (m = i - 1; m > k; --m) {
-                        const zc h11 = h(m, m), h22 = h(m + 1, m + 1);
-                        zc h11s = h11 - t;
+                    // two consecutive small subdiagonal elements: start the sweep at row m,
+                    // the largest in (k, i-1] that has them, else k; the bulge's first vector
+                    auto start = [&](int m) {
+                        zc h11s = h(m, m) - t;
                         double h21 = h(m + 1, m).re;
-                        const double s = abs1(h11s) + fabs(h21);
-                        h11s = h11s / s;
-                        h21 /= s;
-                        v0 = h11s;
-                        v1 = mk(h21);
-                        const double h10 = h(m, m - 1).re;
-                        if (fabs(h10) * fabs(h21) <= ulp * (abs1(h11s) * (abs1(h11) + abs1(h22)))) break;
-                    }
-                    if (m == k) {
-                        const zc h11s = h(k, k) - t;
-                        const double h21 = h(k + 1, k).re;
                         const double s = abs1(h11s) + fabs(h21);
                         v0 = h11s / s;
                         v1 = mk(h21 / s);
+                    };
+                    int m = k;
+                    for (int top = i - 1; top > k; top -= 32) {
+                        bool ok = false;
+                        const int mm = top - tid;
+                        if (mm > k) {
+                            start(mm);
+                            const double h10 = h(mm, mm - 1).re;
+                            ok = fabs(h10) * fabs(v1.re) <= ulp * (abs1(v0) * (abs1(h(mm, mm)) + abs1(h(mm + 1, mm + 1))));
+                        }
+                        const unsigned hit = __ballot_sync(0xffffffffu, ok);
+                        if (hit) {
+                            m = top - (__ffs(hit) - 1);
+                            break;
+                        }
                     }
-                    q.m = m;
+                    start(m);
+                    if (tid == 0) q.m = m;
                 }
             }
             __syncthreads();
@@ -262,46 +325,64 @@ static __device__ int hqr_cta(zc* __restrict__ H, int n, zc* __restrict__ w, Hqr
             ++kdefl;
             const int i1 = l, i2 = i, m = q.m;
             // the single-shift QR sweep
-            for (int kk = m; kk < i; ++kk) {
-                if (tid == 0) {
-                    if (kk > m) {
-                        v0 = h(kk, kk - 1);
-                        v1 = h(kk + 1, kk - 1);
+            int prev_lo = 0, prev_hi = -1, prev_ns = 0, par = 0;  // the window whose far part is still to do
+            for (int lo = m; lo < i;) {
+                // a sweep that starts below l rescales the block after its first step: that one alone
+                const int ns = min(lo == m && m > l ? 1 : HQR_W, i - lo), hi = min(lo + ns + 1, i), dim = hi - lo + 1;
+                if (tid < 32) {
+                    for (int e = tid; e < dim * dim; e += 32) q.win[e % dim][e / dim] = h(lo + e % dim, lo + e / dim);
+                    if (lo > m) {
+                        v0 = h(lo, lo - 1);
+                        v1 = h(lo + 1, lo - 1);
                     }
-                    const zc t1 = larfg2(v0, v1);
-                    if (kk > m) {
-                        h(kk, kk - 1) = v0;
-                        h(kk + 1, kk - 1) = mk(0.0);
+                    __syncwarp();
+                    for (int s = 0; s < ns; ++s) {
+                        if (s > 0) {
+                            v0 = q.win[s][s - 1];
+                            v1 = q.win[s + 1][s - 1];
+                        }
+                        const zc t1 = larfg2(v0, v1);
+                        const zc v2 = v1;
+                        const double t2 = (t1 * v1).re;
+                        __syncwarp();
+                        if (tid == 0) {
+                            q.t1[par][s] = t1;
+                            q.v2[par][s] = v2;
+                            q.t2[par][s] = t2;
+                            if (s > 0) {
+                                q.win[s][s - 1] = v0;
+                                q.win[s + 1][s - 1] = mk(0.0);
+                            } else if (lo > m) {
+                                h(lo, lo - 1) = v0;
+                                h(lo + 1, lo - 1) = mk(0.0);
+                            }
+                        }
+                        if (tid >= s && tid < dim) hqr_left(t1, v2, t2, q.win[s][tid], q.win[s + 1][tid]);
+                        __syncwarp();
+                        if (tid <= min(s + 2, dim - 1)) hqr_right(t1, v2, t2, q.win[tid][s], q.win[tid][s + 1]);
+                        __syncwarp();
                     }
-                    q.t1 = t1;
-                    q.v2 = v1;
-                    q.t2 = (t1 * v1).re;
+                    for (int e = tid; e < dim * dim; e += 32) h(lo + e % dim, lo + e / dim) = q.win[e % dim][e / dim];
+                } else if (prev_ns > 0 && (tid >> 5) % 4 != 0) {
+                    // the far part of the window before, by the warps that do not share warp 0's FP64 pipe
+                    hqr_far(H, n, q, par ^ 1, prev_lo, prev_ns, min(prev_hi + HQR_D, i2) + 1, i2, i1, prev_lo - 1,
+                            (tid >> 5) / 4 * 3 + (tid >> 5) % 4 - 1, NT / 128 * 3);
                 }
                 __syncthreads();
-                const zc t1 = q.t1, v2 = q.v2;
-                const double t2 = q.t2;
-                // from the left: rows kk, kk+1, columns kk..i2
-                const zc ct1 = conjz(t1);
-                for (int j = kk + tid; j <= i2; j += NT) {
-                    const zc sum = ct1 * h(kk, j) + t2 * h(kk + 1, j);
-                    h(kk, j) -= sum;
-                    h(kk + 1, j) -= sum * v2;
-                }
+                // the columns of the next window first
+                hqr_far(H, n, q, par, lo, ns, hi + 1, min(hi + HQR_D, i2), 0, -1, tid >> 5, NT / 32);
                 __syncthreads();
-                // from the right: columns kk, kk+1, rows i1..min(kk+2, i)
-                const zc cv2 = conjz(v2);
-                const int jt = min(kk + 2, i);
-                for (int j = i1 + tid; j <= jt; j += NT) {
-                    const zc sum = t1 * h(j, kk) + t2 * h(j, kk + 1);
-                    h(j, kk) -= sum;
-                    h(j, kk + 1) -= sum * cv2;
-                }
-                if (kk == m && m > l) {
-                    // the sweep started below l: keep H(m, m-1) real.  Row j in S =
+                prev_lo = lo;
+                prev_hi = hi;
+                prev_ns = ns;
+                if (lo == m && m > l) {
+                    // far part at once, then keep H(m, m-1) real.  Row j in S =
                     // [m, i] \ {m+1} takes temp right of the diagonal, column j in S takes
                     // conj(temp) above it (zlahqr, one row and column at a time); an
                     // entry in both keeps its value
-                    zc temp = 1.0 - t1;
+                    hqr_far(H, n, q, par, lo, ns, min(hi + HQR_D, i2) + 1, i2, i1, lo - 1, tid >> 5, NT / 32);
+                    prev_ns = 0;
+                    zc temp = 1.0 - q.t1[par][0];
                     temp = temp / zabs(temp);
                     __syncthreads();
                     if (tid == 0) {
@@ -317,7 +398,13 @@ static __device__ int hqr_cta(zc* __restrict__ H, int n, zc* __restrict__ w, Hqr
                         if (a && !b) h(r, c) = h(r, c) * temp;
                         else if (b && !a) h(r, c) = h(r, c) * conjz(temp);
                     }
+                    __syncthreads();
                 }
+                lo += ns;
+                par ^= 1;
+            }
+            if (prev_ns > 0) {
+                hqr_far(H, n, q, par ^ 1, prev_lo, prev_ns, min(prev_hi + HQR_D, i2) + 1, i2, i1, prev_lo - 1, tid >> 5, NT / 32);
                 __syncthreads();
             }
             // H(i, i-1) made real
