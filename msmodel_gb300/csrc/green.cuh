@@ -182,6 +182,104 @@ MSG_D zc free_green(int d, zc k, double r) {
 
 MSG_D zc dk_free_green(int d, zc k, double r) { return (k / TWOPI) * free_green(d - 2, k, r); }
 
+// ---------------------------------------------------------------------------
+// e^{ikr} of d = 3 by tables, for the assembly of FP64 matrices: N^2/2 elements, and
+// the FP64 pipe (2 FMAs a clock per SM) is what bounds them.  The phase kr = Re k r
+// is reduced modulo pi/32 and the growth -Im k r modulo ln2/32 (two-part constants,
+// FMA, the product's own rounding error carried along), sin and cos of j pi/32 and
+// 2^{j/32} come from tables in global memory, the remainders from Taylor
+// polynomials (|y| <= pi/64: next terms below 2e-20; |y| <= ln2/64: below 4e-18), and the
+// addition theorem puts them together (table-driven evaluation as in Tang, ACM TOMS
+// 15, 144 (1989)).  About 35 FP64 operations where sincos and exp took about twice that.
+__device__ const double2 g_cis64[64] = {
+    {1.0, 0.0}, {0.9951847266721969, 0.0980171403295606},
+    {0.9807852804032304, 0.19509032201612828}, {0.9569403357322088, 0.2902846772544624},
+    {0.9238795325112867, 0.3826834323650898}, {0.881921264348355, 0.47139673682599764},
+    {0.8314696123025452, 0.5555702330196022}, {0.773010453362737, 0.6343932841636455},
+    {0.7071067811865476, 0.7071067811865476}, {0.6343932841636455, 0.773010453362737},
+    {0.5555702330196022, 0.8314696123025452}, {0.47139673682599764, 0.881921264348355},
+    {0.3826834323650898, 0.9238795325112867}, {0.2902846772544624, 0.9569403357322088},
+    {0.19509032201612828, 0.9807852804032304}, {0.0980171403295606, 0.9951847266721969},
+    {0.0, 1.0}, {-0.0980171403295606, 0.9951847266721969},
+    {-0.19509032201612828, 0.9807852804032304}, {-0.2902846772544624, 0.9569403357322088},
+    {-0.3826834323650898, 0.9238795325112867}, {-0.47139673682599764, 0.881921264348355},
+    {-0.5555702330196022, 0.8314696123025452}, {-0.6343932841636455, 0.773010453362737},
+    {-0.7071067811865476, 0.7071067811865476}, {-0.773010453362737, 0.6343932841636455},
+    {-0.8314696123025452, 0.5555702330196022}, {-0.881921264348355, 0.47139673682599764},
+    {-0.9238795325112867, 0.3826834323650898}, {-0.9569403357322088, 0.2902846772544624},
+    {-0.9807852804032304, 0.19509032201612828}, {-0.9951847266721969, 0.0980171403295606},
+    {-1.0, 0.0}, {-0.9951847266721969, -0.0980171403295606},
+    {-0.9807852804032304, -0.19509032201612828}, {-0.9569403357322088, -0.2902846772544624},
+    {-0.9238795325112867, -0.3826834323650898}, {-0.881921264348355, -0.47139673682599764},
+    {-0.8314696123025452, -0.5555702330196022}, {-0.773010453362737, -0.6343932841636455},
+    {-0.7071067811865476, -0.7071067811865476}, {-0.6343932841636455, -0.773010453362737},
+    {-0.5555702330196022, -0.8314696123025452}, {-0.47139673682599764, -0.881921264348355},
+    {-0.3826834323650898, -0.9238795325112867}, {-0.2902846772544624, -0.9569403357322088},
+    {-0.19509032201612828, -0.9807852804032304}, {-0.0980171403295606, -0.9951847266721969},
+    {0.0, -1.0}, {0.0980171403295606, -0.9951847266721969},
+    {0.19509032201612828, -0.9807852804032304}, {0.2902846772544624, -0.9569403357322088},
+    {0.3826834323650898, -0.9238795325112867}, {0.47139673682599764, -0.881921264348355},
+    {0.5555702330196022, -0.8314696123025452}, {0.6343932841636455, -0.773010453362737},
+    {0.7071067811865476, -0.7071067811865476}, {0.773010453362737, -0.6343932841636455},
+    {0.8314696123025452, -0.5555702330196022}, {0.881921264348355, -0.47139673682599764},
+    {0.9238795325112867, -0.3826834323650898}, {0.9569403357322088, -0.2902846772544624},
+    {0.9807852804032304, -0.19509032201612828}, {0.9951847266721969, -0.0980171403295606},
+};
+__device__ const double g_exp32[32] = {
+    1.0, 1.0218971486541166, 1.0442737824274138, 1.0671404006768237,
+    1.0905077326652577, 1.1143867425958924, 1.1387886347566916, 1.1637248587775775,
+    1.189207115002721, 1.215247359980469, 1.241857812073484, 1.2690509571917332,
+    1.2968395546510096, 1.3252366431597413, 1.3542555469368927, 1.383909881963832,
+    1.4142135623730951, 1.4451808069770467, 1.4768261459394993, 1.5091644275934228,
+    1.5422108254079407, 1.5759808451078865, 1.6104903319492543, 1.645755478153965,
+    1.681792830507429, 1.718619298122478, 1.7562521603732995, 1.7947090750031072,
+    1.8340080864093424, 1.8741676341103, 1.9152065613971474, 1.9571441241754002,
+};
+
+// cos and sin of k r
+MSG_D void cis_product(double k, double r, double& cs, double& sn) {
+    const double phi = k * r;
+    if (!(fabs(phi) < 1.0e5)) {
+        sincos(phi, &sn, &cs);
+        return;
+    }
+    const double e = fma(k, r, -phi);
+    const double t = fma(phi, 10.185916357881302, 6755399441055744.0);  // 32 / pi; 1.5 2^52 rounds to the nearest integer
+    const double q = t - 6755399441055744.0;
+    const double y = fma(-q, 3.827021247335479e-18, fma(-q, 0.09817477042468103, phi)) + e;
+    const double2 tab = g_cis64[__double2loint(t) & 63];
+    const double z = y * y;
+    const double s = fma(y * z, fma(z, fma(z, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), y);
+    const double c = z * fma(z, fma(z, fma(z, 1.0 / 40320.0, -1.0 / 720.0), 1.0 / 24.0), -0.5);  // cos y - 1
+    sn = tab.y + fma(tab.x, s, tab.y * c);
+    cs = tab.x + fma(-tab.y, s, tab.x * c);
+}
+
+// e^x
+MSG_D double exp_table(double x) {
+    if (!(fabs(x) < 690.0)) return exp(x);
+    const double t = fma(x, 46.16624130844683, 6755399441055744.0);  // 32 / ln 2
+    const double q = t - 6755399441055744.0;
+    const double y = fma(-q, 7.247021293269686e-19, fma(-q, 0.02166084939249829, x));
+    const int j = __double2loint(t);
+    const double p = y * fma(y, fma(y, fma(y, fma(y, fma(y, 1.0 / 720.0, 1.0 / 120.0), 1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0);
+    const double m = g_exp32[j & 31], v = fma(m, p, m);
+    return __hiloint2double(__double2hiint(v) + ((j >> 5) << 20), __double2loint(v));
+}
+
+// M_ij = e^{ikr} / (4 pi r) and dM_ij/dk = i e^{ikr} / (4 pi)
+MSG_D void pair_elements_d3(zc k, double r, bool want_deriv, zc& m, zc& dm) {
+    double cs, sn;
+    cis_product(k.re, r, cs, sn);
+    const double e = k.im != 0.0 ? exp_table(-k.im * r) : 1.0;
+    const double w = e / (FOURPI * r);
+    m = mk(w * cs, w * sn);
+    if (want_deriv) {
+        const double v = e * 0.07957747154594767;  // 1 / (4 pi)
+        dm = mk(-v * sn, v * cs);
+    }
+}
+
 // regularized 0F1(;a;z) power series (reference green_bessel.c:254)
 MSG_D zc hyp0f1(double a, zc z) {
     zc t = mk(1.0);

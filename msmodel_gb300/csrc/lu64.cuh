@@ -829,10 +829,7 @@ static __device__ void lu_solve_vec(const zc* A, zc* x, int n, const int* ipiv,
 // Off-diagonal matrix elements -G (and -dG/dk) for one pair distance.
 __device__ __forceinline__ void pair_elements(int d, zc k, double r, bool want_deriv, zc& m, zc& dm) {
     if (d == 3) {
-        // G = -e^{ikr}/(4 pi r);  dG/dk = (k/2pi) G_1 = (k/2pi) e^{ikr}/(2ik) = -i e^{ikr}/(4pi)
-        zc e = zexp(mk(-k.im * r, k.re * r));
-        m = e / (FOURPI * r);
-        if (want_deriv) dm = mk(-e.im, e.re) / FOURPI;
+        pair_elements_d3(k, r, want_deriv, m, dm);
         return;
     }
     if (d == 2 && want_deriv) {
