@@ -479,6 +479,21 @@ static __device__ void load_lower(const zc* A, int n, int j0, int jb, S& s) {
     __syncthreads();
 }
 
+// the upper triangle, its diagonal as reciprocals
+template <class S>
+static __device__ void load_upper(const zc* A, int n, int j0, int jb, S& s) {
+    for (int e = threadIdx.x; e < NB * NB; e += S::NTH) {
+        int r = e % NB, q = e / NB;
+        zc v = mk(r == q ? 1.0 : 0.0);
+        if (r < jb && q < jb && q >= r) {
+            v = A[(j0 + r) + (size_t)(j0 + q) * n];
+            if (q == r) v = 1.0 / v;
+        }
+        s.T[r][q] = v;
+    }
+    __syncthreads();
+}
+
 // Apply the panel's interchanges to every other column and compute
 // U12 = L11^-1 A12 (columns right of the panel).  keep_l = false leaves the
 // columns left of the panel alone: a ln det reads only U's diagonal and the
@@ -767,12 +782,13 @@ static __device__ zc lu_trace_solve(const zc* A, zc* B, int n, const int* ipiv,
 
 // x <- A^-1 x for one right-hand side x[n] (global), LAPACK-layout LU: the
 // interchanges, then blocked forward and backward substitution; each block's
-// small triangle is solved by warp 0 (one row per lane), the rectangular
-// remainder by all threads (one row per thread, coalesced column reads).
+// triangle comes into shared memory, with the reciprocals of U's diagonal (a
+// division a step by one lane held up the chain), and is solved by warp 0 (one row
+// per lane), the rectangular remainder by all threads (one row per thread,
+// coalesced column reads).
 template <class S>
-static __device__ void lu_solve_vec(const zc* A, zc* x, int n, const int* ipiv,
-                             S& s) {
-    const unsigned FULL = 0xffffffffu;
+static __device__ void lu_solve_vec(const zc* A, zc* x, int n, const int* ipiv, S& s) {
+    constexpr int NTH = S::NTH;
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid < 32)
         for (int j0 = 0; j0 < n; j0 += NB) {
@@ -786,43 +802,35 @@ static __device__ void lu_solve_vec(const zc* A, zc* x, int n, const int* ipiv,
             __syncwarp();
         }
     __syncthreads();
+    auto rows = [&](int j0, int jb, int r0, int r1) {
+        for (int i = r0 + tid; i < r1; i += NTH) {
+            zc acc = x[i];
+            const zc* a = A + i + (size_t)j0 * n;
+#pragma unroll 8
+            for (int q = 0; q < jb; ++q) acc = zfms(acc, a[(size_t)q * n], s.urow[q]);
+            x[i] = acc;
+        }
+        __syncthreads();
+    };
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
+        load_lower(A, n, j0, jb, s);
         if (tid < 32) {
-            zc v = lane < jb ? x[j0 + lane] : mk(0.0);
-            for (int q = 0; q < jb - 1; ++q) {
-                zc xq = mk(__shfl_sync(FULL, v.re, q), __shfl_sync(FULL, v.im, q));
-                if (lane > q && lane < jb) v -= A[(j0 + lane) + (size_t)(j0 + q) * n] * xq;
-            }
-            if (lane < jb) x[j0 + lane] = v;
+            const zc v = row_solve_lower_unit(lane < jb ? x[j0 + lane] : mk(0.0), jb, s.T);
+            if (lane < jb) x[j0 + lane] = s.urow[lane] = v;
         }
         __syncthreads();
-        for (int i = j0 + jb + tid; i < n; i += S::NTH) {
-            zc acc = x[i];
-            for (int q = 0; q < jb; ++q) acc -= A[i + (size_t)(j0 + q) * n] * x[j0 + q];
-            x[i] = acc;
-        }
-        __syncthreads();
+        rows(j0, jb, j0 + jb, n);
     }
-    const int nblk = (n + NB - 1) / NB;
-    for (int kb = nblk - 1; kb >= 0; --kb) {
-        const int j0 = kb * NB, jb = min(NB, n - j0);
+    for (int j0 = (n - 1) / NB * NB; j0 >= 0; j0 -= NB) {
+        const int jb = min(NB, n - j0);
+        load_upper(A, n, j0, jb, s);
         if (tid < 32) {
-            zc v = lane < jb ? x[j0 + lane] : mk(0.0);
-            for (int q = jb - 1; q >= 0; --q) {
-                if (lane == q) v = v / A[(j0 + q) + (size_t)(j0 + q) * n];
-                zc xq = mk(__shfl_sync(FULL, v.re, q), __shfl_sync(FULL, v.im, q));
-                if (lane < q) v -= A[(j0 + lane) + (size_t)(j0 + q) * n] * xq;
-            }
-            if (lane < jb) x[j0 + lane] = v;
+            const zc v = row_solve_upper(lane < jb ? x[j0 + lane] : mk(0.0), jb, s.T);
+            if (lane < jb) x[j0 + lane] = s.urow[lane] = v;
         }
         __syncthreads();
-        for (int i = tid; i < j0; i += S::NTH) {
-            zc acc = x[i];
-            for (int q = 0; q < jb; ++q) acc -= A[i + (size_t)(j0 + q) * n] * x[j0 + q];
-            x[i] = acc;
-        }
-        __syncthreads();
+        rows(j0, jb, 0, j0);
     }
 }
 

@@ -1205,74 +1205,58 @@ static __device__ zc tracelog_df(const float4* __restrict__ A, int n, const int*
 }
 
 // x <- (LU)^-1 x, one right-hand side, double-float (LAPACK-layout LU): the
-// interchanges, then blocked substitution; each block's triangle by warp 0
-// (one row per lane), the rectangular part by all threads (one row each)
-static __device__ void df_solve_vec(const float4* A, float4* x, int n, const int* ipiv, MixSmem& s) {
-    const unsigned FULL = 0xffffffffu;
+// interchanges, then blocked substitution; each block's triangle (the reciprocals
+// of U's diagonal with it) in shared memory by the team's first warp, one row per
+// lane, the rectangular part by all threads of the team, one row each.
+template <class Team>
+static __device__ void df_solve_vec(const float4* A, float4* x, int n, const int* ipiv, MixSmem& s, const Team& tm) {
     const int tid = threadIdx.x, lane = tid & 31;
-    if (tid < 32)
+    const dfc zero{df{0, 0}, df{0, 0}};
+    if (tm.rank == 0 && tid < 32)
         for (int j0 = 0; j0 < n; j0 += NB) {
             int inner, orow, ocur;
             panel_moves(ipiv, j0, min(NB, n - j0), inner, orow, ocur);
             move_rows(x, j0, min(NB, n - j0), inner, orow, ocur);
             __syncwarp();
         }
-    __syncthreads();
-    auto shfl4 = [&](float4 v, int src) {
-        return make_float4(__shfl_sync(FULL, v.x, src), __shfl_sync(FULL, v.y, src), __shfl_sync(FULL, v.z, src),
-                           __shfl_sync(FULL, v.w, src));
+    tm.sync();
+    auto rows = [&](int j0, int jb, int r0, int r1) {
+        tm.sync();  // the block's solution is there
+        if (tid < jb) s.u.p.urow[tid] = x[j0 + tid];
+        __syncthreads();
+        const int mine = cta_columns(r1 - r0, tm);  // rows dealt out in blocks of 32, like columns
+        for (int y = tid; y < mine; y += NT) {
+            const int i = r0 + cta_column(y, tm);
+            if (i >= r1) continue;
+            dfc acc = dfc_load(x + i);
+            const float4* a = A + i + (size_t)j0 * n;
+#pragma unroll 4
+            for (int q = 0; q < jb; ++q) acc = dfc_fms(acc, dfc_load(a + (size_t)q * n), dfc_load(&s.u.p.urow[q]));
+            dfc_store(x + i, acc);
+        }
+        tm.sync();
     };
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
-        if (tid < 32) {
-            float4 v = lane < jb ? x[j0 + lane] : make_float4(0, 0, 0, 0);
-            for (int q = 0; q < jb - 1; ++q) {
-                const float4 xq = shfl4(v, q);
-                if (lane > q && lane < jb) {
-                    dfc r = dfc_fms(dfc{df{v.x, v.y}, df{v.z, v.w}}, dfc_load(A + (j0 + lane) + (size_t)(j0 + q) * n),
-                                    dfc{df{xq.x, xq.y}, df{xq.z, xq.w}});
-                    v = make_float4(r.re.h, r.re.l, r.im.h, r.im.l);
-                }
+        if (tm.rank == 0) {
+            load_lower_block(A, n, j0, jb, s);
+            if (tid < 32) {
+                const dfc v = drow_lower_unit(lane < jb ? dfc_load(x + j0 + lane) : zero, jb, s.u.p.T);
+                if (lane < jb) dfc_store(x + j0 + lane, v);
             }
-            if (lane < jb) x[j0 + lane] = v;
         }
-        __syncthreads();
-        for (int i = j0 + jb + tid; i < n; i += NT) {
-            dfc acc = dfc_load(x + i);
-            for (int q = 0; q < jb; ++q) acc = dfc_fms(acc, dfc_load(A + i + (size_t)(j0 + q) * n), dfc_load(x + j0 + q));
-            dfc_store(x + i, acc);
-        }
-        __syncthreads();
+        rows(j0, jb, j0 + jb, n);
     }
-    const int nblk = (n + NB - 1) / NB;
-    for (int kb = nblk - 1; kb >= 0; --kb) {
-        const int j0 = kb * NB, jb = min(NB, n - j0);
-        if (tid < 32) {
-            float4 v = lane < jb ? x[j0 + lane] : make_float4(0, 0, 0, 0);
-            for (int q = jb - 1; q >= 0; --q) {
-                if (lane == q) {
-                    const dfc u = dfc_load(A + (j0 + q) + (size_t)(j0 + q) * n);
-                    const zc xv = mk(df_to_double(df{v.x, v.y}), df_to_double(df{v.z, v.w}));
-                    const zc qv = xv / mk(df_to_double(u.re), df_to_double(u.im));
-                    const df a = df_from_double(qv.re), b = df_from_double(qv.im);
-                    v = make_float4(a.h, a.l, b.h, b.l);
-                }
-                const float4 xq = shfl4(v, q);
-                if (lane < q) {
-                    dfc r = dfc_fms(dfc{df{v.x, v.y}, df{v.z, v.w}}, dfc_load(A + (j0 + lane) + (size_t)(j0 + q) * n),
-                                    dfc{df{xq.x, xq.y}, df{xq.z, xq.w}});
-                    v = make_float4(r.re.h, r.re.l, r.im.h, r.im.l);
-                }
+    for (int j0 = (n - 1) / NB * NB; j0 >= 0; j0 -= NB) {
+        const int jb = min(NB, n - j0);
+        if (tm.rank == 0) {
+            load_upper_block(A, n, j0, jb, s);
+            if (tid < 32) {
+                const dfc v = drow_upper(lane < jb ? dfc_load(x + j0 + lane) : zero, jb, s.u.p.T);
+                if (lane < jb) dfc_store(x + j0 + lane, v);
             }
-            if (lane < jb) x[j0 + lane] = v;
         }
-        __syncthreads();
-        for (int i = tid; i < j0; i += NT) {
-            dfc acc = dfc_load(x + i);
-            for (int q = 0; q < jb; ++q) acc = dfc_fms(acc, dfc_load(A + i + (size_t)(j0 + q) * n), dfc_load(x + j0 + q));
-            dfc_store(x + i, acc);
-        }
-        __syncthreads();
+        rows(j0, jb, 0, j0);
     }
 }
 
@@ -1281,7 +1265,7 @@ static __device__ void df_solve_vec(const float4* A, float4* x, int n, const int
 // a kept in FP64), until |r| <= 1e-14 |phi| (max norms), the residual stops
 // halving, or 8 corrections.  Returns sigma = -Im(conj(phi).a)/k (the optical
 // theorem of total_cross_section, ms_matrix_util.c:361).
-// The team shares the residuals (a row a thread), its first CTA takes the solves.
+// The team shares the residuals (a row a thread) and the solves' rectangular parts.
 template <class Team>
 static __device__ zc refine_solve(const float4* LU, const zc* M, const zc* phi, zc* x, float4* r, float4* t, const MedDev& md,
                            zc k, const int* ipiv, MixSmem& s, const Team& tm) {
@@ -1290,15 +1274,15 @@ static __device__ zc refine_solve(const float4* LU, const zc* M, const zc* phi, 
         const df a = df_from_double(v.re), b = df_from_double(v.im);
         return make_float4(a.h, a.l, b.h, b.l);
     };
-    if (tm.rank == 0) {
+    if (tm.rank == 0)
         for (int i = tid; i < n; i += NT) t[i] = to4(phi[i]);
-        __syncthreads();
-        df_solve_vec(LU, t, n, ipiv, s);
+    __syncthreads();
+    df_solve_vec(LU, t, n, ipiv, s, tm);
+    if (tm.rank == 0)
         for (int i = tid; i < n; i += NT) {
             const dfc v = dfc_load(t + i);
             x[i] = mk(df_to_double(v.re), df_to_double(v.im));
         }
-    }
     tm.sync();
     double pmax = 0.0;
     for (int i = tid; i < n; i += NT) pmax = fmax(pmax, zabs(phi[i]));
@@ -1330,13 +1314,12 @@ static __device__ zc refine_solve(const float4* LU, const zc* M, const zc* phi, 
         }
         if (!(rmax > 1e-14 * pmax) || !(rmax < 0.5 * prev)) break;
         prev = rmax;
-        if (tm.rank == 0) {
-            df_solve_vec(LU, r, n, ipiv, s);
+        df_solve_vec(LU, r, n, ipiv, s, tm);
+        if (tm.rank == 0)
             for (int i = tid; i < n; i += NT) {
                 const dfc v = dfc_load(r + i);
                 x[i] = x[i] + mk(df_to_double(v.re), df_to_double(v.im));
             }
-        }
         tm.sync();
     }
     double dr = 0.0, di = 0.0, z = 0.0;
@@ -1459,9 +1442,11 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
                 // incident plane wave along +x (incident_wave_util.c:76)
                 EntryRange er;
                 __syncthreads();
+                stat_start(s);
                 assemble(Mc, nullptr, md.n, md.d, md.pos, md.model, k, s.u.lu, tm, er);
                 if (tm.rank == 0)
                     for (int i = tid; i < md.n; i += NT) vphi[i] = zexp(mk(0.0, 1.0) * k * md.pos[i * md.d]);
+                stat_add(s, PH_ASSEMBLE);
             }
             tm.sync();
             if (wide) lu_mixed<6>(A, md.n, ipiv, KIND != 0, s, X, tmem, ph, tm);
@@ -1472,7 +1457,9 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
                 res = wide ? trace_solve_mixed<6>(A, B, md.n, ipiv, s, X, tmem, ph, tm)
                            : trace_solve_mixed<4>(A, B, md.n, ipiv, s, X, tmem, ph, tm);
             } else {
+                stat_start(s);
                 res = refine_solve(A, Mc, vphi, vx, vr, vt, md, k, ipiv, s, tm);
+                stat_add(s, PH_SOLVE);
                 if (P.amps && tm.rank == 0)
                     for (int i = tid; i < md.n; i += NT) {
                         P.amps[2 * (P.amp_off[it] + i)] = vx[i].re;
