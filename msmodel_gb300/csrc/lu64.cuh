@@ -101,16 +101,16 @@ __device__ __forceinline__ void cluster_store(long long* p, int rank, long long 
     asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
 
-// shared memory of a CTA of NTH threads: NTH / 16 x 4 = TNC columns per DFMA tile
-template <int NTHREADS>
+// shared memory of a CTA of NTH threads: tiles of TMR rows, NTH / 16 x 4 = TNC columns
+template <int NTHREADS, int TILE_ROWS = TM>
 struct __align__(16) LuSmemT {
-    static constexpr int NTH = NTHREADS;
+    static constexpr int NTH = NTHREADS, TMR = TILE_ROWS;
     static constexpr int TNC = NTHREADS / 4;  // trailing-update tile columns (64 for 256 threads)
-    zc As[NB][TM];       // 32 KB  L21 tile  (k-major)
+    zc As[NB][TMR];      // L21 tile  (k-major; 32 KB for 64 rows)
     zc Bs[NB][TNC];      // U12 tile  (k-major)
     // the two tiles' space holds a panel between updates
     __device__ __forceinline__ void* panel_buf() { return &As[0][0]; }
-    static constexpr size_t PANEL_BYTES = sizeof(zc) * NB * (TM + TNC);
+    static constexpr size_t PANEL_BYTES = sizeof(zc) * NB * (TMR + TNC);
     zc T[NB][NB + 1];    // 16.5 KB diagonal block / assembly transpose
     zc urow[NB];         // pivot row of the panel
     zc piv, rpiv;        // the pivot and its reciprocal
@@ -612,8 +612,8 @@ static __device__ void gemm_sub_r(zc* C, int ldc, const zc* Ab, int lda, const z
 template <class S, class Team>
 static __device__ void gemm_sub(zc* C, int ldc, const zc* Ab, int lda, const zc* Bb, int ldb, int m, int nn, int kk, S& s,
                          const Team& tm, int tri = 0) {
-    if (m <= 32 || nn <= 32) gemm_sub_r<2>(C, ldc, Ab, lda, Bb, ldb, m, nn, kk, s, tm, tri);
-    else gemm_sub_r<4>(C, ldc, Ab, lda, Bb, ldb, m, nn, kk, s, tm, tri);
+    if (S::TMR < TM || m <= 32 || nn <= 32) gemm_sub_r<2>(C, ldc, Ab, lda, Bb, ldb, m, nn, kk, s, tm, tri);
+    else if constexpr (S::TMR >= TM) gemm_sub_r<4>(C, ldc, Ab, lda, Bb, ldb, m, nn, kk, s, tm, tri);
 }
 
 // the trailing update on the FP64 pipe (DFMA); another kernel may pass its own
@@ -927,8 +927,10 @@ static __device__ void assemble(zc* __restrict__ A, zc* __restrict__ B, int n, i
     rg.add(dg0);
     if (B) rg.add(dg1);
     zc (*T2)[NB + 1] = reinterpret_cast<zc(*)[NB + 1]>(&s.As[0][0]);
-    // d != 3: pair lists of the regime grouping in the (idle) U12 tile buffer
-    unsigned short* list = reinterpret_cast<unsigned short*>(&s.Bs[0][0]);
+    // d != 3: pair lists of the regime grouping behind it, in the (idle) tile buffers
+    constexpr size_t T2_BYTES = sizeof(zc) * NB * (NB + 1), AS_BYTES = sizeof(zc) * NB * S::TMR;
+    unsigned short* list = reinterpret_cast<unsigned short*>(reinterpret_cast<char*>(&s.As[0][0]) +
+                                                             (AS_BYTES > T2_BYTES ? AS_BYTES : T2_BYTES));
     int* cnt = reinterpret_cast<int*>(list + 3 * 1024);
     const bool grouped = d != 3 && d != 1;
     if (grouped && tid < 3) cnt[tid] = 0;

@@ -61,7 +61,7 @@ constexpr int TC_BAD = 1 << 20;  // exponent of a row or column with an infinity
 // shared memory: what lasts through an item, then the FP64 pipe's tiles (panel,
 // TRSM, assembly; names as in LuSmemT) over the tensor core's operand buffers
 struct Tc64Smem {
-    static constexpr int NTH = TC_NT, TNC = TC_NT / 4;
+    static constexpr int NTH = TC_NT, TNC = TC_NT / 4, TMR = TM;
     static constexpr size_t PANEL_BYTES = TC_ABAND + 2 * (size_t)((TC_BTILE + 127) / 128 * 128);
     __device__ __forceinline__ void* panel_buf() { return g.a; }  // a panel between updates
     uint64_t bar_b[2], bar_mma;
