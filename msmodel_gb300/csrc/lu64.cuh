@@ -439,6 +439,12 @@ __device__ __forceinline__ int cta_column(int x, const Team& tm) { return ((x >>
 // (~2k cycles a column on the whole SM, against ~127k for up to 128 columns with
 // a thread each: 166k -> 59k cycles a panel at n = 100)
 __device__ __forceinline__ bool few_columns(int cols) { return cols <= 64; }
+// ... so of a CTA's columns as many go a thread each as fill its nth threads, and
+// the rest too unless they are few
+__device__ __forceinline__ int thread_columns(int cols, int nth) {
+    const int full = cols / nth * nth;
+    return few_columns(cols - full) ? full : cols;
+}
 
 // The net effect of a panel's interchanges, worked out by every warp for
 // itself: row j0 + lane receives row `inner`, and row `orow` (-1: none), one of
@@ -507,7 +513,7 @@ static __device__ void panel_swaps_trsm(zc* A, int n, int j0, int jb, const int*
     panel_moves(ipiv, j0, jb, inner, orow, ocur);
     const bool moves = __any_sync(0xffffffffu, inner != j0 + lane);
     const int right = j0 + jb, nr = cta_columns(n - right, tm);
-    const bool few = few_columns(nr);
+    const int wide = thread_columns(nr, S::NTH);  // the first `wide` a thread each
     if (keep_l && moves) {
         const int nl = cta_columns(j0, tm);
         for (int x = warp; x < nl; x += NW) {
@@ -520,21 +526,21 @@ static __device__ void panel_swaps_trsm(zc* A, int n, int j0, int jb, const int*
             if (orow >= 0) a[orow] = w;
         }
     }
-    if (few || moves)
-        for (int x = warp; x < nr; x += NW) {
+    if (wide < nr || moves)
+        for (int x = (moves ? 0 : wide) + warp; x < nr; x += NW) {
             const int col = right + cta_column(x, tm);
             if (col >= n) continue;
             zc* a = A + (size_t)col * n;
             zc v = lane < jb ? a[inner] : mk(0.0);
             const zc w = orow >= 0 ? a[ocur] : mk(0.0);
             __syncwarp();
-            if (few) v = row_solve_lower_unit(v, jb, s.T);
+            if (x >= wide) v = row_solve_lower_unit(v, jb, s.T);
             if (lane < jb) a[j0 + lane] = v;
             if (orow >= 0) a[orow] = w;
         }
-    if (!few) {
+    if (wide > 0) {
         __syncthreads();
-        for (int x = tid; x < nr; x += S::NTH) {
+        for (int x = tid; x < wide; x += S::NTH) {
             const int col = right + cta_column(x, tm);
             if (col < n) col_solve_lower_unit(A + (size_t)col * n + j0, jb, s.T);
         }
@@ -717,19 +723,17 @@ static __device__ zc lu_trace_solve(const zc* A, zc* B, int n, const int* ipiv,
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
         load_lower(A, n, j0, jb, s);
-        if (few_columns(mine)) {
-            for (int x = warp; x < mine; x += NW) {
-                const int col = cta_column(x, tm);
-                if (col >= n) continue;
-                zc* b = B + (size_t)col * n + j0;
-                const zc v = row_solve_lower_unit(lane < jb ? b[lane] : mk(0.0), jb, s.T);
-                if (lane < jb) b[lane] = v;
-            }
-        } else {
-            for (int x = tid; x < mine; x += NTH) {
-                const int col = cta_column(x, tm);
-                if (col < n) col_solve_lower_unit(B + (size_t)col * n + j0, jb, s.T);
-            }
+        const int wide = thread_columns(mine, NTH);
+        for (int x = wide + warp; x < mine; x += NW) {
+            const int col = cta_column(x, tm);
+            if (col >= n) continue;
+            zc* b = B + (size_t)col * n + j0;
+            const zc v = row_solve_lower_unit(lane < jb ? b[lane] : mk(0.0), jb, s.T);
+            if (lane < jb) b[lane] = v;
+        }
+        for (int x = tid; x < wide; x += NTH) {
+            const int col = cta_column(x, tm);
+            if (col < n) col_solve_lower_unit(B + (size_t)col * n + j0, jb, s.T);
         }
         tm.sync();
         const int r0 = j0 + jb;
@@ -740,30 +744,19 @@ static __device__ zc lu_trace_solve(const zc* A, zc* B, int n, const int* ipiv,
     const int nblk = (n + NB - 1) / NB;
     for (int kb = nblk - 1; kb >= 0; --kb) {
         const int j0 = kb * NB, jb = min(NB, n - j0), ncol = j0 + jb;
-        for (int e = tid; e < NB * NB; e += NTH) {
-            int r = e % NB, q = e / NB;
-            zc v = mk(r == q ? 1.0 : 0.0);
-            if (r < jb && q < jb && q >= r) {
-                v = A[(j0 + r) + (size_t)(j0 + q) * n];
-                if (q == r) v = 1.0 / v;
-            }
-            s.T[r][q] = v;
-        }
-        __syncthreads();
+        load_upper(A, n, j0, jb, s);
         const int cols = cta_columns(ncol, tm);
-        if (few_columns(cols)) {
-            for (int x = warp; x < cols; x += NW) {
-                const int col = cta_column(x, tm);
-                if (col >= ncol) continue;
-                zc* b = B + (size_t)col * n + j0;
-                const zc v = row_solve_upper(lane < jb ? b[lane] : mk(0.0), jb, s.T);
-                if (lane < jb) b[lane] = v;
-            }
-        } else {
-            for (int x = tid; x < cols; x += NTH) {
-                const int col = cta_column(x, tm);
-                if (col < ncol) col_solve_upper(B + (size_t)col * n + j0, jb, s.T);
-            }
+        const int wide = thread_columns(cols, NTH);
+        for (int x = wide + warp; x < cols; x += NW) {
+            const int col = cta_column(x, tm);
+            if (col >= ncol) continue;
+            zc* b = B + (size_t)col * n + j0;
+            const zc v = row_solve_upper(lane < jb ? b[lane] : mk(0.0), jb, s.T);
+            if (lane < jb) b[lane] = v;
+        }
+        for (int x = tid; x < wide; x += NTH) {
+            const int col = cta_column(x, tm);
+            if (col < ncol) col_solve_upper(B + (size_t)col * n + j0, jb, s.T);
         }
         tm.sync();
         // Y[0:j0, 0:ncol] -= U[0:j0, j0:j0+jb] X[j0:j0+jb, 0:ncol]   (rows >= cols only)

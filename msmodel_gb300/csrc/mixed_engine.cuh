@@ -797,7 +797,7 @@ static __device__ void df_swaps_trsm(float4* A, int n, int j0, int jb, const int
     panel_moves(ipiv, j0, jb, inner, orow, ocur);
     const bool moves = __any_sync(0xffffffffu, inner != j0 + lane);
     const int right = j0 + jb, nr = cta_columns(n - right, tm);
-    const bool few = few_columns(nr);
+    const int wide = thread_columns(nr, NT);  // the first `wide` a thread each
     if (keep_l && moves) {
         const int nl = cta_columns(j0, tm);
         for (int x = warp; x < nl; x += NW) {
@@ -810,18 +810,16 @@ static __device__ void df_swaps_trsm(float4* A, int n, int j0, int jb, const int
             const int col = right + cta_column(x, tm);
             if (col < n) move_rows(A + (size_t)col * n, j0, jb, inner, orow, ocur);
         }
-    if (few) {
-        __syncwarp();  // a warp solves the columns it moved
-        for (int x = warp; x < nr; x += NW) {
-            const int col = right + cta_column(x, tm);
-            if (col >= n) continue;
-            float4* a = A + (size_t)col * n + j0;
-            const dfc v = drow_lower_unit(lane < jb ? dfc_load(a + lane) : dfc{df{0, 0}, df{0, 0}}, jb, s.u.p.T);
-            if (lane < jb) dfc_store(a + lane, v);
-        }
-    } else {
-        __syncthreads();
-        for (int x = tid; x < nr; x += NT) {
+    __syncthreads();
+    for (int x = wide + warp; x < nr; x += NW) {
+        const int col = right + cta_column(x, tm);
+        if (col >= n) continue;
+        float4* a = A + (size_t)col * n + j0;
+        const dfc v = drow_lower_unit(lane < jb ? dfc_load(a + lane) : dfc{df{0, 0}, df{0, 0}}, jb, s.u.p.T);
+        if (lane < jb) dfc_store(a + lane, v);
+    }
+    if (wide > 0) {
+        for (int x = tid; x < wide; x += NT) {
             const int col = right + cta_column(x, tm);
             if (col < n) dcol_lower_unit(A + (size_t)col * n + j0, jb, s.u.p.T);
         }
@@ -870,19 +868,17 @@ static __device__ zc trace_solve_mixed(const float4* A, float4* B, int n, const 
     for (int j0 = 0; j0 < n; j0 += NB) {
         const int jb = min(NB, n - j0);
         load_lower_block(A, n, j0, jb, s);
-        if (few_columns(mine)) {
-            for (int x = warp; x < mine; x += NW) {
-                const int col = cta_column(x, tm);
-                if (col >= n) continue;
-                float4* b = B + (size_t)col * n + j0;
-                const dfc v = drow_lower_unit(lane < jb ? dfc_load(b + lane) : zero, jb, s.u.p.T);
-                if (lane < jb) dfc_store(b + lane, v);
-            }
-        } else {
-            for (int x = tid; x < mine; x += NT) {
-                const int col = cta_column(x, tm);
-                if (col < n) dcol_lower_unit(B + (size_t)col * n + j0, jb, s.u.p.T);
-            }
+        const int wide = thread_columns(mine, NT);
+        for (int x = wide + warp; x < mine; x += NW) {
+            const int col = cta_column(x, tm);
+            if (col >= n) continue;
+            float4* b = B + (size_t)col * n + j0;
+            const dfc v = drow_lower_unit(lane < jb ? dfc_load(b + lane) : zero, jb, s.u.p.T);
+            if (lane < jb) dfc_store(b + lane, v);
+        }
+        for (int x = tid; x < wide; x += NT) {
+            const int col = cta_column(x, tm);
+            if (col < n) dcol_lower_unit(B + (size_t)col * n + j0, jb, s.u.p.T);
         }
         tm.sync();
         const int r0 = j0 + jb;
@@ -894,19 +890,17 @@ static __device__ zc trace_solve_mixed(const float4* A, float4* B, int n, const 
         const int j0 = kb * NB, jb = min(NB, n - j0), ncol = j0 + jb;
         load_upper_block(A, n, j0, jb, s);
         const int cols = cta_columns(ncol, tm);
-        if (few_columns(cols)) {
-            for (int x = warp; x < cols; x += NW) {
-                const int col = cta_column(x, tm);
-                if (col >= ncol) continue;
-                float4* b = B + (size_t)col * n + j0;
-                const dfc v = drow_upper(lane < jb ? dfc_load(b + lane) : zero, jb, s.u.p.T);
-                if (lane < jb) dfc_store(b + lane, v);
-            }
-        } else {
-            for (int x = tid; x < cols; x += NT) {
-                const int col = cta_column(x, tm);
-                if (col < ncol) dcol_upper(B + (size_t)col * n + j0, jb, s.u.p.T);
-            }
+        const int wide = thread_columns(cols, NT);
+        for (int x = wide + warp; x < cols; x += NW) {
+            const int col = cta_column(x, tm);
+            if (col >= ncol) continue;
+            float4* b = B + (size_t)col * n + j0;
+            const dfc v = drow_upper(lane < jb ? dfc_load(b + lane) : zero, jb, s.u.p.T);
+            if (lane < jb) dfc_store(b + lane, v);
+        }
+        for (int x = tid; x < wide; x += NT) {
+            const int col = cta_column(x, tm);
+            if (col < ncol) dcol_upper(B + (size_t)col * n + j0, jb, s.u.p.T);
         }
         tm.sync();
         mixed_gemm_sub<NS>(B, n, A + (size_t)j0 * n, n, B + j0, n, j0, ncol, jb, 1, s, X, tmem, ph, tm);
