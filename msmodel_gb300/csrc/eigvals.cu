@@ -114,21 +114,31 @@ static __device__ void hessenberg(zc* __restrict__ A, int n, LuSmem& s) {
     }
 }
 
-// zlarfg for n = 2: on return a = beta (real), x scaled, the reflector
-// I - tau (1, x)(1, x)^H.  On the bulge-chasing chain of every QR step: one square
-// root, then two independent divisions (zlarfg's dlapy3 scaling guards against
-// overflow of |a|^2 + |x|^2, far beyond M(k)'s entries)
-__device__ __forceinline__ zc larfg2(zc& a, zc& x) {
-    const double x2 = zabs2(x);
-    if (x2 == 0.0 && a.im == 0.0) return mk(0.0);
-    const double beta = -copysign(sqrt(a.re * a.re + a.im * a.im + x2), a.re);
-    const double rb = 1.0 / beta;
-    const zc d = a - beta;
-    const double rd = 1.0 / zabs2(d);
-    const zc tau = mk((beta - a.re) * rb, -a.im * rb);
-    x = x * mk(d.re * rd, -d.im * rd);
+// zlarfg for n = 2 and real x: on return a = beta (real), v2 the reflector's second
+// entry, the reflector I - t1 (1, v2)(1, v2)^H, and t2 = t1 v2, which is real.  (The
+// bulge's lower entry is a product of t2 and a subdiagonal entry, both real.)  The
+// warp that chases the bulge is bound by how many FP64 instructions it issues, 64
+// clocks each: one reciprocal square root gives beta and 1 / beta, one division the
+// rest, 32 of them in all where a square root, two divisions and complex products
+// took 47 (zlarfg's dlapy3 scaling guards against overflow of |a|^2 + x^2, far
+// beyond M(k)'s entries).
+__device__ __forceinline__ void larfg2(zc& a, double x, zc& t1, zc& v2, double& t2) {
+    const double b2 = fma(x, x, fma(a.re, a.re, a.im * a.im));
+    if (x == 0.0 && a.im == 0.0) {
+        t1 = v2 = mk(0.0);
+        t2 = 0.0;
+        return;
+    }
+    const double rs = rsqrt(b2);
+    double beta = b2 * rs;
+    beta = -copysign(fma(0.5 * rs, fma(-beta, beta, b2), beta), a.re);
+    const double rb = copysign(rs, beta);
+    const zc d = mk(a.re - beta, a.im);
+    t1 = mk(-d.re * rb, -d.im * rb);
+    t2 = -x * rb;
+    const double y = x / fma(d.re, d.re, d.im * d.im);
+    v2 = mk(d.re * y, -d.im * y);
     a = mk(beta);
-    return tau;
 }
 
 // reflectors a bulge-chase window makes, and its rows and columns
@@ -341,9 +351,9 @@ static __device__ int hqr_cta(zc* __restrict__ H, int n, zc* __restrict__ w, Hqr
                             v0 = q.win[s][s - 1];
                             v1 = q.win[s + 1][s - 1];
                         }
-                        const zc t1 = larfg2(v0, v1);
-                        const zc v2 = v1;
-                        const double t2 = (t1 * v1).re;
+                        zc t1, v2;
+                        double t2;
+                        larfg2(v0, v1.re, t1, v2, t2);
                         __syncwarp();
                         if (tid == 0) {
                             q.t1[par][s] = t1;
