@@ -593,7 +593,7 @@ msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int n
     } else if (nitem < held && te.ctas != 1) {
         // a mixed job may turn wide with later points: count the teams of the wide launch
         int teams[5] = {held, 0, 0, 0, 0};
-        for (int j = 1; j < 5; ++j) teams[j] = mixed_max_teams(kind, J->d3only, 1 << j, true);
+        for (int j = 1; j < 5; ++j) teams[j] = mixed_max_teams(kind, J->d3only, 1 << j);
         J->team = pick_team(teams, 0.25, 1.6, nitem, J->nmax);
         held = teams[ilog2(J->team)];
     }

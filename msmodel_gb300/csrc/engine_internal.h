@@ -96,8 +96,8 @@ constexpr int TC_NMIN = 97;
 // P.wide_ok: launch with the shared memory for six-way slicing; grid matrices at a time,
 // `team` CTAs on each.
 int mixed_run(const EngineParams& P, int grid, int team, int nmax, bool d3only, cudaStream_t st);
-// clusters of `team` CTAs of that variant the device holds at once (0: none of that size)
-int mixed_max_teams(int kind, bool d3only, int team, bool wide);
+// clusters of `team` CTAs of that variant's wide launch the device holds at once (0: none of that size)
+int mixed_max_teams(int kind, bool d3only, int team);
 // Allocates the mixed engine's scratch for `grid` matrices up to nmax
 // (mixed_run does so itself; called before a stream capture, which must not allocate).
 int mixed_prepare(int grid, int nmax);

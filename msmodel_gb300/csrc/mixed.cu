@@ -74,9 +74,19 @@ unsigned long long mixed_generation() {
     return g_mix_gen;
 }
 
-int mixed_max_teams(int kind, bool d3only, int team, bool wide) {
-    return variant(kind, d3only, team)(EngineParams{}, MixScratch{},
-                                       {0, team, wide ? MIX_SMEM_WIDE : MIX_SMEM_NARROW, nullptr, true});
+// clusters of the wide launch (asked for at every small job's creation: kept per
+// device, the query takes tens of microseconds)
+int mixed_max_teams(int kind, bool d3only, int team) {
+    static int held[64][6][5];  // 1 + the answer
+    int dev = 0, j = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    while ((1 << j) < team) ++j;
+    std::lock_guard<std::mutex> lk(g_mx);
+    int* h = dev < 64 && j < 5 ? &held[dev][(d3only ? 0 : 3) + (kind < 0 ? 0 : kind > 2 ? 2 : kind)][j] : nullptr;
+    if (h && *h) return *h - 1;
+    const int n = variant(kind, d3only, team)(EngineParams{}, MixScratch{}, {0, team, MIX_SMEM_WIDE, nullptr, true});
+    if (h && n >= 0) *h = 1 + n;
+    return n < 0 ? 0 : n;
 }
 
 int mixed_run(const EngineParams& P, int grid, int team, int nmax, bool d3only, cudaStream_t st) {

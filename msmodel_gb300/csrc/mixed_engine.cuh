@@ -60,8 +60,12 @@ constexpr float SPAN_WIDE_REFINED = 1048576.0f;
 
 // slice configurations: NS slices per operand, TN tile columns, NG TMEM accumulator groups
 template <int NS> struct SliceCfg;
-template <> struct SliceCfg<4> { static constexpr int TN = 32, NG = 3; };
-template <> struct SliceCfg<6> { static constexpr int TN = 16, NG = 4; };
+// and TMEM columns per group: Re, Im of A B for four slices; for six, whose MMAs are
+// what bounds a tile (126 of them 6.6k of its 15.4k cycles), A_re (Re B, Im B) and
+// A_im (Re B, Im B) apart, two MMAs a complex product and the sums in the epilogue:
+// 304 ln det at d = 2, n = 2048 561 -> 512 ms, 512 dlogf at n = 300 23.0 -> 21.8
+template <> struct SliceCfg<4> { static constexpr int TN = 32, NG = 3, GC = 2 * 32; };
+template <> struct SliceCfg<6> { static constexpr int TN = 16, NG = 4, GC = 4 * 16; };
 template <int NS> __host__ __device__ constexpr int a_band() { return 2 * NS * A_SUB; }  // NS slices x {Re, Im}
 // A B tile's operand rows, per slice: Re, Im of its columns, so that A_re times
 // (Re, Im) is one MMA of N = 2 TN: three MMAs a complex product.  304 ln det at
@@ -277,7 +281,7 @@ static __device__ void slice_block_cols(const float4* Bp, int ld, int nn, int K,
 }
 
 // ---------------------------------------------------------------- tensor-core update
-// Accumulator group g (TMEM columns 2 TN g .. +TN for Re, +TN .. +2 TN for Im)
+// Accumulator group g (TMEM columns GC g ..: Re, Im, or the two pairs)
 // holds slice level l = g for g < NG - 1 and levels >= NG - 1 in the last
 // group, so that the low levels stay exact whatever the tensor core's FP32
 // summation order and rounding.
@@ -302,10 +306,14 @@ __device__ __forceinline__ void issue_tile_mmas(uint32_t a0, uint32_t b0, uint64
             for (int i = 0; i <= l; ++i) {
                 const int j = l - i;
                 const uint32_t acc = (ks == 0 && i == 0 && l == g) ? 0u : 1u;  // first product of group g
-                const uint32_t tre = tmem + 2 * TN * g, tim = tre + TN;
+                const uint32_t tre = tmem + SliceCfg<NS>::GC * g, tim = tre + TN;
                 umma_bf16_lead(tre, dA(i, 0, ks), dB(j, 0, ks), id2, acc, lead);
-                umma_bf16_lead(tre, dA(i, 1, ks), dB(j, TN, ks), idn, 1, lead);
-                umma_bf16_lead(tim, dA(i, 1, ks), dB(j, 0, ks), idp, 1, lead);
+                if (NS == 6) {
+                    umma_bf16_lead(tre + 2 * TN, dA(i, 1, ks), dB(j, 0, ks), id2, acc, lead);
+                } else {
+                    umma_bf16_lead(tre, dA(i, 1, ks), dB(j, TN, ks), idn, 1, lead);
+                    umma_bf16_lead(tim, dA(i, 1, ks), dB(j, 0, ks), idp, 1, lead);
+                }
             }
         }
     }
@@ -377,14 +385,41 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
         mbar_arrive_expect_tx(&s.bar_b, BB);
         bulk_g2s(sB, imgB + (size_t)bj * BB, BB, &s.bar_b);
     }
-    bool new_band = true, first = true;
+    // warp 0: have this tile's operands landed?
+    auto operands = [&](bool new_band, int limit) {
+        bool ok = pend;
+        if (pend) {
+            if (new_band) {
+                ok = mbar_wait(&s.bar_a, ph.a, limit);
+                if (!ok) mbar_wait(&s.bar_a, ph.a);  // let the copy in flight land before moving on
+                ph.a ^= 1;
+            }
+            ok = mbar_wait(&s.bar_b, ph.b) && ok;
+            ph.b ^= 1;
+        }
+        return __all_sync(0xffffffffu, ok) != 0;
+    };
+    // The wait for a tile's operands comes before the barrier that ends the tile before,
+    // so that its MMAs are issued at once: behind the barrier the wait queued up with the
+    // CTA's loads of C (2.4k of 19.5k cycles a tile at n = 1024, and 3k for the loads).
+    bool ready = warp == 0 && todo > 0 && operands(true, X.first_wait);
     const int q = warp & 3, hcol = warp >> 2;  // TMEM lane quadrant, column half of this warp
     const int rloc = 32 * q + lane;
     while (todo > 0) {
         int nbi2 = bi, nbj2 = bj + 1;
         if (nbj2 >= width(bi)) { nbj2 = 0; ++nbi2; }
-        // this thread's row and CW columns of C, and its row scale, fetched before
-        // the MMAs complete so the memory latency hides behind the tensor core
+        if (warp == 0) {
+            if (ready) {
+                tc_fence_after();
+                issue_tile_mmas<NS>(smem_u32(sA), smem_u32(sB), &s.bar_mma, tmem, elect_lane());
+            } else if (lane == 0) {
+                s.err = 1;                // operands missing: no MMA is issued;
+                mbar_arrive(&s.bar_mma);  // release this tile's MMA wait at once
+            }
+            __syncwarp();
+        }
+        // this thread's row and CW columns of C, and its row scale, on their way while the
+        // tensor core works
         const int row = bi * MT_M + rloc;
         const bool row_ok = row < m;
         const float ea_r = row_ok ? gea[row] : 0.0f;
@@ -394,27 +429,6 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
             const int col = bj * TN + CW * hcol + j;
             cpre[j] = (row_ok && col < nn) ? C[row + (size_t)col * ldc] : make_float4(0, 0, 0, 0);
         }
-        if (warp == 0) {
-            bool ok = pend;
-            if (pend) {
-                if (new_band) {
-                    ok = mbar_wait(&s.bar_a, ph.a, first ? X.first_wait : WAIT_LIMIT);
-                    if (!ok) mbar_wait(&s.bar_a, ph.a);  // let the copy in flight land before moving on
-                    ph.a ^= 1;
-                }
-                ok = mbar_wait(&s.bar_b, ph.b) && ok;
-                ph.b ^= 1;
-            }
-            if (__all_sync(0xffffffffu, ok)) {
-                tc_fence_after();
-                issue_tile_mmas<NS>(smem_u32(sA), smem_u32(sB), &s.bar_mma, tmem, elect_lane());
-            } else if (lane == 0) {
-                s.err = 1;                // operands missing: no MMA is issued;
-                mbar_arrive(&s.bar_mma);  // release this tile's MMA wait at once
-            }
-            __syncwarp();
-        }
-        first = false;
         const bool mw = mbar_wait(&s.bar_mma, ph.mma);
         if (!mw && lane == 0) {
             s.err = 1;
@@ -436,37 +450,60 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
         }
         tc_fence_after();
         // epilogue: TMEM lanes 32(w%4).. (rows), columns CW(w/4)..+CW-1
+        constexpr int EC = NS == 6 ? 2 : 4;  // columns at a time
 #pragma unroll
-        for (int cc = 0; cc < CW; cc += 4) {
-            float g[2 * NG][4];
+        for (int cc = 0; cc < CW; cc += EC) {
+            float lr[EC][NG], li[EC][NG];
             const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + CW * hcol + cc;
+            if constexpr (NS == 6) {
+                float g[4 * NG][2];
 #pragma unroll
-            for (int a = 0; a < 2 * NG; ++a) tmem_ld4(base + TN * a, g[a]);
-            tmem_wait_ld();
+                for (int a = 0; a < 4 * NG; ++a) tmem_ld2(base + TN * a, g[a][0], g[a][1]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < EC; ++j)
+#pragma unroll
+                    for (int gg = 0; gg < NG; ++gg) {
+                        // integers below 2^24 in the exact groups: exact sums
+                        lr[j][gg] = __fsub_rn(g[4 * gg][j], g[4 * gg + 3][j]);
+                        li[j][gg] = __fadd_rn(g[4 * gg + 1][j], g[4 * gg + 2][j]);
+                    }
+            } else {
+                float g[2 * NG][4];
+#pragma unroll
+                for (int a = 0; a < 2 * NG; ++a) tmem_ld4(base + TN * a, g[a]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < EC; ++j)
+#pragma unroll
+                    for (int gg = 0; gg < NG; ++gg) {
+                        lr[j][gg] = g[2 * gg][j];
+                        li[j][gg] = g[2 * gg + 1][j];
+                    }
+            }
             if (row_ok) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < EC; ++j) {
                     const int col = bj * TN + CW * hcol + cc + j;
                     if (col < nn) {
                         const float sc = ea_r * geb[col];  // 2^(ea+eb-16), exact
                         const float4 cv = cpre[cc + j];
                         dfc c = dfc{df{cv.x, cv.y}, df{cv.z, cv.w}};
-                        float lr[NG], li[NG];
 #pragma unroll
                         for (int gg = 0; gg < NG; ++gg) {
-                            lr[gg] = g[2 * gg][j] * sc;
-                            li[gg] = g[2 * gg + 1][j] * sc;
+                            lr[j][gg] *= sc;
+                            li[j][gg] *= sc;
                         }
-                        c.re = df_sub_levels<NG>(c.re, lr);
-                        c.im = df_sub_levels<NG>(c.im, li);
+                        c.re = df_sub_levels<NG>(c.re, lr[j]);
+                        c.im = df_sub_levels<NG>(c.im, li[j]);
                         dfc_store(C + row + (size_t)col * ldc, c);
                     }
                 }
             }
         }
+        if (warp == 0) ready = todo > 1 && operands(nbi2 != bi, WAIT_LIMIT);
         tc_fence_before();
         __syncthreads();
-        new_band = (nbi2 != bi);
         bi = nbi2;
         bj = nbj2;
         --todo;
