@@ -287,10 +287,12 @@ MSG_D zc hyp0f1(double a, zc z) {
     t = t / tgamma(a);
     zc s = t;
     for (int i = 1; i <= 50; i++) {
-        t = t * z / (i * a);
+        // one reciprocal and squared moduli: a step is on the one thread's chain that the
+        // hard-sphere diagonal waits for
+        t = (t * z) * (1.0 / (i * a));
         s += t;
         a += 1.0;
-        if (zabs(t) < 1e-16 * zabs(s)) break;
+        if (zabs2(t) < 1e-32 * zabs2(s)) break;
     }
     return s;
 }
