@@ -9,9 +9,11 @@ sample = 4096).  One step = the hot path over the whole cut.
   value  : evals/s with positions and k already resident in HBM (msgpu_job_run)
   e2e    : evals/s through the C-ABI call a user makes with host buffers
            (msgpu_tracelog_batch: H2D of inputs, the kernels, D2H of results)
-  roofline: the engine's binding unit (the FP64 pipe, peak = a DFMA probe run
-           here) with achieved = 8/3 N^3 flops per ln det / step time, and
-           the DRAM traffic of one ncu capture scaled to the launch
+  roofline: the tensor pipe, which carries the N^3 work: achieved = the bf16
+           flops of the digit products (28 of them for 8/3 N^3 real flops per ln
+           det) / step time, peak from MEASURED_PEAKS.json; beside it the
+           algorithmic rate and the FP64 pipe's (DFMA probe run here), and the
+           DRAM traffic of one ncu capture scaled to the launch
   cpu_baseline: the reference algorithm on all host cores, bounded sample
   clocks: nvidia-smi samples during the timed region
   gpu_launches: this library's kernel launches in the timed region
@@ -823,12 +825,14 @@ def main():
     peaks = read_peaks()
     if args.precision == "fp64":
         peak = ms.probe_fp64_tflops()
-        # the FP64 tensor path (warp-level m8n8k4 MMA) measured beside it: the engine
-        # runs on whichever is faster, DFMA on GB300
+        # the FP64 pipe (DFMA) and the FP64 tensor path (warp-level m8n8k4 MMA), measured here
         peak_mma = ms.probe_fp64_mma_tflops()
-        roof = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                "peak_source": "measured DFMA probe on this GPU (MEASURED_PEAKS.json has no FP64 entry)",
-                "fp64_mma_probe_tflops": peak_mma,
+        bf16 = peaks.get("bf16_tflops_sustained", 1728.6)
+        # trailing updates: 28 products of 9-bit digits for every FP64 one
+        roof = {"bound": "tensor", "achieved": 28 * achieved, "peak": bf16, "unit": "TFLOP/s", "frac": 28 * achieved / bf16,
+                "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained",
+                "executed": "28 bf16 digit products per real product of the complex LU (8/3 N^3 real flops)",
+                "algorithmic_tflops": achieved, "fp64_fma_probe_tflops": peak, "fp64_mma_probe_tflops": peak_mma,
                 "algorithmic": "8/3 N^3 real flops per ln det (complex LU), N=1024: 2.863e9",
                 "traffic": None}
     else:

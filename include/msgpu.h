@@ -157,9 +157,10 @@ int msgpu_amplitude_batch(int nmed, const msgpu_medium* media, int nitem, const 
  * the library (held by every GPU that loads it): n <= 2048, nk <= 65536, else
  * MSGPU_E_SIZE.  The array holds floor(~128 MiB / (16 n^2)) matrix slots, one
  * per engine CTA, capped at 2 per SM: 304 CTAs for n <= 165, 127 at n = 256,
- * 31 at n = 512, 7 at n = 1024 and 1 at n = 2048, against the 304 the
- * allocating entry points run, so large n runs at a fraction of their
- * throughput (1/43 at n = 1024).  Calls share that array, so calls that
+ * 31 at n = 512, 7 at n = 1024 and 1 at n = 2048, all on the FP64 pipe,
+ * against the hundreds of CTAs (and, above n = 104, the tensor cores) of the
+ * allocating entry points, so large n runs at a small fraction of their
+ * throughput.  Calls share that array, so calls that
  * overlap on the GPU race: keep them on one stream.  The first call on a
  * device looks up the array's address; make it before any stream capture.
  * Counted in msgpu_launch_count (two launches per call); errors set the text
@@ -289,7 +290,9 @@ int msgpu_eigvals_batch_mtype(int mtype, int nmed, const msgpu_medium* media, in
 
 /* Launch choices (autotuning).  Per (kind, requested precision, size bucket
  * of the job's largest n: (2^(b-1), 2^b]) the engine that runs and the
- * resident CTAs per SM of the persistent grid.  engine: MSGPU_FP64,
+ * resident CTAs per SM of the persistent grid (1: as asked; otherwise as many
+ * as the kernel for that size holds, and clusters of CTAs per matrix where the
+ * batch would leave SMs idle).  engine: MSGPU_FP64,
  * MSGPU_MIXED (only for a mixed request) or -1 = the requested one; ctas 0 =
  * as many as fit.  The FP64 engine may serve a mixed request: it meets the
  * mixed accuracy bound with room to spare. */
