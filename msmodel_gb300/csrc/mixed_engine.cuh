@@ -75,13 +75,13 @@ template <int NS> __host__ __device__ constexpr int a_band() { return 2 * NS * A
 template <int NS> __host__ __device__ constexpr int b_rows() { return 2 * SliceCfg<NS>::TN; }
 template <int NS> __host__ __device__ constexpr int b_sub() { return b_rows<NS>() * NB * 2; }
 template <int NS> __host__ __device__ constexpr int b_band() { return NS * b_sub<NS>(); }
+constexpr int EB_BYTES = 128;  // a tile's column scales, behind its slices in the image
 // shared-memory operand buffer: A band then B band (NS = 4: 64 + 16 KB; NS = 6: 96 + 12 KB)
 constexpr int GEMM_BYTES = a_band<6>() + b_band<6>() > a_band<4>() + b_band<4>() ? a_band<6>() + b_band<6>()
                                                                                    : a_band<4>() + b_band<4>();
 // global image bytes per 128 rows of A and per column of B, the larger of the two configurations
 constexpr int A_IMG_BAND = a_band<6>();
-constexpr int B_IMG_COL = b_band<6>() / SliceCfg<6>::TN > b_band<4>() / SliceCfg<4>::TN
-                              ? b_band<6>() / SliceCfg<6>::TN : b_band<4>() / SliceCfg<4>::TN;
+constexpr int B_IMG_COL = std::max((b_band<6>() + EB_BYTES) / SliceCfg<6>::TN, (b_band<4>() + EB_BYTES) / SliceCfg<4>::TN);
 
 // per-phase cycle accounting (thread 0, only when X.stats is set)
 enum { PH_ASSEMBLE = 0, PH_PANEL, PH_TRSM, PH_SLICE, PH_TILES, PH_SOLVE, PH_ITEMS, PH_N };
@@ -117,6 +117,7 @@ struct MixSmem {
     int red_i[NT / 32];
     int red_k[2][NT / 32], red_p[2][NT / 32];
     float4 rpiv;          // reciprocal of the panel's pivot
+    alignas(16) float eb[2][EB_BYTES / 4];  // column scales of this tile and the next
     int nz;
     int rng[2];           // the item's entry range, this CTA's part (float bits), and every CTA's of the team
     int team_rng[16][2];
@@ -151,8 +152,8 @@ __device__ __forceinline__ void stat_add(MixSmem& s, int ph) {
 struct MixScratch {
     uint8_t* imgA;   // ceil(nmax/128) * A_IMG_BAND per CTA
     uint8_t* imgB;   // (ceil(nmax/32) * 32) * B_IMG_COL per CTA
-    float* ea;       // row and column scales 2^(e-8) of the sliced operands, padded
-    float* eb;
+    float* ea;       // row scales 2^(e-8) of the sliced A operand, padded
+    float* eb;       // column scales (four slices; six keep them in the image)
     size_t a_stride, b_stride, e_stride;
     int* err;        // device flag: 1 = an mbarrier wait timed out
     unsigned long long* stats;  // per-phase SM cycles summed over CTAs, or nullptr
@@ -260,19 +261,20 @@ static __device__ void slice_panel_rows(const float4* P, int ld, int m, int K, u
 
 // B operand: columns [0, nn) of the K x nn block Bp (column-major, ld); eb[j] = 2^(e_j - 8)
 template <int NS, class Team>
-static __device__ void slice_block_cols(const float4* Bp, int ld, int nn, int K, uint8_t* img, float* eb, const Team& tm) {
+static __device__ void slice_block_cols(const float4* Bp, int ld, int nn, int K, uint8_t* img, float* geb, const Team& tm) {
     constexpr int TN = SliceCfg<NS>::TN;
     const int np = (nn + TN - 1) / TN * TN;
     for (int j = tm.rank * NT + threadIdx.x; j < np; j += NT * tm.size) {
-        uint8_t* band = img + (size_t)(j / TN) * b_band<NS>();
+        uint8_t* band = img + (size_t)(j / TN) * (b_band<NS>() + EB_BYTES);
         const int r = j % TN;
+        float* eb = NS == 6 ? reinterpret_cast<float*>(band + b_band<NS>()) + r : geb + j;
         auto put = [&](int sl, int c, int k, uint4 w) {
             *reinterpret_cast<uint4*>(band + sl * b_sub<NS>() + cm_offset(c * TN + r, k, b_rows<NS>())) = w;
         };
         if (j < nn) {
-            eb[j] = ldexpf(1.0f, slice_operand_row<NS>(Bp + (size_t)j * ld, 1, K, put) - 8);
+            *eb = ldexpf(1.0f, slice_operand_row<NS>(Bp + (size_t)j * ld, 1, K, put) - 8);
         } else {
-            eb[j] = 0.0f;
+            *eb = 0.0f;
             for (int k = 0; k < NB; k += 8)
                 for (int sl = 0; sl < NS; ++sl)
                     for (int c = 0; c < 2; ++c) put(sl, c, k, make_uint4(0, 0, 0, 0));
@@ -376,15 +378,25 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
         todo = (int)((long long)total * (tm.rank + 1) / tm.size) - bj;
         while (bi < nbi && bj >= width(bi)) bj -= width(bi++);
     }
+    // A tile's B operand, and with six slices its column scales (read in the epilogue, beside
+    // the next tile's copy, hence two of them): 304 ln det at d = 2, n = 2048 513 -> 486 ms
+    // against a global load each, which waits behind the stores to C.  With four slices the
+    // second copy cost 3% at n = 1024.
+    auto load_b = [&](int col, int p) {
+        const uint8_t* src = imgB + (size_t)col * (BB + EB_BYTES);
+        mbar_arrive_expect_tx(&s.bar_b, NS == 6 ? BB + EB_BYTES : BB);
+        bulk_g2s(sB, src, BB, &s.bar_b);
+        if (NS == 6) bulk_g2s(s.eb[p], src + BB, EB_BYTES, &s.bar_b);
+    };
     bool pend = todo > 0 && !s.err;  // warp 0: this tile's operand copies were issued
     pend = __shfl_sync(0xffffffffu, pend, 0);
     if (tid == 0 && pend) {
         mbar_arrive_expect_tx(&s.bar_a, AB);
         bulk_g2s(sA, imgA + (size_t)bi * AB, AB / 2, &s.bar_a);
         bulk_g2s(sA + AB / 2, imgA + (size_t)bi * AB + AB / 2, AB / 2, &s.bar_a);
-        mbar_arrive_expect_tx(&s.bar_b, BB);
-        bulk_g2s(sB, imgB + (size_t)bj * BB, BB, &s.bar_b);
+        load_b(bj, 0);
     }
+    int par = 0;  // which of s.eb the current tile's scales are in
     // warp 0: have this tile's operands landed?
     auto operands = [&](bool new_band, int limit) {
         bool ok = pend;
@@ -444,8 +456,7 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
                     bulk_g2s(sA, imgA + (size_t)nbi2 * AB, AB / 2, &s.bar_a);
                     bulk_g2s(sA + AB / 2, imgA + (size_t)nbi2 * AB + AB / 2, AB / 2, &s.bar_a);
                 }
-                mbar_arrive_expect_tx(&s.bar_b, BB);
-                bulk_g2s(sB, imgB + (size_t)nbj2 * BB, BB, &s.bar_b);
+                load_b(nbj2, par ^ 1);
             }
         }
         tc_fence_after();
@@ -486,7 +497,8 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
                 for (int j = 0; j < EC; ++j) {
                     const int col = bj * TN + CW * hcol + cc + j;
                     if (col < nn) {
-                        const float sc = ea_r * geb[col];  // 2^(ea+eb-16), exact
+                        // 2^(ea+eb-16), exact
+                        const float sc = ea_r * (NS == 6 ? s.eb[par][CW * hcol + cc + j] : geb[col]);
                         const float4 cv = cpre[cc + j];
                         dfc c = dfc{df{cv.x, cv.y}, df{cv.z, cv.w}};
 #pragma unroll
@@ -506,6 +518,7 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
         __syncthreads();
         bi = nbi2;
         bj = nbj2;
+        par ^= 1;
         --todo;
     }
     stat_add(s, PH_TILES);
