@@ -121,6 +121,8 @@ struct MixSmem {
     int nz;
     int rng[2];           // the item's entry range, this CTA's part (float bits), and every CTA's of the team
     int team_rng[16][2];
+    int team_bad[16];     // every CTA's flag of a wait that ran out (a word of its own: a CTA ahead of the
+                          // others writes it while they may still read the ranges)
     double team_max[16];
     double red_s[3][NT / 32];
     int info, bcast_i, item;
@@ -1515,9 +1517,9 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
         __syncthreads();
         int bad = s.err;
         if (tm.size > 1) {
-            if (tid < tm.size) cluster_store(&s.team_rng[tm.rank][0], tid, bad);
+            if (tid < tm.size) cluster_store(&s.team_bad[tm.rank], tid, bad);
             tm.sync();
-            for (int r = 0; r < tm.size; ++r) bad |= s.team_rng[r][0];
+            for (int r = 0; r < tm.size; ++r) bad |= s.team_bad[r];
         }
         if (bad) {
             alive = false;

@@ -71,6 +71,7 @@ struct Tc64Smem {
     int emax[TC_M];
     int rng[2];               // the item's entry range (EntryRange), this CTA's part
     int team_rng[16][2];      // ... and every CTA's of the team
+    int team_bad[16];         // every CTA's flag of a wait that ran out
     zc urow[NB];
     zc piv, rpiv;
     zc diag[2];
@@ -415,9 +416,9 @@ struct TcUpdate {
     __device__ __forceinline__ bool failed(Tc64Smem& s, const Team& tm) const {
         int bad = s.err;
         if (tm.size > 1) {
-            if (threadIdx.x < tm.size) cluster_store(&s.team_rng[tm.rank][0], threadIdx.x, bad);
+            if (threadIdx.x < tm.size) cluster_store(&s.team_bad[tm.rank], threadIdx.x, bad);
             tm.sync();
-            for (int r = 0; r < tm.size; ++r) bad |= s.team_rng[r][0];
+            for (int r = 0; r < tm.size; ++r) bad |= s.team_bad[r];
         }
         return bad != 0;
     }
