@@ -307,7 +307,11 @@ int msgpu_autotune(int kind, int precision, int d, int n, int nitem, double* sec
 /* Resident jobs: inputs uploaded once, the hot path run on device-resident
  * data (asynchronously on `stream`, a cudaStream_t or NULL), results fetched
  * separately.  kind: 0 = ln det / n, 1 = dlogf, 2 = amplitudes (as above),
- * 3 = traceinv, 4 = inverse iteration (FP64 engine). */
+ * 3 = traceinv, 4 = inverse iteration (FP64 engine).  The runs of all jobs
+ * and batched calls share one workspace: runs that may overlap on the GPU
+ * belong on one stream (or fetch a job's results before the next run on
+ * another); msgpu_tracelog_matrix has buffers of its own and may be called
+ * beside a run. */
 typedef struct msgpu_job msgpu_job;
 msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int nitem, const int* item_med,
                             const double* ks, int precision);

@@ -706,26 +706,19 @@ static int launch_locked(msgpu_job* J, void* ws, cudaStream_t st) {
     return 0;
 }
 
-// One matrix of the caller's through the FP64 engine: it goes straight into the
-// engine's slot and is shared by a cluster of CTAs (n = 300: one CTA took 14 ms).
-int msgpu_tracelog_matrix(int n, const double* mat, double* out, int* info) {
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (int e = init_locked(-1)) return e;
-    if (n < 1 || !mat || !out) return set_err(MSGPU_E_ARG, "bad argument");
+// One matrix of the caller's through the FP64 engine, shared by a cluster of CTAs
+// (n = 300: one CTA took 14 ms).  Its buffers are its own block of the pool, not the
+// shared workspace: a job may still be running there, on a stream this one does not wait for.
+static int tracelog_matrix_in(unsigned char* b, size_t img_off, size_t piv_off, size_t out_off, int n, const double* mat,
+                              double* out, int* info) {
     const bool tc = n >= TC_NMIN;
-    const size_t mat_b = sizeof(zc) * (size_t)n * n, img_off = (mat_b + 127) / 128 * 128;
-    const size_t piv_off = img_off + (tc ? (tc64_image_bytes(n) + 127) / 128 * 128 : 0);
-    const size_t out_off = piv_off + (sizeof(int) * (size_t)n + 127) / 128 * 128;
-    void* ws = nullptr;
-    if (int e = ensure_ws(out_off + 256, &ws)) return e;
-    unsigned char* b = static_cast<unsigned char*>(ws);
     // results and queue: {out[2], info, status}, then the counter words {0, 1}
     const unsigned queue[2] = {0u, 1u};
-    CK(cudaMemcpy(b, mat, mat_b, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(b, mat, sizeof(zc) * (size_t)n * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b + out_off + 128, queue, sizeof(queue), cudaMemcpyHostToDevice));
     EngineParams P{};
     P.nitem = 1;
-    P.ws = reinterpret_cast<zc*>(ws);
+    P.ws = reinterpret_cast<zc*>(b);
     P.slot = (size_t)n * n;
     P.piv = reinterpret_cast<int*>(b + piv_off);
     P.piv_stride = n;
@@ -748,6 +741,22 @@ int msgpu_tracelog_matrix(int n, const double* mat, double* out, int* info) {
     out[1] = h[1];
     if (info) *info = st[0];
     return 0;
+}
+
+int msgpu_tracelog_matrix(int n, const double* mat, double* out, int* info) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (int e = init_locked(-1)) return e;
+    if (n < 1 || !mat || !out) return set_err(MSGPU_E_ARG, "bad argument");
+    const size_t img_off = (sizeof(zc) * (size_t)n * n + 127) / 128 * 128;
+    const size_t piv_off = img_off + (n >= TC_NMIN ? (tc64_image_bytes(n) + 127) / 128 * 128 : 0);
+    const size_t out_off = piv_off + (sizeof(int) * (size_t)n + 127) / 128 * 128;
+    size_t bytes = out_off + 256;
+    void* b = pool_get(bytes);
+    if (!b) return set_err(MSGPU_E_CUDA, "tracelog_matrix: device allocation");
+    const int e = tracelog_matrix_in(static_cast<unsigned char*>(b), img_off, piv_off, out_off, n, mat, out, info);
+    if (e) cudaFree(b);  // (waits for what may still run on it)
+    else pool_put(b, bytes);
+    return e;
 }
 
 int msgpu_job_run(msgpu_job* J, void* stream) {

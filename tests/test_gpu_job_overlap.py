@@ -1,0 +1,26 @@
+"""Calls made while a resident job runs asynchronously on a stream of the caller's
+(a torch side stream, which does not synchronise with the default stream): the
+job's results and the calls' own must be those of each alone."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_tracelog_lu_beside_running_job(ms, precision):
+    torch = pytest.importorskip("torch")
+    med = ms.Medium(3, 1200, seed=3)
+    ks = 0.7 + 0.08 * np.arange(24) - 0.05j
+    want, wst = ms.tracelog_batch([med], ks, precision=precision)
+    mats = [ms.build_ms_matrix(ms.Medium(3, n, seed=n), 1.1 - 0.1j) for n in (40, 300)]
+    alone = [ms.tracelog_lu(m) for m in mats]
+    job = ms.Job("tracelog", [med], ks, precision=precision)
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        job.run(side.cuda_stream)
+        beside = [ms.tracelog_lu(m) for _ in range(4) for m in mats]
+        got, st = job.results()
+        assert beside == 4 * alone
+        assert np.array_equal(got, want) and np.array_equal(st, wst)
+    job.close()
