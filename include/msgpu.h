@@ -343,8 +343,9 @@ void msgpu_job_destroy(msgpu_job* job);
  * TRSM, slicing, tensor tiles, solves, items.  Returns the count written. */
 int msgpu_engine_stats(double* out, int n);
 /* Failure-path test hook, no counterpart in the reference: the poll limit of
- * the first operand wait (an mbarrier wait on a bulk copy) of every mixed
- * trailing update in later runs; polls < 0 restores the normal limit.  With 0
+ * the first operand wait (an mbarrier wait on a bulk copy) of every trailing
+ * update on the tensor cores (the mixed engine's and, above 96 rows, the FP64
+ * engine's) in later runs; polls < 0 restores the normal limit.  With 0
  * that wait runs out at once: the engine issues no MMA, lets the copy in
  * flight land, marks the item and every item not yet taken MSGPU_S_TIMEOUT
  * (value NaN), frees its tensor memory and returns; the device stays usable. */

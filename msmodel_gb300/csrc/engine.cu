@@ -692,6 +692,7 @@ static int launch_locked(msgpu_job* J, void* ws, cudaStream_t st) {
     P.warm = J->warm ? 1 : 0;
     P.given_n = 0;
     P.info = nullptr;
+    P.first_wait = first_wait_limit();
     P.amps = J->d_amps;
     P.amp_off = J->d_amp_off;
     if (J->precision == MSGPU_MIXED) {
@@ -727,6 +728,7 @@ static int tracelog_matrix_in(unsigned char* b, size_t img_off, size_t piv_off, 
     P.status = P.info + 1;
     P.counter = reinterpret_cast<unsigned*>(b + out_off + 128);
     P.given_n = n;
+    P.first_wait = first_wait_limit();
     const int team = pick_team_fp64(tc, 1, n);
     if (tc ? tc64_run(P, 1, team, n, b + img_off, nullptr)
            : launch_teams(k_engine_fp64, 1, team, NT, smem_bytes(), (cudaStream_t) nullptr, P))

@@ -34,6 +34,7 @@ struct EngineParams {
     int given_n;          // > 0: one item, the caller's matrix of given_n rows, already in the first slot
     int* info;            // given matrix: 1-based index of the first zero pivot, or 0
     int warm;             // kind 4: start each inverse iteration from the item's vector in amps
+    int first_wait;       // FP64 engine on the tensor cores: poll limit of an update's first operand wait
 };
 
 
@@ -101,7 +102,10 @@ int mixed_max_teams(int kind, bool d3only, int team);
 // Allocates the mixed engine's scratch for `grid` matrices up to nmax
 // (mixed_run does so itself; called before a stream capture, which must not allocate).
 int mixed_prepare(int grid, int nmax);
-// Changes whenever the mixed engine's scratch is reallocated (captured graphs hold its address).
+// poll limit of the first operand wait of every tensor-core update (msgpu_debug_first_wait_limit)
+int first_wait_limit();
+// Changes whenever the mixed engine's scratch is reallocated or that limit is set (captured
+// graphs hold both).
 unsigned long long mixed_generation();
 // per-phase SM cycles of the last mixed run made with MSGPU_STATS set:
 // assemble, panel, trsm, slice, tiles, solve, items

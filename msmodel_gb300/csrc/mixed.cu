@@ -63,6 +63,11 @@ static int prepare_locked(int grid, int nmax, MixScratch& X) {
     return 0;
 }
 
+int first_wait_limit() {
+    std::lock_guard<std::mutex> lk(g_mx);
+    return g_first_wait;
+}
+
 int mixed_prepare(int grid, int nmax) {
     std::lock_guard<std::mutex> lk(g_mx);
     MixScratch X;
@@ -162,8 +167,8 @@ __global__ void __launch_bounds__(128, 1) k_probe_umma(const float* A, const flo
 
 }  // namespace msg
 
-// Poll limit of the first operand wait of every mixed trailing update in later
-// runs (polls < 0: the normal limit).  A test sets 0 to make that wait run out
+// Poll limit of the first operand wait of every tensor-core trailing update, of
+// both engines, in later runs (polls < 0: the normal limit).  A test sets 0 to make that wait run out
 // and checks that the items report MSGPU_S_TIMEOUT and the context stays usable.
 extern "C" int msgpu_debug_first_wait_limit(int polls) {
     std::lock_guard<std::mutex> lk(msg::g_mx);

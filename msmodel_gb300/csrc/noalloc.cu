@@ -125,6 +125,7 @@ extern "C" int msgpu_tracelog_batch_noalloc(int d, int n, const double* d_pos, m
     P.warm = 0;
     P.given_n = 0;
     P.info = nullptr;
+    P.first_wait = 0;  // (no device waits on the FP64 pipe)
     k_engine_fp64<<<(unsigned)grid, NT, sizeof(LuSmem), st>>>(P);
     if (cudaGetLastError() != cudaSuccess) return record_error(MSGPU_E_CUDA, "noalloc: engine kernel launch failed");
     count_launches(2);

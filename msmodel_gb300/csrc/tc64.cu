@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(TC_NT, 1) k_engine_tc64(EngineParams P, uint8_
     __syncthreads();
     tc_fence_after();
     const ClusterTeam tm = this_team();
-    TcState t{img + (size_t)(blockIdx.x / tm.size) * img_stride, s.tmem, 0, 0, false};
+    TcState t{img + (size_t)(blockIdx.x / tm.size) * img_stride, s.tmem, 0, 0, P.first_wait, false};
     run_items_fp64(P, s, tm, TcUpdate{t});
     // an MMA completion wait that ran out may leave MMAs in flight: give them a bounded chance to land
     if (s.mma_stuck && tid == 0) mbar_wait(&s.bar_mma, (uint32_t)(s.mma_stuck - 1), 1 << 20);

@@ -158,6 +158,7 @@ struct TcState {
     uint8_t* img;      // the team's B image: ceil(nmax / 32) tiles of TC_BTILE
     uint32_t tmem;
     uint32_t ph_b, ph_mma;  // phases of bar_b (a bit each) and bar_mma
+    int first_wait;    // poll limit of an update's first operand wait
     bool use;          // the item's updates run on the tensor cores
 };
 
@@ -288,8 +289,10 @@ static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int 
     auto next = [&](int& i, int& j) {
         if (++j >= width(i)) { j = 0; ++i; }
     };
-    int buf = 0;
-    if (tid == 0 && todo > 0 && !s.err) load_b(0, bj);
+    int buf = 0, limit = t.first_wait;
+    // warp 0: this tile's B copy is under way (none is issued once a wait has run out)
+    bool pend = __shfl_sync(0xffffffffu, todo > 0 && !s.err, 0);
+    if (tid == 0 && pend) load_b(0, bj);
     int band = -1;
     const int q = warp & 3, cg = warp >> 2;  // TMEM lane quadrant, group of 8 columns
     const int rloc = 32 * q + lane;
@@ -303,15 +306,22 @@ static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int 
             band = bi;
         }
         if (warp == 0) {
-            const bool ok = !s.err && mbar_wait(&s.bar_b[buf], (ph_b >> buf) & 1);
-            ph_b ^= 1u << buf;
-            if (__all_sync(0xffffffffu, ok)) {
+            bool ok = pend;
+            if (pend) {
+                ok = mbar_wait(&s.bar_b[buf], (ph_b >> buf) & 1, limit);
+                if (!ok) mbar_wait(&s.bar_b[buf], (ph_b >> buf) & 1);  // let the copy in flight land before moving on
+                ph_b ^= 1u << buf;
+                limit = WAIT_LIMIT;
+            }
+            pend = false;
+            if (__all_sync(0xffffffffu, ok && !s.err)) {
                 tc_fence_after();
                 tc_issue_tile(smem_u32(s.g.a), smem_u32(s.g.b[buf]), &s.bar_mma, tmem, elect_lane());
-                if (lane == 0 && todo > 1) load_b(buf ^ 1, bj2);
+                pend = todo > 1;
+                if (lane == 0 && pend) load_b(buf ^ 1, bj2);
             } else if (lane == 0) {
-                s.err = 1;
-                mbar_arrive(&s.bar_mma);
+                s.err = 1;                // operands missing: no MMA is issued;
+                mbar_arrive(&s.bar_mma);  // release this tile's MMA wait at once
             }
             __syncwarp();
         }
@@ -368,10 +378,6 @@ static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int 
         --todo;
     }
     t.ph_b = ph_b;
-    // a failed wait may leave a B copy in flight: let it land before the buffer changes hands
-    if (s.err && tid == 0)
-        for (int b = 0; b < 2; ++b) mbar_wait(&s.bar_b[b], (ph_b >> b) & 1, 1 << 16);
-    __syncthreads();
 }
 
 // the FP64 pipe's update, kept out of line beside it
