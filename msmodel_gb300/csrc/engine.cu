@@ -276,7 +276,6 @@ struct msgpu_job {
     // the job's device arrays, all in one block
     void* block = nullptr;
     size_t block_bytes = 0;
-    bool ran = false;        // a run may still be on the device
     MedDev* d_media = nullptr;
     double* d_pos = nullptr;
     size_t items_b = 0;      // bytes from d_ks to the live count: the item arrays at full capacity
@@ -508,10 +507,10 @@ static int set_items_locked(msgpu_job* J, int nitem, const int* item_med, const 
     return 0;
 }
 
+// (the job's runs have completed: its block may be another job's next)
 static void destroy_locked(msgpu_job* J) {
     if (J->gexec) cudaGraphExecDestroy(J->gexec);
     if (J->cap_stream) cudaStreamDestroy(J->cap_stream);
-    if (J->ran) cudaDeviceSynchronize();  // the block may be another job's next
     pool_put(J->block, J->block_bytes);
     delete J;
 }
@@ -767,7 +766,6 @@ int msgpu_job_run(msgpu_job* J, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     void* ws = nullptr;
     if (int e = ensure_ws(J->ws_bytes, &ws)) return e;
-    J->ran = true;
     if (!J->use_graph) {
         if (int e = launch_locked(J, ws, st)) return e;
         g_launches++;
@@ -810,7 +808,6 @@ double msgpu_job_flops(const msgpu_job* J) { return J ? J->flops : 0.0; }
 int msgpu_job_results(msgpu_job* J, double* out, int* status) {
     if (!J) return set_err(MSGPU_E_ARG, "null job");
     CK(cudaDeviceSynchronize());
-    J->ran = false;
     if (out) CK(cudaMemcpy(out, J->d_out, sizeof(double) * 2 * J->nitem, cudaMemcpyDeviceToHost));
     if (status) CK(cudaMemcpy(status, J->d_status, sizeof(int) * J->nitem, cudaMemcpyDeviceToHost));
     return 0;
@@ -835,6 +832,10 @@ int msgpu_job_set_vectors(msgpu_job* J, const double* vecs) {
 
 void msgpu_job_destroy(msgpu_job* J) {
     if (!J) return;
+    // A run may be on the device that this library does not know of (a graph of the caller's
+    // that captured msgpu_job_run), so every destroy waits, as cudaFree of the arrays would
+    // have; outside the lock, so that other threads' calls go on meanwhile.
+    cudaDeviceSynchronize();
     std::lock_guard<std::mutex> lk(g_mu);
     destroy_locked(J);
 }

@@ -24,3 +24,31 @@ def test_tracelog_lu_beside_running_job(ms, precision):
         assert beside == 4 * alone
         assert np.array_equal(got, want) and np.array_equal(st, wst)
     job.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_destroy_waits_for_a_callers_graph(ms, precision):
+    """A run captured in a CUDA graph of the caller's and replayed after the job's
+    results were fetched: destroying the job must wait for the replay, whose arrays
+    the next job of that size is given."""
+    torch = pytest.importorskip("torch")
+    med = ms.Medium(3, 700, seed=4)
+    ks = 0.7 + 0.02 * np.arange(100) - 0.05j
+    want, _ = ms.tracelog_batch([med], ks + 0.3, precision=precision)
+    for _ in range(3):
+        job = ms.Job("tracelog", [med], ks, precision=precision)
+        job.run()
+        first, _ = job.results()
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=side):
+            job.run(torch.cuda.current_stream().cuda_stream)
+        graph.replay()
+        again, _ = job.results()
+        assert np.array_equal(first, again)
+        graph.replay()
+        job.close()
+        nxt = ms.Job("tracelog", [med], ks + 0.3, precision=precision)
+        nxt.run()
+        got, st = nxt.results()
+        nxt.close()
+        assert np.all(st == 0) and np.array_equal(got, want)
