@@ -143,7 +143,8 @@ int msgpu_dk_log_det_batch(int nmed, const msgpu_medium* media, int nitem, const
  * and the optical-theorem cross section -Im(conj(phi).a)/k in out[2i]
  * (total_cross_section, src/core/ms_matrix_util.c:344; out[2i+1] is its
  * imaginary part for complex k).  amps (may be NULL) receives a for every
- * item, n_i complex values each, concatenated in item order. */
+ * item, n_i complex values each, concatenated in item order; NaN for an item
+ * without a result (MSGPU_S_RANGE, MSGPU_S_TIMEOUT). */
 int msgpu_amplitude_batch(int nmed, const msgpu_medium* media, int nitem, const int* item_med, const double* ks,
                           double* out, double* amps, int* status, int precision);
 

@@ -38,6 +38,17 @@ struct EngineParams {
 };
 
 
+#ifdef __CUDACC__
+// An amplitude item without a result: NaN for its amplitudes, entries first, first + step, ...
+// (the job's array is a pooled block and may hold another job's).
+__device__ inline void void_amplitudes(const EngineParams& P, int it, int first, int step) {
+    if (P.kind != 2 || !P.amps) return;
+    double* a = P.amps + 2 * P.amp_off[it];
+    const int n2 = 2 * P.media[P.item_med[it]].n;
+    for (int i = first; i < n2; i += step) a[i] = nan("");
+}
+#endif
+
 // adds to the library's count of kernel launches (msgpu_launch_count)
 void count_launches(int n);
 

@@ -157,7 +157,10 @@ static __device__ void run_items_fp64(const EngineParams& P, S& s, const Cluster
             res = mk(-di, 0.0) / k;
         }
         const bool bad = up.failed(s, tm);
-        if (bad) res = mk(nan(""), nan(""));
+        if (bad) {
+            res = mk(nan(""), nan(""));
+            if (tm.rank == 0 && P.given_n <= 0) void_amplitudes(P, it, tid, S::NTH);
+        }
         if (tm.rank == 0 && tid == 0) {
             P.out[2 * it] = res.re;
             P.out[2 * it + 1] = res.im;
@@ -173,6 +176,7 @@ static __device__ void run_items_fp64(const EngineParams& P, S& s, const Cluster
                      u = atomicAdd(P.counter, 1u)) {
                     P.out[2 * P.order[u]] = P.out[2 * P.order[u] + 1] = nan("");
                     P.status[P.order[u]] = MSGPU_S_TIMEOUT;
+                    void_amplitudes(P, P.order[u], 0, 1);
                 }
         }
         tm.sync();

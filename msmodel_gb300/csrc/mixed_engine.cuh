@@ -1526,6 +1526,7 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
             st |= MSGPU_S_TIMEOUT;
             res = mk(nan(""), nan(""));
         }
+        if (KIND == 2 && tm.rank == 0 && (st & (MSGPU_S_TIMEOUT | MSGPU_S_RANGE))) void_amplitudes(P, it, tid, NT);
         if (tm.rank == 0 && tid == 0) {
             s.stat[PH_ITEMS] += 1;
             if (span_wide && !wide) st |= MSGPU_S_SPAN;
@@ -1545,6 +1546,7 @@ __global__ void __launch_bounds__(NT, 2) k_engine_mixed(EngineParams P, MixScrat
             const int it = P.order[q];
             P.out[2 * it] = P.out[2 * it + 1] = nan("");
             P.status[it] = MSGPU_S_TIMEOUT;
+            void_amplitudes(P, it, 0, 1);
         }
     }
     if (X.stats && tid == 0)
