@@ -96,10 +96,11 @@ int max_teams(K kern, int team, int threads, size_t smem) {
 int tc64_run(const EngineParams& P, int teams, int team, int nmax, void* img, cudaStream_t st);
 size_t tc64_image_bytes(int nmax);
 int tc64_max_teams(int team);
-// Rows from which an item's trailing updates run on the tensor cores.  Smaller items stay on the FP64 pipe: 912 ln det take 4.6 ms there against
-// 5.5 ms at n = 96, 8.6 against 7.0 at n = 112 (dlogf 11.4 against 9.9 and 20.0
-// against 12.7).  The rule looks at the item alone, so that no result depends
-// on the batch it is in.
+// Rows from which an item's trailing updates run on the tensor cores.  Smaller items
+// stay on the FP64 pipe: 912 ln det take 3.4 ms there against 3.9 at n = 96, 4.5
+// against 4.5 at n = 97, 6.4 against 6.2 at n = 128; dlogf 8.4 against 8.7, 12.1 against
+// 10.3 and 16.5 against 13.4.  The rule looks at the item alone, so that no result
+// depends on the batch it is in.
 constexpr int TC_NMIN = 97;
 
 // Mixed-precision engine (mixed.cu).  Returns 0 when it ran the job, a

@@ -14,8 +14,7 @@ __global__ void __launch_bounds__(TC_NT, 1) k_engine_tc64(EngineParams P, uint8_
         tmem_relinquish();
     }
     if (tid == 0) {
-        mbar_init(&s.bar_b[0], 1);
-        mbar_init(&s.bar_b[1], 1);
+        mbar_init(&s.bar_b, 1);
         mbar_init(&s.bar_mma, 1);
         s.err = 0;
         s.mma_stuck = 0;
