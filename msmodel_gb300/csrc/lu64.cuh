@@ -113,6 +113,7 @@ struct __align__(16) LuSmemT {
     static constexpr size_t PANEL_BYTES = sizeof(zc) * NB * (TMR + TNC);
     zc T[NB][NB + 1];    // 16.5 KB diagonal block / assembly transpose
     zc urow[NB];         // pivot row of the panel
+    zc dlo[NB];          // what the reciprocals of U's diagonal in T leave out (DiagQuot)
     zc piv, rpiv;        // the pivot and its reciprocal
     zc diag[2];          // F^-1(k), d F^-1/dk
     long long red_k[2][NTHREADS / 32];
@@ -374,8 +375,38 @@ __device__ __forceinline__ void col_solve_lower_unit(zc* __restrict__ b, int jb,
     }
 }
 
-// the upper solve; T's diagonal holds the reciprocals of U_rr
-__device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, const zc (*T)[NB + 1]) {
+// Division by a diagonal element U_rr, prepared once for the block's columns: hi the
+// rounded reciprocal, lo = hi (1 - U_rr hi), so that a hi + a lo loses nothing to the
+// reciprocal's rounding (|error| <= 2 2^-53 of the quotient; Smith's quotient reaches 2.2,
+// a product with the rounded reciprocal alone 2.7).  Far from 1 in the exponent range,
+// where a reciprocal may overflow, hi is U_rr itself, lo marked by an infinity, and the
+// solve divides.
+struct DiagQuot {
+    zc hi, lo;
+    static __device__ __forceinline__ DiagQuot prepare(zc u) {
+        const int e = max(__double2hiint(u.re) & 0x7fffffff, __double2hiint(u.im) & 0x7fffffff) >> 20;
+        if (e < 1023 - 500 || e > 1023 + 500) return {u, mk(__longlong_as_double(0x7ff0000000000000LL))};
+        const zc h = pivot_recip(u);
+        // 1 - u h, every difference exact: the two products of the real part add up to 1
+        // within rounding, those of the imaginary part to 0
+        const double p = __dmul_rn(u.re, h.re), q = -__dmul_rn(u.im, h.im);
+        const double pe = fma(u.re, h.re, -p), qe = fma(-u.im, h.im, -q);
+        const double r = __dmul_rn(u.re, h.im), t = __dmul_rn(u.im, h.re);
+        const double re = fma(u.re, h.im, -r), te = fma(u.im, h.re, -t);
+        const zc d = mk(((1.0 - fmax(p, q)) - fmin(p, q)) - (pe + qe), -((r + t) + (re + te)));
+        return {h, zmulf(h, d)};
+    }
+    // a / U_rr; far: some element of the block is one to divide by (load_upper)
+    static __device__ __forceinline__ zc of(zc a, zc hi, zc lo, bool far) {
+        if (far && __double2hiint(lo.re) == 0x7ff00000) return a / hi;
+        const zc t = zmulf(a, lo);
+        return mk(fma(a.re, hi.re, fma(-a.im, hi.im, t.re)), fma(a.re, hi.im, fma(a.im, hi.re, t.im)));
+    }
+};
+
+// the upper solve; T's diagonal and dlo hold the prepared divisions by U_rr
+__device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, const zc (*T)[NB + 1], const zc* dlo,
+                                                bool far) {
     for (int rb = ((jb - 1) / CH) * CH; rb >= 0; rb -= CH) {
         zc y[CH];
 #pragma unroll
@@ -392,7 +423,7 @@ __device__ __forceinline__ void col_solve_upper(zc* __restrict__ b, int jb, cons
 #pragma unroll
                 for (int q = CH - 1; q > r; --q)
                     if (rb + q < jb) acc = zfms(acc, T[rb + r][rb + q], y[q]);
-                y[r] = zmulf(acc, T[rb + r][rb + r]);
+                y[r] = DiagQuot::of(acc, T[rb + r][rb + r], dlo[rb + r], far);
             }
         }
 #pragma unroll
@@ -414,12 +445,26 @@ __device__ __forceinline__ zc row_solve_lower_unit(zc x, int jb, const zc (*T)[N
     }
     return x;
 }
-__device__ __forceinline__ zc row_solve_upper(zc x, int jb, const zc (*T)[NB + 1]) {
+// (The division of row q is one lane's, but its instructions take the pipe for the whole
+// warp: the halves of the warp do its real and its imaginary part, 4 instructions in
+// place of 8: 32 dlogf at n = 100 1.26 -> 1.19 ms.)
+__device__ __forceinline__ zc row_solve_upper(zc x, int jb, const zc (*T)[NB + 1], const zc* dlo, bool far) {
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, part = lane >> 4;
     for (int q = jb - 1; q >= 0; --q) {
-        if (lane == q) x = zmulf(x, T[q][q]);
-        const zc xq = mk(__shfl_sync(FULL, x.re, q), __shfl_sync(FULL, x.im, q));
+        const double ar = __shfl_sync(FULL, x.re, q), ai = __shfl_sync(FULL, x.im, q);
+        zc xq;
+        if (far && __double2hiint(dlo[q].re) == 0x7ff00000) {
+            xq = mk(ar, ai) / T[q][q];
+        } else {
+            // DiagQuot::of, component `part`
+            const double* h = &T[q][q].re;
+            const double* l = &dlo[q].re;
+            const double b = part ? ai : -ai;
+            const double v = fma(ar, h[part], fma(b, h[1 - part], fma(ar, l[part], __dmul_rn(b, l[1 - part]))));
+            xq = mk(__shfl_sync(FULL, v, 0), __shfl_sync(FULL, v, 16));
+        }
+        if (lane == q) x = xq;
         if (lane < q) x = zfms(x, T[lane][q], xq);
     }
     return x;
@@ -485,19 +530,23 @@ static __device__ void load_lower(const zc* A, int n, int j0, int jb, S& s) {
     __syncthreads();
 }
 
-// the upper triangle, its diagonal as reciprocals
+// the upper triangle, its diagonal as prepared divisions; true if one of them divides
 template <class S>
-static __device__ void load_upper(const zc* A, int n, int j0, int jb, S& s) {
+static __device__ bool load_upper(const zc* A, int n, int j0, int jb, S& s) {
+    bool far = false;
     for (int e = threadIdx.x; e < NB * NB; e += S::NTH) {
         int r = e % NB, q = e / NB;
-        zc v = mk(r == q ? 1.0 : 0.0);
-        if (r < jb && q < jb && q >= r) {
-            v = A[(j0 + r) + (size_t)(j0 + q) * n];
-            if (q == r) v = 1.0 / v;
+        zc v = mk(0.0);
+        if (r < jb && q < jb && q >= r) v = A[(j0 + r) + (size_t)(j0 + q) * n];
+        if (q == r && r < jb) {
+            const DiagQuot d = DiagQuot::prepare(v);
+            v = d.hi;
+            s.dlo[r] = d.lo;
+            far |= __double2hiint(d.lo.re) == 0x7ff00000;
         }
         s.T[r][q] = v;
     }
-    __syncthreads();
+    return __syncthreads_or(far) != 0;
 }
 
 // Apply the panel's interchanges to every other column and compute
@@ -744,19 +793,19 @@ static __device__ zc lu_trace_solve(const zc* A, zc* B, int n, const int* ipiv,
     const int nblk = (n + NB - 1) / NB;
     for (int kb = nblk - 1; kb >= 0; --kb) {
         const int j0 = kb * NB, jb = min(NB, n - j0), ncol = j0 + jb;
-        load_upper(A, n, j0, jb, s);
+        const bool far = load_upper(A, n, j0, jb, s);
         const int cols = cta_columns(ncol, tm);
         const int wide = thread_columns(cols, NTH);
         for (int x = wide + warp; x < cols; x += NW) {
             const int col = cta_column(x, tm);
             if (col >= ncol) continue;
             zc* b = B + (size_t)col * n + j0;
-            const zc v = row_solve_upper(lane < jb ? b[lane] : mk(0.0), jb, s.T);
+            const zc v = row_solve_upper(lane < jb ? b[lane] : mk(0.0), jb, s.T, s.dlo, far);
             if (lane < jb) b[lane] = v;
         }
         for (int x = tid; x < wide; x += NTH) {
             const int col = cta_column(x, tm);
-            if (col < ncol) col_solve_upper(B + (size_t)col * n + j0, jb, s.T);
+            if (col < ncol) col_solve_upper(B + (size_t)col * n + j0, jb, s.T, s.dlo, far);
         }
         tm.sync();
         // Y[0:j0, 0:ncol] -= U[0:j0, j0:j0+jb] X[j0:j0+jb, 0:ncol]   (rows >= cols only)
@@ -775,8 +824,8 @@ static __device__ zc lu_trace_solve(const zc* A, zc* B, int n, const int* ipiv,
 
 // x <- A^-1 x for one right-hand side x[n] (global), LAPACK-layout LU: the
 // interchanges, then blocked forward and backward substitution; each block's
-// triangle comes into shared memory, with the reciprocals of U's diagonal (a
-// division a step by one lane held up the chain), and is solved by warp 0 (one row
+// triangle comes into shared memory, with the divisions by U's diagonal prepared (a
+// whole division a step by one lane held up the chain), and is solved by warp 0 (one row
 // per lane), the rectangular remainder by all threads (one row per thread,
 // coalesced column reads).
 template <class S>
@@ -817,9 +866,9 @@ static __device__ void lu_solve_vec(const zc* A, zc* x, int n, const int* ipiv, 
     }
     for (int j0 = (n - 1) / NB * NB; j0 >= 0; j0 -= NB) {
         const int jb = min(NB, n - j0);
-        load_upper(A, n, j0, jb, s);
+        const bool far = load_upper(A, n, j0, jb, s);
         if (tid < 32) {
-            const zc v = row_solve_upper(lane < jb ? x[j0 + lane] : mk(0.0), jb, s.T);
+            const zc v = row_solve_upper(lane < jb ? x[j0 + lane] : mk(0.0), jb, s.T, s.dlo, far);
             if (lane < jb) x[j0 + lane] = s.urow[lane] = v;
         }
         __syncthreads();
