@@ -64,6 +64,14 @@ __device__ __forceinline__ double dlapy3(double x, double y, double z) {
     return w * sqrt(a * a + b * b + c * c);
 }
 
+// 2^-e of a modulus m = f 2^e; 1 where there is nothing to scale by (0, infinite, NaN)
+__device__ __forceinline__ double unit_scale(double m) {
+    if (!(m > 0.0) || !(m < INFINITY)) return 1.0;
+    return scalbn(1.0, max(-1000, min(1000, -ilogb(m))));
+}
+// do squares that add up to s lose nothing to the exponent range?
+__device__ __forceinline__ bool squares_safe(double s) { return s > 1e-280 && s < 1e280; }
+
 // Householder reduction to upper Hessenberg form (zgehd2, ilo = 1, ihi = n)
 static __device__ void hessenberg(zc* __restrict__ A, int n, LuSmem& s) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -74,12 +82,28 @@ static __device__ void hessenberg(zc* __restrict__ A, int n, LuSmem& s) {
         double ss = 0.0, z1 = 0.0, z2 = 0.0;
         for (int i = 1 + tid; i < m; i += NT) ss += zabs2(col[i]);
         block_sum3(ss, z1, z2, s);
+        double xnorm = sqrt(ss);
+        if (!squares_safe(ss)) {
+            // squares out of range, or zeros: the norm of the column scaled by its largest entry
+            double mx = 0.0;
+            int im = m, at;
+            for (int i = 1 + tid; i < m; i += NT) {
+                const double v = fmax(fabs(col[i].re), fabs(col[i].im));
+                if (v > mx) { mx = v; im = i; }
+            }
+            block_argmax(mx, im, s, at);
+            const double sc = at < m ? unit_scale(fmax(fabs(col[at].re), fabs(col[at].im))) : 1.0;
+            ss = 0.0;
+            for (int i = 1 + tid; i < m; i += NT) ss += zabs2(sc * col[i]);
+            block_sum3(ss, z1, z2, s);
+            xnorm = sqrt(ss) / sc;
+        }
         const zc alpha = col[0];
         __syncthreads();  // every thread has read alpha before column j changes
-        if (ss == 0.0 && alpha.im == 0.0) continue;  // H = I (tau = 0)
+        if (xnorm == 0.0 && alpha.im == 0.0) continue;  // H = I (tau = 0)
         // zlarfg: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta,
         // v = (1, x / (alpha - beta))
-        const double beta = -copysign(dlapy3(alpha.re, alpha.im, sqrt(ss)), alpha.re);
+        const double beta = -copysign(dlapy3(alpha.re, alpha.im, xnorm), alpha.re);
         const zc tau = mk((beta - alpha.re) / beta, -alpha.im / beta);
         const zc scal = 1.0 / (alpha - beta);
         for (int i = tid; i < m; i += NT) {
@@ -120,14 +144,21 @@ static __device__ void hessenberg(zc* __restrict__ A, int n, LuSmem& s) {
 // warp that chases the bulge is bound by how many FP64 instructions it issues, 64
 // clocks each: one reciprocal square root gives beta and 1 / beta, one division the
 // rest, 32 of them in all where a square root, two divisions and complex products
-// took 47 (zlarfg's dlapy3 scaling guards against overflow of |a|^2 + x^2, far
-// beyond M(k)'s entries).
+// took 47.  Where |a|^2 + x^2 leaves the exponent range (entries below 1e-140 or above
+// 1e140) both are scaled to 1 first, as zlarfg does; only beta depends on the scale.
 __device__ __forceinline__ void larfg2(zc& a, double x, zc& t1, zc& v2, double& t2) {
-    const double b2 = fma(x, x, fma(a.re, a.re, a.im * a.im));
+    double b2 = fma(x, x, fma(a.re, a.re, a.im * a.im)), back = 1.0;
     if (x == 0.0 && a.im == 0.0) {
         t1 = v2 = mk(0.0);
         t2 = 0.0;
         return;
+    }
+    if (!squares_safe(b2)) {
+        const double sc = unit_scale(fmax(fabs(x), fmax(fabs(a.re), fabs(a.im))));
+        a = sc * a;
+        x *= sc;
+        b2 = fma(x, x, fma(a.re, a.re, a.im * a.im));
+        back = 1.0 / sc;  // a power of two
     }
     const double rs = rsqrt(b2);
     double beta = b2 * rs;
@@ -138,7 +169,7 @@ __device__ __forceinline__ void larfg2(zc& a, double x, zc& t1, zc& v2, double& 
     t2 = -x * rb;
     const double y = x / fma(d.re, d.re, d.im * d.im);
     v2 = mk(d.re * y, -d.im * y);
-    a = mk(beta);
+    a = mk(beta * back);
 }
 
 // reflectors a bulge-chase window makes, and its rows and columns
