@@ -291,18 +291,20 @@ int msgpu_eigvals_batch_mtype(int mtype, int nmed, const msgpu_medium* media, in
 
 /* Launch choices (autotuning).  Per (kind, requested precision, size bucket
  * of the job's largest n: (2^(b-1), 2^b]) the engine that runs and the
- * resident CTAs per SM of the persistent grid (1: as asked; otherwise as many
- * as the kernel for that size holds, and clusters of CTAs per matrix where the
- * batch would leave SMs idle).  engine: MSGPU_FP64,
- * MSGPU_MIXED (only for a mixed request) or -1 = the requested one; ctas 0 =
- * as many as fit.  The FP64 engine may serve a mixed request: it meets the
+ * resident CTAs per SM of the persistent grid where a matrix has a CTA to
+ * itself (1: as asked; otherwise as many as the kernel for that size holds).
+ * Batches that would leave SMs idle take clusters of CTAs per matrix whatever
+ * the table says, and the FP64 engine runs one CTA per SM above 96 rows.
+ * engine: MSGPU_FP64, MSGPU_MIXED (only for a mixed request) or -1 = the
+ * requested one; ctas 0 = as many as fit.  The FP64 engine may serve a mixed request: it meets the
  * mixed accuracy bound with room to spare. */
 int msgpu_tune_set(int kind, int precision, int n, int engine, int ctas_per_sm);
 int msgpu_tune_get(int kind, int precision, int n, int* engine, int* ctas_per_sm);
 /* Time every candidate (engine x 1 or 2 CTAs per SM) on a probe batch of
  * nitem k for n scatterers of d dimensions (the reference ball, seed 1) and
- * keep the fastest for that size bucket.  seconds[4] receives the times
- * (fp64 x1, fp64 x2, mixed x1, mixed x2; -1 where not run). */
+ * keep the fastest for that size bucket (ctas 0 where that is the FP64 engine
+ * above 96 rows).  seconds[4] receives the times (fp64 x1, fp64 x2, mixed x1,
+ * mixed x2; -1 where not run, as fp64 x2 above 96 rows). */
 int msgpu_autotune(int kind, int precision, int d, int n, int nitem, double* seconds);
 
 /* Resident jobs: inputs uploaded once, the hot path run on device-resident

@@ -589,12 +589,14 @@ msgpu_job* msgpu_job_create(int kind, int nmed, const msgpu_medium* media, int n
         // (one CTA per SM asked for by the tuning table: as asked)
         J->small = J->nmax < TC_NMIN && J->team == 1 && te.ctas != 1 && nitem > held;
         if (J->small) held = g_sms * SMALL_CTAS;
-    } else if (nitem < held && te.ctas != 1) {
-        // a mixed job may turn wide with later points: count the teams of the wide launch
-        int teams[5] = {held, 0, 0, 0, 0};
+    } else if (nitem < g_sms * g_ctas_fp64) {
+        // (whatever the tuning table asks for a full chip: one wavefunction at n = 1024 takes
+        // 31 ms on a cluster, 74 on a CTA)  A mixed job may turn wide with later points: count
+        // the teams of the wide launch
+        int teams[5] = {g_sms * g_ctas_fp64, 0, 0, 0, 0};
         for (int j = 1; j < 5; ++j) teams[j] = mixed_max_teams(kind, J->d3only, 1 << j);
         J->team = pick_team(teams, 0.25, 1.6, nitem, J->nmax);
-        held = teams[ilog2(J->team)];
+        if (J->team > 1) held = teams[ilog2(J->team)];
     }
     int grid = std::min(nitem, held);
     if ((size_t)grid * per_cta + 128 > g_ws_bytes) {  // else the workspace that is there holds them
@@ -890,6 +892,9 @@ int msgpu_autotune(int kind, int precision, int d, int n, int nitem, double* sec
             double& t = seconds[ei * 2 + (c - 1)];
             t = -1.0;
             if (c > g_ctas_fp64) continue;
+            // above 96 rows the FP64 engine runs one CTA per SM whatever is asked: timed once
+            const bool tc = eng == MSGPU_FP64 && n >= TC_NMIN;
+            if (tc && c > 1) continue;
             if (int e = msgpu_tune_set(kind, precision, n, eng, c)) return e;
             msgpu_job* J = msgpu_job_create(kind, 1, &med, nitem, nullptr, ks.data(), precision);
             if (!J) return MSGPU_E_CUDA;
@@ -913,7 +918,7 @@ int msgpu_autotune(int kind, int precision, int d, int n, int nitem, double* sec
             if (best == 0.0 || t < best) {
                 best = t;
                 best_e = eng;
-                best_c = c;
+                best_c = tc ? 0 : c;
             }
         }
     return msgpu_tune_set(kind, precision, n, best_e, best_c);
