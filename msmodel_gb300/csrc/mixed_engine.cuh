@@ -417,6 +417,9 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
     // so that its MMAs are issued at once: behind the barrier the wait queued up with the
     // CTA's loads of C (2.4k of 19.5k cycles a tile at n = 1024, and 3k for the loads).
     bool ready = warp == 0 && todo > 0 && operands(true, X.first_wait);
+    // Six slices: the other warps read the first tile's column scales, which came with the copy
+    // warp 0 has waited for.  (The later tiles' wait is ahead of the barrier between tiles.)
+    if (NS == 6) __syncthreads();
     const int q = warp & 3, hcol = warp >> 2;  // TMEM lane quadrant, column half of this warp
     const int rloc = 32 * q + lane;
     while (todo > 0) {
