@@ -287,9 +287,10 @@ MSG_D zc hyp0f1(double a, zc z) {
     t = t / tgamma(a);
     zc s = t;
     for (int i = 1; i <= 50; i++) {
-        // one reciprocal and squared moduli: a step is on the one thread's chain that the
-        // hard-sphere diagonal waits for
-        t = (t * z) * (1.0 / (i * a));
+        // (squared moduli in the test: a step is on the one thread's chain that the hard-sphere
+        // diagonal waits for.  A product with 1 / (i a) would save a division of two and cost a
+        // sixth more error at a = 3/2.)
+        t = t * z / (i * a);
         s += t;
         a += 1.0;
         if (zabs2(t) < 1e-32 * zabs2(s)) break;
