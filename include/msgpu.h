@@ -159,9 +159,9 @@ int msgpu_amplitude_batch(int nmed, const msgpu_medium* media, int nitem, const 
  * MSGPU_E_SIZE.  The array holds floor(~128 MiB / (16 n^2)) matrix slots, one
  * per engine CTA, capped at 2 per SM: 304 CTAs for n <= 165, 127 at n = 256,
  * 31 at n = 512, 7 at n = 1024 and 1 at n = 2048, all on the FP64 pipe,
- * against the hundreds of CTAs (and, above n = 104, the tensor cores) of the
+ * against the hundreds of CTAs (and, above 96 rows, the tensor cores) of the
  * allocating entry points, so large n runs at a small fraction of their
- * throughput.  Calls share that array, so calls that
+ * throughput, and above 96 rows the last bits of ln det are not theirs.  Calls share that array, so calls that
  * overlap on the GPU race: keep them on one stream.  The first call on a
  * device looks up the array's address; make it before any stream capture.
  * Counted in msgpu_launch_count (two launches per call); errors set the text

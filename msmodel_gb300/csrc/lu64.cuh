@@ -6,9 +6,9 @@
 // factor concurrently with no inter-CTA traffic, or the CTAs of a cluster.
 // Every element takes the same operations in the same order in any team.
 //
-// The FP64 pipe of GB300 is the roofline of this path (about 2 FP64 FMA
-// lanes per SM per clock): every loop below keeps the SM's FP64 FMAs fed
-// from shared-memory tiles; memory traffic is a few percent of the time.
+// GB300's FP64 pipe (about 2 FMA lanes per SM per clock) bounds what is here: panel,
+// TRSM, assembly, solves, and the trailing updates of matrices up to 96 rows (larger
+// ones': tc64.cuh).  Memory traffic is a few percent of the time.
 //
 // Pivoting follows LAPACK zgetf2/zgetrf: the pivot of column j is the first
 // row of maximum |Re|+|Im| (IZAMAX), ipiv is kept 0-based here, interchanges
@@ -226,7 +226,8 @@ __device__ __forceinline__ zc pivot_recip(zc b) {
 // barriers.  4096 ln det at n = 64 (d = 3): 19.6 ms with the full-width rank-1
 // form and a reciprocal per thread; 11.6 ms with one reciprocal; 6.8 ms with the
 // columns of few rows spread over the warps, warp reductions in the pivot search
-// and the small update tiles (11k -> 6k cycles a column at n = 100).
+// and the small update tiles (11k -> 6k cycles a column at n = 100); 5.7 ms with four
+// CTAs of 128 threads per SM.
 constexpr int SWP = 4;
 template <class S>
 static __device__ __noinline__ void panel_factor(zc* A, int n, int j0, int jb, int* ipiv, S& s) {

@@ -1,14 +1,15 @@
 // mixed_engine.cuh -- device side of the mixed-precision engine, shared by
-// mixed.cu (host side, launches) and the mixed_k*.cu units, each of which
-// defines MSG_MIXED_KERNEL_BODY and explicitly instantiates one (kind,
-// d = 3 only) variant of k_engine_mixed, so that the six variants compile in
-// parallel.
+// mixed.cu (host side, launches) and the mixed_k*.cu (a CTA per matrix) and
+// mixed_t*.cu (a cluster per matrix) units, each of which defines
+// MSG_MIXED_KERNEL_BODY and instantiates one (kind, d = 3 only) variant of
+// k_engine_mixed, so that the twelve variants compile in parallel.
 #pragma once
 // The mixed-precision engine: the LU trailing updates run on the
 // tcgen05 tensor cores as exact products of bf16 slices, everything else in
-// double-float (FP32 hi + lo) on the FP32 pipe: the panel, the TRSM, the
-// epilogue and, for d = 3, the whole matrix assembly; the pivot reciprocals,
-// ln and the d = 2 Green functions (K_nu) in FP64.
+// double-float (FP32 hi + lo) on the FP32 pipe: the panel with its pivots'
+// reciprocals, the TRSM, the epilogue and, for d = 3 and d = 2, the matrix
+// assembly.  In FP64: the elements on the diagonal, those of other dimensions, the
+// reciprocals of U's diagonal in the solves, the refinement's residuals and ln.
 //
 // Trailing update C -= A B (A: m x K panel, B: K x nn rows, K <= 32, complex):
 //  * every row of A (column of B) is scaled by a power of two so its largest
@@ -30,9 +31,10 @@
 //    ~1.4e-9 of FP64, while at d = 2, Im k = -0.3, N = 2048 (span 2^19, the
 //    exponential growth e^{|Im k| r} over a disk of radius 25) they leave
 //    ~1e-5 and six slices are needed;
-//  * complex = 3 MMAs: A_re (Re B, Im B) together, A_im Im B with the negate-B bit of
-//    the instruction descriptor, A_im Re B; the accumulators use 2 NG TN TMEM
-//    columns (192 or 128);
+//  * a complex product is three MMAs with four slices, A_re (Re B, Im B) together,
+//    A_im Im B with the negate-B bit of the instruction descriptor and A_im Re B, into
+//    2 NG TN = 192 TMEM columns; with six slices two, A_re and A_im with (Re B, Im B),
+//    into 4 NG TN = 256;
 //  * epilogue: C (double-float, global) -= 2^(ea+eb-16) (sum of the levels).
 // Operand slices are written to global images in the tensor core's
 // core-matrix layout and moved to shared memory by bulk copies (TMA engine).
@@ -51,7 +53,7 @@ namespace msg {
 
 constexpr int MT_M = 128;               // tile rows = TMEM lanes
 constexpr int A_SUB = MT_M * NB * 2;    // one 128 x 32 bf16 operand tile: 8 KB
-constexpr int TMEM_COLS = 256;          // accumulators: 2 NG TN <= 192 columns (allocation rounded to 2^k)
+constexpr int TMEM_COLS = 256;          // accumulators: 192 (four slices) or 256 columns; two CTAs share the SM's 512
 constexpr float RANGE_LIMIT = 1.0e18f;  // larger entries leave the safe FP32 exponent range
 constexpr float SPAN_WIDE = 256.0f;     // entry span above which an item is sliced six ways
 // amplitude items (iterative refinement to an FP64 residual): the LU only has to
@@ -66,10 +68,12 @@ template <int NS> struct SliceCfg;
 // 304 ln det at d = 2, n = 2048 561 -> 512 ms, 512 dlogf at n = 300 23.0 -> 21.8
 template <> struct SliceCfg<4> { static constexpr int TN = 32, NG = 3, GC = 2 * 32; };
 template <> struct SliceCfg<6> { static constexpr int TN = 16, NG = 4, GC = 4 * 16; };
+static_assert(SliceCfg<4>::NG * SliceCfg<4>::GC <= TMEM_COLS && SliceCfg<6>::NG * SliceCfg<6>::GC <= TMEM_COLS,
+              "the accumulators fit the allocation");
 template <int NS> __host__ __device__ constexpr int a_band() { return 2 * NS * A_SUB; }  // NS slices x {Re, Im}
 // A B tile's operand rows, per slice: Re, Im of its columns, so that A_re times
-// (Re, Im) is one MMA of N = 2 TN: three MMAs a complex product.  304 ln det at
-// d = 2, n = 2048: 647 ms with four, 605 with three; 512 dlogf 10% less.  (A third block of
+// (Re, Im) is one MMA of N = 2 TN.  304 ln det at d = 2, n = 2048: 647 ms with four
+// MMAs a complex product, 605 with three (before six slices took two); 512 dlogf 10% less.  (A third block of
 // rows, -Im, makes it two, but the shared memory comes out of the L1 cache: 2% slower
 // at n = 64, and no room for two CTAs per SM with six slices.)
 template <int NS> __host__ __device__ constexpr int b_rows() { return 2 * SliceCfg<NS>::TN; }
@@ -381,7 +385,7 @@ static __device__ void mixed_gemm_sub(float4* __restrict__ C, int ldc, const flo
         while (bi < nbi && bj >= width(bi)) bj -= width(bi++);
     }
     // A tile's B operand, and with six slices its column scales (read in the epilogue, beside
-    // the next tile's copy, hence two of them): 304 ln det at d = 2, n = 2048 513 -> 486 ms
+    // the next tile's copy, hence two of them): 304 ln det at d = 2, n = 2048 513 -> 491 ms
     // against a global load each, which waits behind the stores to C.  With four slices the
     // second copy cost 3% at n = 1024.
     auto load_b = [&](int col, int p) {
