@@ -9,11 +9,12 @@ sample = 4096).  One step = the hot path over the whole cut.
   value  : evals/s with positions and k already resident in HBM (msgpu_job_run)
   e2e    : evals/s through the C-ABI call a user makes with host buffers
            (msgpu_tracelog_batch: H2D of inputs, the kernels, D2H of results)
-  roofline: the tensor pipe, which carries the N^3 work: achieved = the bf16
-           flops of the digit products (28 of them for 8/3 N^3 real flops per ln
-           det) / step time, peak from MEASURED_PEAKS.json; beside it the
-           algorithmic rate and the FP64 pipe's (DFMA probe run here), and the
-           DRAM traffic of one ncu capture scaled to the launch
+  roofline: the FP64 pipe, the busiest unit of the step: achieved = what
+           panel, column solves, assembly and the updates' additions put on it /
+           step time, peak = a DFMA probe run here; beside it the tensor pipe (the
+           bf16 flops of the digit products, 36 of them for 8/3 N^3 real flops per
+           ln det, against MEASURED_PEAKS.json), the algorithmic rate, and the DRAM
+           traffic of one ncu capture scaled to the launch
   cpu_baseline: the reference algorithm on all host cores, bounded sample
   clocks: nvidia-smi samples during the timed region
   gpu_launches: this library's kernel launches in the timed region
@@ -728,6 +729,19 @@ def run_reference(args):
     return 0
 
 
+def fp64_pipe_slots(n):
+    """FP64 FMAs and additions of one ln det of the FP64 engine above 96 rows: per
+    32-column panel of m rows the rank-1 updates (4 FMAs an element), the column
+    solves right of it, one addition a component and updated element; and about 35 a
+    pair of scatterers in the assembly (d = 3)."""
+    slots = 35 * n * n / 2
+    for j0 in range(0, n, 32):
+        m, jb = n - j0, min(32, n - j0)
+        r = m - jb
+        slots += 4 * (m * jb * (jb - 1) / 2) + 4 * (r * jb * (jb - 1) / 2) + 2 * r * r
+    return slots
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -828,11 +842,15 @@ def main():
         # the FP64 pipe (DFMA) and the FP64 tensor path (warp-level m8n8k4 MMA), measured here
         peak_mma = ms.probe_fp64_mma_tflops()
         bf16 = peaks.get("bf16_tflops_sustained", 1728.6)
-        # trailing updates: 28 products of 9-bit digits for every FP64 one
-        roof = {"bound": "tensor", "achieved": 28 * achieved, "peak": bf16, "unit": "TFLOP/s", "frac": 28 * achieved / bf16,
-                "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained",
-                "executed": "28 bf16 digit products per real product of the complex LU (8/3 N^3 real flops)",
-                "algorithmic_tflops": achieved, "fp64_fma_probe_tflops": peak, "fp64_mma_probe_tflops": peak_mma,
+        pipe = 2 * fp64_pipe_slots(natom) * len(ks) / (tot / args.steps) / 1e12
+        # trailing updates: 36 products of 9-bit digits for every FP64 one
+        roof = {"bound": "fp64", "achieved": pipe, "peak": peak, "unit": "TFLOP/s", "frac": pipe / peak,
+                "peak_source": "measured DFMA probe on this GPU (MEASURED_PEAKS.json has no FP64 entry)",
+                "executed": "FP64 FMAs and additions of panel, column solves, assembly and update epilogues (full "
+                            "warps assumed), 2 flops a slot",
+                "tensor": {"achieved": 36 * achieved, "peak": bf16, "frac": 36 * achieved / bf16,
+                           "executed": "36 bf16 digit products per real product of the complex LU (8/3 N^3 real flops)"},
+                "algorithmic_tflops": achieved, "fp64_mma_probe_tflops": peak_mma,
                 "algorithmic": "8/3 N^3 real flops per ln det (complex LU), N=1024: 2.863e9",
                 "traffic": None}
     else:
