@@ -276,6 +276,8 @@ struct msgpu_job {
     // the job's device arrays, all in one block
     void* block = nullptr;
     size_t block_bytes = 0;
+    std::atomic<unsigned> runs{0}, done{0};  // runs queued, and how many of them are known to be over
+    bool captured = false;   // a run went into a graph of the caller's, which may replay it at any time
     MedDev* d_media = nullptr;
     double* d_pos = nullptr;
     size_t items_b = 0;      // bytes from d_ks to the live count: the item arrays at full capacity
@@ -507,7 +509,7 @@ static int set_items_locked(msgpu_job* J, int nitem, const int* item_med, const 
     return 0;
 }
 
-// (the job's runs have completed: its block may be another job's next)
+// (the block, if it is still the job's, is idle: it may be another job's next)
 static void destroy_locked(msgpu_job* J) {
     if (J->gexec) cudaGraphExecDestroy(J->gexec);
     if (J->cap_stream) cudaStreamDestroy(J->cap_stream);
@@ -771,6 +773,9 @@ int msgpu_job_run(msgpu_job* J, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     void* ws = nullptr;
     if (int e = ensure_ws(J->ws_bytes, &ws)) return e;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) J->captured = true;
+    ++J->runs;
     if (!J->use_graph) {
         if (int e = launch_locked(J, ws, st)) return e;
         g_launches++;
@@ -812,7 +817,9 @@ double msgpu_job_flops(const msgpu_job* J) { return J ? J->flops : 0.0; }
 
 int msgpu_job_results(msgpu_job* J, double* out, int* status) {
     if (!J) return set_err(MSGPU_E_ARG, "null job");
+    const unsigned runs = J->runs;
     CK(cudaDeviceSynchronize());
+    J->done = runs;
     if (out) CK(cudaMemcpy(out, J->d_out, sizeof(double) * 2 * J->nitem, cudaMemcpyDeviceToHost));
     if (status) CK(cudaMemcpy(status, J->d_status, sizeof(int) * J->nitem, cudaMemcpyDeviceToHost));
     return 0;
@@ -837,10 +844,13 @@ int msgpu_job_set_vectors(msgpu_job* J, const double* vecs) {
 
 void msgpu_job_destroy(msgpu_job* J) {
     if (!J) return;
-    // A run may be on the device that this library does not know of (a graph of the caller's
-    // that captured msgpu_job_run), so every destroy waits, as cudaFree of the arrays would
-    // have; outside the lock, so that other threads' calls go on meanwhile.
-    cudaDeviceSynchronize();
+    // The block is kept for the next job only if no run can be on the device: a run whose
+    // results were not fetched may be, and a replay of a graph of the caller's.  Else it is
+    // freed, which waits; outside the lock, so that other threads' calls go on meanwhile.
+    if (J->captured || J->done != J->runs) {
+        cudaFree(J->block);
+        J->block = nullptr;
+    }
     std::lock_guard<std::mutex> lk(g_mu);
     destroy_locked(J);
 }

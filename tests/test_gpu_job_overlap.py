@@ -52,3 +52,35 @@ def test_destroy_waits_for_a_callers_graph(ms, precision):
         got, st = nxt.results()
         nxt.close()
         assert np.all(st == 0) and np.array_equal(got, want)
+
+
+def test_destroy_beside_a_capture(ms):
+    """Destroying an idle job asks nothing of the device: a capture of the caller's
+    that is under way (a job collected as garbage meanwhile) stays valid."""
+    torch = pytest.importorskip("torch")
+    job = ms.Job("tracelog", [ms.Medium(3, 60, seed=4)], [1.1 + 0j, 2.0 + 0j])
+    job.run()
+    job.results()
+    x = torch.zeros(16, device="cuda")
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side, capture_error_mode="relaxed"):
+        x += 1
+        job.close()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.all(x == 1)
+
+
+def test_destroy_while_running(ms):
+    """A job destroyed with its run in flight, the next of its size at once."""
+    torch = pytest.importorskip("torch")
+    med = ms.Medium(3, 700, seed=4)
+    ks = 0.7 + 0.02 * np.arange(100) - 0.05j
+    want, _ = ms.tracelog_batch([med], ks + 0.3)
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        job = ms.Job("tracelog", [med], ks)
+        job.run(side.cuda_stream)
+        job.close()
+        got, st = ms.tracelog_batch([med], ks + 0.3)
+        assert np.all(st == 0) and np.array_equal(got, want)
