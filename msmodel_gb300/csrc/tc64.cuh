@@ -22,7 +22,7 @@
 // while the tensor core has the next tile.
 //
 // Measured against the FP64 pipe's update in the same kernel: 198 ln det at d = 3,
-// n = 1024 130 ms and 627, 152 at n = 512 15.2 and 57.9, 304 at n = 160 3.0 and 5.2, 152 dlogf
+// n = 1024 126 ms and 627, 152 at n = 512 14.5 and 57.9, 304 at n = 160 3.0 and 5.2, 152 dlogf
 // at n = 300 11.7 and 45.8; 152 ln det at d = 2, n = 700, where more is redone, 162 and 258.
 // Error of ln det / n against a wider LU of the same matrix (n = 300, rms of 6): d = 3,
 // real k 2.0e-16 and 1.9e-16, Im k = -0.05 1.3e-16 and 2.4e-16, -1 4.9e-16 and 4.7e-16; d = 2,
@@ -308,7 +308,20 @@ __device__ __forceinline__ double tc_double(long long v, int xe) {
 static __device__ __noinline__ void tc_redo(zc* C, int ldc, const zc* Ap, int lda, const zc* Bp, int ldb, int K, int row,
                                             int col) {
     zc a = C[row + (size_t)col * ldc];
-    for (int k = 0; k < K; ++k) a = zfms(a, Ap[row + (size_t)k * lda], Bp[k + (size_t)col * ldb]);
+    const zc* l = Ap + row;
+    const zc* u = Bp + (size_t)col * ldb;
+    int k = 0;
+    for (; k + 8 <= K; k += 8) {  // eight operands on their way ahead of the chain
+        zc lk[8], uk[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            lk[j] = l[(size_t)(k + j) * lda];
+            uk[j] = u[k + j];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a = zfms(a, lk[j], uk[j]);
+    }
+    for (; k < K; ++k) a = zfms(a, l[(size_t)k * lda], u[k]);
     C[row + (size_t)col * ldc] = a;
 }
 
@@ -341,10 +354,13 @@ static __device__ __noinline__ void tc_update(zc* C, int ldc, const zc* Ap, int 
         mbar_arrive_expect_tx(&s.bar_b, TC_BDIG);
         bulk_g2s(s.g.b, t.img + (size_t)col * TC_BTILE, TC_BDIG, &s.bar_b);
     };
-    // the elements on the list of tile number x, tile (i, j)
+    // the elements on the list of tile number x, tile (i, j): a chain of 64 FMAs, 4 k cycles, that
+    // is over before the next tile's MMAs unless warp 0, which issues them, takes part
+    // (ln det at n = 1024, one such element a tile: update 80 M cycles, 84 with warp 0)
     auto redo = [&](int x, int i, int j) {
         const int cnt = s.redo_n[x % 3];
-        for (int e = tid; e < cnt; e += TC_NT) {
+        if (warp == 0) return;
+        for (int e = tid - 32; e < cnt; e += TC_NT - 32) {
             const int c = s.redo[x & 1][e];
             tc_redo(C, ldc, Ap, lda, Bp, ldb, K, i * TC_M + c / TC_N, j * TC_N + c % TC_N);
         }
